@@ -21,7 +21,7 @@ LIB = os.path.join(HERE, "libpaintop_cuda.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CU_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
                    "--expt-relaxed-constexpr", "-I" + os.path.join(ROOT, "include")]
-SOURCES = ["rbsor_kernels.cu", "solver_host.cu", "op_host.cpp", "autotune.cpp", "noalloc.cu",
+SOURCES = ["rbsor_kernels.cu", "rbsor_cluster.cu", "solver_host.cu", "op_host.cpp", "autotune.cpp", "noalloc.cu",
            "mask_kernels.cu", "mg_solver.cu", "unet/unet_kernels.cu", "unet/conv_tma.cu", "unet/unet.cu"]
 
 

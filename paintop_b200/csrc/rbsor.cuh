@@ -137,6 +137,48 @@ struct Tile {
   int sys, tx, ty, pad;
 };
 
+// How a cluster of thread blocks holds a region (rbsor_cluster.cu). The box is
+// cut into patches of 8 columns x `rows` rows from (x0, y0), one per thread: nq
+// across, and m rows of patches in each of the n blocks (the last one what is
+// left of the box's bm). limit: patches a block may hold.
+struct Route {
+  int n, x0, y0, nq, bm, m, rows, limit;
+};
+
+constexpr int kClusterMax = 16;       // blocks per cluster
+constexpr int kClusterMost = 480;     // patches per block at most (a warp more keeps the books)
+constexpr int kClusterLeast = 224;    // ... and the least that are asked for before a second block
+
+// The split of a region with this bounding box, or false when it does not fit
+// a cluster. It depends on the box alone, so a system's partial sums, and with
+// them its results, do not depend on what else the call solves.
+__host__ __device__ inline bool cluster_route(int bx0, int by0, int bx1, int by1, Route *r) {
+  if (bx1 < bx0 || by1 < by0) return false;
+  const int x0 = (bx0 - 1) & ~7, y0 = by0 & ~1;  // an even first row: a row's colours sit alike in every patch
+  const int nq = (bx1 + 1 - x0) / 8 + 1, bh = by1 + 1 - y0;
+  // two-row patches halve a half-sweep's latency, four-row ones hold more and
+  // convert less; blocks of the least size leave an SM room for a second one
+  for (int k = 0; k < 4; ++k) {
+    const int rows = k & 1 ? 4 : 2, t = k < 2 ? kClusterLeast : kClusterMost;
+    const int bm = (bh + rows - 1) / rows;
+    if (nq > t || (bm + t / nq - 1) / (t / nq) > kClusterMax) continue;
+    // even shares; of a region that needs more than the least blocks, to all 16
+    const int n = k > 1 ? kClusterMax : (bm + t / nq - 1) / (t / nq);
+    const int m = (bm + n - 1) / n;
+    r->x0 = x0; r->y0 = y0; r->nq = nq; r->bm = bm; r->m = m; r->rows = rows; r->limit = t;
+    r->n = (bm + m - 1) / m;
+    return true;
+  }
+  return false;
+}
+
+// A block's windows in shared memory (rbsor_cluster.cu): four arrays of first
+// and last rows, (m + 1) nq <= most + nq <= 2 most groups of four, and four of
+// edges, m (nq + 2) <= 3 most pairs. Fixed places, so that a thread's accesses
+// differ by constants; two blocks of the least size fit an SM.
+constexpr int kWinRows = 16 * 2 * kClusterMost, kWinEdges = 8 * 3 * kClusterMost;
+constexpr int kClusterSmem = 4 * kWinRows + 4 * kWinEdges;
+
 struct KParams {
   const SysDesc *sys;
   SysState *st;
@@ -165,6 +207,7 @@ struct KParams {
   int *label;              // per pixel: region root (local pixel index) or -1
   int *rsize;              // per pixel: region size, at the root
   int *rmax;               // per RegionDesc: largest region size
+  Route *route;            // per system: its cluster's split, n = 0 for k_solve's (null: all are)
 };
 
 }  // namespace ptk

@@ -1,29 +1,13 @@
 // rbsor_kernels.cu -- device kernels of the red-black SOR solver (sm_100a).
 // See rbsor.cuh for the method, the HBM layout and the control scheme.
 #include "rbsor.cuh"
+#include "rbsor_device.cuh"
 #include "rbsor_launch.h"
 
 #include <cmath>
 #include <cstdio>
 
 namespace ptk {
-
-// ----------------------------------------------------------------------------
-// small device helpers
-// ----------------------------------------------------------------------------
-__device__ __forceinline__ unsigned long long gtimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ int ld_vol(const int *p) { return *reinterpret_cast<const volatile int *>(p); }
 
 // Asynchronous global -> shared copies (Ampere+ cp.async). `in == false` copies
 // no bytes and zero-fills the destination.
@@ -41,25 +25,6 @@ __device__ __forceinline__ void cp_async4(void *smem_dst, const void *gmem_src, 
 }
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-}
-
-// Deterministic block sum: fixed xor-butterfly inside each warp, then warps in
-// index order. The total is valid in thread 0. Uses sred[0 .. blockDim.x/32).
-__device__ __forceinline__ double block_sum(double v, double *sred) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (lane == 0) sred[warp] = v;
-  __syncthreads();
-  double tot = 0.0;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += sred[w];
-  __syncthreads();
-  return tot;
-}
-
-__device__ __forceinline__ long long plane_index(const SysDesc &d, int c, int y, int i) {
-  return d.off + (long long)c * d.plane + (long long)y * d.pw + i;
 }
 
 // ----------------------------------------------------------------------------
@@ -324,8 +289,18 @@ __global__ void k_init(KParams P) {
   for (int o = 16; o > 0; o >>= 1) nact += __shfl_xor_sync(0xffffffffu, nact, o);
   __shared__ int sn[kWarps];
   if ((threadIdx.x & 31) == 0) sn[threadIdx.x >> 5] = nact;
+  // the region's bounding box, over the tiles (min and max do not depend on the order)
+  __shared__ int sbox[4];
+  if (threadIdx.x < 4) sbox[threadIdx.x] = threadIdx.x < 2 ? 0x7fffffff : -1;
+  __syncthreads();
+  for (int k = threadIdx.x; k < d.ntiles; k += blockDim.x) {
+    if (P.tcount[d.tile0 + k] == 0) continue;
+    const int4 b = P.tbox[d.tile0 + k];
+    atomicMin(&sbox[0], b.x); atomicMin(&sbox[1], b.y); atomicMax(&sbox[2], b.z); atomicMax(&sbox[3], b.w);
+  }
   __syncthreads();
   if (threadIdx.x != 0) return;
+  const int bx0 = sbox[0], by0 = sbox[1], bx1 = sbox[2], by1 = sbox[3];
   int n = 0;
   for (int w = 0; w < (int)(blockDim.x >> 5); ++w) n += sn[w];
   SysState s;
@@ -348,13 +323,6 @@ __global__ void k_init(KParams P) {
     // automatic SOR factor: Young's optimum for red-black SOR with the Jacobi
     // spectral radius of (4+lambda)I - N on the region's bounding box (a x b
     // cells including the boundary ring): (2cos(pi/a) + 2cos(pi/b)) / (4+lambda)
-    int bx0 = 0x7fffffff, by0 = 0x7fffffff, bx1 = -1, by1 = -1;
-    for (int k = 0; k < d.ntiles; ++k) {
-      const int t = d.tile0 + k;
-      if (P.tcount[t] == 0) continue;
-      const int4 b = P.tbox[t];
-      bx0 = min(bx0, b.x); by0 = min(by0, b.y); bx1 = max(bx1, b.z); by1 = max(by1, b.w);
-    }
     double om = 1.0;
     if (bx1 >= 0) {
       const double a = (double)(bx1 - bx0 + 2), b = (double)(by1 - by0 + 2);
@@ -396,9 +364,16 @@ __global__ void k_init(KParams P) {
   } else {
     s.s = d.max_it < P.S ? d.max_it : P.S;
   }
+  // a region that one thread-block cluster can hold is k_cluster_solve's: for
+  // k_solve it counts as done
+  Route r{};
+  if (P.route) {
+    if (s.mode != M_DONE && cluster_route(bx0, by0, bx1, by1, &r)) atomicAdd(P.bar + 2, 1u);
+    P.route[sys] = r;
+  }
   P.st[sys] = s;
   P.arrive[sys] = 0;
-  P.claim[sys] = s.mode == M_DONE ? (unsigned long long)kClaimDone : 0ull;
+  P.claim[sys] = (s.mode == M_DONE || r.n) ? (unsigned long long)kClaimDone : 0ull;
 }
 
 // Restore the anchor start (u = anchor, g = -r(anchor), as k_assemble writes
@@ -764,107 +739,19 @@ __device__ void resid_tile(const KParams &P, const SysDesc &d, int t, const Tile
   if (threadIdx.x == 0) P.partial[t] = acc;
 }
 
-__device__ __forceinline__ void apply_stall(SysState &s, double rel, int &done) {
-  // poisson.rs:219-228 (window 16 for a given omega; see k_init for automatic omega)
-  if (rel < s.best * (1.0 - kStallImprovement)) {
-    s.best = rel;
-    s.since = 0;
-  } else {
-    s.since += 1;
-    if (s.since >= s.stall_window) done = 1;
-  }
-}
-
-__device__ SysState load_state(const SysState *p) {
-  SysState s;
-  const int *pi = reinterpret_cast<const int *>(p);
-  int *si = reinterpret_cast<int *>(&s);
-  for (int k = 0; k < (int)(sizeof(SysState) / sizeof(int)); ++k) si[k] = __ldcg(pi + k);
-  return s;
-}
-
 // The state machine step run by the last tile of a system to finish a step
 // (thread 0 only). sums[j] = sum of the tile partials of sweep j (tile order).
 __device__ void advance(const KParams &P, const SysDesc &d, SysState *stp, int mode,
                         const double *sums) {
-  SysState s = load_state(stp);
-  double *hist = P.hist + d.hist_off;
-  const int cap = P.S;
-  switch (mode) {
-    case M_SWEEP: {
-      int kind = P_NONE, stop_j = -1;
-      bool refine = false;
-      for (int j = 0; j < s.s; ++j) {
-        const double nrm = sqrt(sums[j]);
-        const double rel = nrm / s.r0;  // poisson.rs:206
-        s.iterations += 1;
-        hist[s.iterations - 1] = rel;
-        s.last = rel;
-        if (rel <= d.tol) { kind = P_CONV; stop_j = j; break; }  // poisson.rs:210-214
-        int stalled = 0;
-        apply_stall(s, rel, stalled);
-        if (stalled) { kind = P_STALL; stop_j = j; break; }
-        if (s.iterations >= d.max_it) { kind = P_MAX; stop_j = j; break; }
-        // residual-correction trigger (does not change the iterate, only when
-        // the FP64 fold happens, so it waits for the end of the block)
-        if (nrm <= kRefineFactor * s.ibase) refine = true;
-        if (nrm < s.ibest * kInnerGain) { s.ibest = nrm; s.isince = 0; }
-        else if (++s.isince >= kInnerWindow) refine = true;
-      }
-      if (kind == P_NONE) {
-        s.cur ^= 1;
-        if (refine) { s.pending = P_REFINE; s.mode = M_FOLD; }
-        else { s.mode = M_SWEEP; s.s = min(cap, d.max_it - s.iterations); }
-      } else if (stop_j == s.s - 1) {
-        s.cur ^= 1; s.pending = kind; s.mode = M_FOLD;
-      } else {
-        // stop inside the block: re-run the block from the same start with
-        // exactly stop_j+1 sweeps (identical arithmetic), so the iterate kept is
-        // the one after the reported sweep.
-        s.pending = kind; s.mode = M_REDO; s.s = stop_j + 1;
-      }
-    } break;
-    case M_REDO:
-      s.cur ^= 1;
-      s.mode = M_FOLD;
-      break;
-    case M_FOLD:
-      s.mode = M_RESID;
-      break;
-    case M_RESID: {
-      const double nrm = sqrt(sums[0]);
-      const double rel = nrm / s.r0;
-      s.outer = nrm;
-      s.ibase = nrm;
-      s.ibest = INFINITY;
-      s.isince = 0;
-      s.refinements += 1;
-      if (s.iterations > 0) { hist[s.iterations - 1] = rel; s.last = rel; }
-      int stop = -1;
-      if (rel <= d.tol) stop = STOP_CONVERGED;
-      else if (s.pending == P_STALL) stop = STOP_STALLED;
-      else if (s.pending == P_MAX || s.iterations >= d.max_it) stop = STOP_MAX;
-      else if (s.pending == P_CONV) {
-        // the per-sweep estimate met the tolerance but the FP64 residual does
-        // not: apply the stall rule the estimate skipped, then keep sweeping
-        int stalled = 0;
-        apply_stall(s, rel, stalled);
-        if (stalled) stop = STOP_STALLED;
-      }
-      s.pending = P_NONE;
-      if (stop >= 0) {
-        s.mode = M_DONE;
-        s.status = stop;
-        atomicAdd(P.bar + 2, 1u);
-      } else {
-        s.mode = M_SWEEP;
-        s.s = min(cap, d.max_it - s.iterations);
-      }
-    } break;
-    default:
-      break;
-  }
-  s.steps += 1;
+  SysState s = load_sys_state(stp);
+  double nrms[4], rels[4];  // at most four sweeps a step (tile_config)
+  const int n = mode == M_SWEEP ? s.s : (mode == M_RESID ? 1 : 0);
+  for (int j = 0; j < 4; ++j)
+    if (j < n) {
+      nrms[j] = sqrt(sums[j]);
+      rels[j] = nrms[j] / s.r0;
+    }
+  if (step_state(d, s, mode, nrms, rels, P.hist + d.hist_off, P.S)) atomicAdd(P.bar + 2, 1u);
   *stp = s;
 }
 

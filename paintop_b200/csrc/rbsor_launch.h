@@ -26,6 +26,18 @@ cudaError_t launch_solve(const KParams &P, int cfg, int sms, cudaStream_t stream
 // stream operation, so it stays outside a stream capture), then launch.
 cudaError_t prepare_solve(const KParams &P, int cfg, int sms, int *grid);
 cudaError_t launch_prepared(const KParams &P, int cfg, int grid, cudaStream_t stream);
+// The systems whose regions a cluster of thread blocks holds (k_cluster_solve,
+// rbsor_cluster.cu), launched in classes of one cluster and block size each:
+// the systems list[first .. first + count), at most `limit` patches and `smem`
+// bytes a block.
+struct ClusterClass {
+  int first, count, blocks, limit, smem;
+  bool rows4;  // a region of the class may take patches of four rows
+};
+constexpr int kClusterAlone = 120 * 1024;  // shared memory that keeps a second block off the SM
+cudaError_t prepare_cluster();  // the kernel's attributes (outside a capture)
+cudaError_t launch_cluster(const KParams &P, const TileConfig &tc, const ClusterClass &k, const int *list,
+                           cudaStream_t stream);
 // k_tile_count alone (interior cells and box per tile; reads only the masks).
 cudaError_t launch_tile_count(const KParams &P, const TileConfig &tc, cudaStream_t stream);
 // spans[2 ty], spans[2 ty + 1] = the first and last tile column of row band ty

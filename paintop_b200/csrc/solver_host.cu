@@ -91,12 +91,14 @@ struct Plan {
   long long out_floats = 0;
   std::vector<RegionDesc> regions;  // images labelled for the automatic omega
   long long rpix = 0;               // their pixels
+  std::vector<int> clist;           // the systems by cluster class
+  std::vector<ClusterClass> classes;
 };
 
 // Arena layout (byte offsets) for one call.
 struct Layout {
   size_t sys, st, claim, arrive, tiles, tcount, tbox, act, e0, e1, g, cell, u, bp, partial, fpart, hist, bar, err, in,
-      mask, out, regions, label, rsize, rmax, bands, total;
+      mask, out, regions, label, rsize, rmax, bands, route, clist, total;
 };
 
 // Row bands of every image (host-buffer solves: two ints each, the band's
@@ -140,8 +142,70 @@ Layout layout(const Plan &pl, bool stage) {
   L.rsize = take((size_t)pl.rpix * sizeof(int));
   L.rmax = take(pl.regions.size() * sizeof(int));
   L.bands = stage ? take(2 * band_count(pl) * sizeof(int)) : 0;
+  L.route = take(ns * sizeof(Route));
+  L.clist = take(pl.clist.size() * sizeof(int));
   L.total = o;
   return L;
+}
+
+// The launches of k_cluster_solve: the systems by the cluster and block size
+// their images can need at most (the masks are on the device, so the regions
+// are not known here; k_init splits each by its bounding box, and a block that
+// a split does not use returns at once). An image that no cluster holds whole
+// may still have a region that one does, so it goes with the largest. Classes
+// keep small regions from being scheduled in gangs of 16 blocks.
+//
+// Like the tile configuration, the choice of kernel depends on the call's
+// shapes alone. A call of fewer than 4e6 values leaves k_solve with fewer tiles
+// than it has places for, each step of it a chain of latencies: 5.9 us a sweep
+// on 512 x 512 RGB against 2.4 here, 5.2 against 1.7 on 97 x 71. A larger call
+// fills k_solve's places, and clusters pay only if all its images fit the least
+// blocks, two to an SM (128 images of 256 x 256: 10.9 against 9.4 ms); with
+// larger ones among them (48 images of side 64 to 1024: 57 against 68 ms) they
+// hold SMs in gangs that the rest could use.
+constexpr double kFewValues = 4.0e6;
+void plan_clusters(Plan &pl, int sms) {
+  struct Want { int blocks, limit; bool rows4; };
+  std::vector<Want> want(pl.sys.size(), Want{0, 0, false});
+  bool least = true;
+  double values = 0.0;
+  for (size_t i = 0; i < pl.sys.size(); ++i) {
+    const SysDesc &d = pl.sys[i];
+    values += (double)d.W * d.H;
+    if (d.W < 3 || d.H < 3) continue;  // no interior (k_init)
+    Route r{};
+    if (!cluster_route(1, 1, d.W - 2, d.H - 2, &r) || r.limit > kClusterLeast) least = false;
+    if (r.limit == 0) {
+      want[i] = Want{kClusterMax, kClusterMost, true};
+      continue;
+    }
+    // a smaller region takes no larger blocks, and more of them only where
+    // this image takes larger ones or four-row patches
+    int blocks = 1;
+    while (blocks < r.n) blocks *= 2;
+    const bool more = r.limit > kClusterLeast || r.rows > 2;
+    want[i] = Want{more ? kClusterMax : blocks, r.limit, more};
+  }
+  if (values >= kFewValues && !least) return;
+  for (size_t i = 0; i < want.size(); ++i) {
+    if (!want[i].blocks) continue;
+    ClusterClass k{(int)pl.clist.size(), 0, want[i].blocks, want[i].limit, kClusterSmem,
+                   want[i].rows4};
+    for (size_t q = i; q < want.size(); ++q) {
+      if (want[q].blocks != k.blocks || want[q].limit != k.limit || want[q].rows4 != k.rows4) continue;
+      pl.clist.push_back((int)q);
+      k.count += 1;
+      want[q].blocks = 0;
+    }
+    pl.classes.push_back(k);
+  }
+  // Blocks whose results are waited for one half-sweep at a time are better
+  // off alone on an SM while there are SMs to spare: shared memory asked for
+  // beyond their own keeps others away.
+  long long total = 0;
+  for (const ClusterClass &k : pl.classes) total += (long long)k.count * k.blocks;
+  if (total <= sms * 3 / 4 + 1)
+    for (ClusterClass &k : pl.classes) k.smem = kClusterAlone;
 }
 
 }  // namespace
@@ -239,6 +303,8 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
     return PT_OK;
   }
 
+  plan_clusters(pl, ctx->sms);
+
   std::lock_guard<std::mutex> lock(ctx->mu);
   cudaError_t ce = cudaSetDevice(ctx->device);
   if (ce != cudaSuccess) return cuda_fail(ctx, ce, "cudaSetDevice");
@@ -283,7 +349,8 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
       }
     }
   }
-  h2d += pl.sys.size() * sizeof(SysDesc) + pl.tiles.size() * sizeof(Tile) + pl.regions.size() * sizeof(RegionDesc);
+  h2d += pl.sys.size() * sizeof(SysDesc) + pl.tiles.size() * sizeof(Tile) + pl.regions.size() * sizeof(RegionDesc) +
+         pl.clist.size() * sizeof(int);
   ce = cudaMemcpyAsync(base + L.sys, pl.sys.data(), pl.sys.size() * sizeof(SysDesc),
                        cudaMemcpyHostToDevice, st);
   if (ce == cudaSuccess)
@@ -292,6 +359,8 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
   if (ce == cudaSuccess && !pl.regions.empty())
     ce = cudaMemcpyAsync(base + L.regions, pl.regions.data(), pl.regions.size() * sizeof(RegionDesc),
                          cudaMemcpyHostToDevice, st);
+  if (ce == cudaSuccess && !pl.clist.empty())
+    ce = cudaMemcpyAsync(base + L.clist, pl.clist.data(), pl.clist.size() * sizeof(int), cudaMemcpyHostToDevice, st);
   if (ce != cudaSuccess) return cuda_fail(ctx, ce, "plan upload");
 
   KParams P{};
@@ -324,6 +393,7 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
   P.label = reinterpret_cast<int *>(base + L.label);
   P.rsize = reinterpret_cast<int *>(base + L.rsize);
   P.rmax = reinterpret_cast<int *>(base + L.rmax);
+  P.route = pl.classes.empty() ? nullptr : reinterpret_cast<Route *>(base + L.route);
 
   // ---- host buffers: upload only the part of the images the solve reads.
   // The tiles are counted from the masks, and for each image and row band of
@@ -452,11 +522,14 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
   }
 
   int grid = 0;
-  ce = prepare_solve(P, pl.cfg, ctx->sms, &grid);
+  ce = prepare_cluster();
+  if (ce == cudaSuccess) ce = prepare_solve(P, pl.cfg, ctx->sms, &grid);
   if (ce != cudaSuccess) return cuda_fail(ctx, ce, "solve prepare");
   ctx->last_grid = grid;
   ctx->last_cfg = pl.cfg;
-  long long launches = 5;  // tile count, compaction, assembly, init, solve
+  long long cluster_launches = 0;
+  for (const ClusterClass &k : pl.classes) cluster_launches += k.rows4 ? 2 : 1;
+  long long launches = 5 + cluster_launches;  // tile count, compaction, assembly, init, solves
   for (uint32_t i = 0; i < n; ++i) launches += ps[i].channels > 0 ? (devptr ? 1 : 2) : 0;  // emits, band flags
   if (!devptr) launches += 1;  // the first tile count
 
@@ -475,6 +548,8 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
     if (e == cudaSuccess) e = cudaMemsetAsync(base + L.err, 0, sizeof(int), st);
     if (e == cudaSuccess) e = launch_assembly(P, pl.tc, st, any_warm);
     if (e == cudaSuccess) e = record(ctx->ev[1], capturing);
+    for (const ClusterClass &k : pl.classes)
+      if (e == cudaSuccess) e = launch_cluster(P, pl.tc, k, reinterpret_cast<const int *>(base + L.clist), st);
     if (e == cudaSuccess) e = launch_prepared(P, pl.cfg, grid, st);
     if (e == cudaSuccess) e = record(ctx->ev[2], capturing);
     for (uint32_t i = 0; i < n && e == cudaSuccess; ++i)

@@ -1,0 +1,71 @@
+"""The in-cluster SOR solve (rbsor_cluster.cu) against the tile kernel.
+
+A call of few values takes the cluster kernel; the same image beside a large
+one takes the tile kernel. Both run the same iteration with the same arithmetic
+a cell, so outputs and iteration counts agree bit for bit; the histories' sums of squares are taken in
+another order (n terms in FP64: a relative difference of at most n 2^-53, 1e-10
+for the largest region here)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from paintop_b200 import _lib
+    with _lib.Context(0) as c:
+        c.set_config(2)
+        yield c
+
+
+def _problem(seed, w, h, c, box):
+    rng = np.random.default_rng(seed)
+    src, tgt = rng.random((h, w, c), dtype=np.float32), rng.random((h, w, c), dtype=np.float32)
+    mask = np.zeros((h, w), np.float32)
+    x0, y0, x1, y1 = box
+    mask[y0:y1 + 1, x0:x1 + 1] = rng.random((y1 + 1 - y0, x1 + 1 - x0)) > 0.1
+    mask[y0, x0] = mask[y1, x1] = 1.0  # the region's bounding box is the box
+    return src.reshape(-1), tgt.reshape(-1), mask.reshape(-1)
+
+
+# (width, height, box): one cell; one row; a patch's edges in x and y; odd first
+# rows; blocks of 224 patches exactly full and one row more (two- and four-row
+# patches); 16 blocks; blocks of 480; an image too wide for any cluster
+CASES = [
+    (3, 3, (1, 1, 1, 1)), (40, 5, (1, 2, 38, 2)), (33, 17, (1, 1, 31, 15)), (34, 20, (8, 3, 15, 10)),
+    (64, 64, (7, 1, 16, 62)), (70, 66, (9, 5, 60, 64)), (250, 30, (1, 1, 248, 14)), (250, 30, (1, 1, 248, 15)),
+    (1800, 36, (1, 1, 1790, 33)), (1800, 36, (3, 2, 1780, 9)), (512, 300, (20, 11, 490, 285)), (700, 420, (1, 1, 698, 418)),
+    (4100, 60, (1, 1, 4098, 40)), (96, 1100, (3, 1, 90, 1090)),
+]
+
+
+@pytest.mark.parametrize("w,h,box", CASES)
+def test_cluster_matches_tiles(ctx, w, h, box):
+    c, cap = (3 if w * h < 40000 else 1), 60
+    src, tgt, mask = _problem(w + h, w, h, c, box)
+    p = dict(source=src, target=tgt, mask=mask, width=w, height=h, channels=c, lam=0.003 * (w % 3), tolerance=1e-7,
+             omega=1.7, max_iterations=cap if w % 2 else 400)
+    big = np.zeros(2048 * 2048, np.float32)
+    other = dict(source=big, target=big, mask=big, width=2048, height=2048, channels=1)
+    small = ctx.solve_batch([p], want_history=True)[0]
+    tiles = ctx.solve_batch([p, other], want_history=True)[0]
+    assert np.array_equal(small[0].view(np.uint32), tiles[0].view(np.uint32))
+    for a, b in zip(small[1], tiles[1]):
+        assert (a["iterations"], a["stop_reason"], a["refinements"]) == (b["iterations"], b["stop_reason"], b["refinements"])
+        np.testing.assert_allclose(a["residual_history"], b["residual_history"], rtol=1e-10)
+
+
+def test_cluster_batch_and_reruns(ctx):
+    """Regions of every class in one call, each as if solved alone, twice the same."""
+    probs = []
+    for k, (w, h, box) in enumerate(CASES[:11]):
+        src, tgt, mask = _problem(k, w, h, 1, box)
+        probs.append(dict(source=src, target=tgt, mask=mask, width=w, height=h, channels=1, lam=0.01 * (k % 2),
+                          tolerance=1e-6, omega=1.8, max_iterations=300))
+    first, again = (ctx.solve_batch(probs, want_history=True) for _ in range(2))
+    for p, a, b in zip(probs, first, again):
+        alone = ctx.solve_batch([p], want_history=True)[0]
+        for x in (b, alone):
+            assert np.array_equal(a[0].view(np.uint32), x[0].view(np.uint32))
+            assert [r["residual_history"] for r in a[1]] == [r["residual_history"] for r in x[1]]
