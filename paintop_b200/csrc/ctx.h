@@ -27,7 +27,7 @@ struct pt_ctx {
   bool graphs = true;          // capture device-pointer solves into a CUDA graph
   cudaGraphExec_t gexec = nullptr;
   std::string gkey;            // the plan the cached graph was captured for
-  cudaGraphExec_t mgexec[2] = {nullptr, nullptr};  // multigrid-CG iteration: first / later
+  cudaGraphExec_t mgexec[3] = {nullptr, nullptr, nullptr};  // multigrid-CG iteration: first / odd / even
   std::string mgkey;           // the problem shape and arena the multigrid graphs were captured for
   long long mgnodes = 0;       // kernels in one of those iterations
 

@@ -27,13 +27,12 @@
 // Batches: every problem of a call (pt_poisson_solve_batch) keeps its own
 // level hierarchy, its own CG scalars per channel and its own stopping, but
 // all of them share each launch. A launch walks a table of blocks, each block
-// one 32 x 8 tile of one instance's plane. The level-0 tiles, whose partial
-// sums are reduced, are laid out per instance exactly as a call with that
-// instance alone lays them out; every other kernel computes each cell from
-// values no other block of the launch writes, so its result does not depend
-// on the tiling. An instance's results are therefore bit for bit what it gets
-// when solved alone. An (instance, channel) pair whose run has stopped skips
-// the vector kernels and, in a call with several instances, the V-cycle.
+// a few strips (or one 32 x 8 tile) of one instance's plane. Sums are taken by
+// bands of rows of an instance's plane, whatever the strips; every other value
+// is computed from values no other block of the launch writes, so it does not
+// depend on them either. An instance's results are therefore bit for bit what
+// it gets when solved alone. An (instance, channel) pair whose run has stopped
+// skips the launches.
 //
 // Report (pt_report): iterations = preconditioned CG iterations (each one
 // V-cycle and one operator application); history[k] = relative residual after
@@ -58,40 +57,30 @@
 
 namespace {
 
-constexpr int kThreads = 256;
 constexpr double kInnerFloor = 2e-6;  // deepest relative reduction asked of one FP32 CG run
 
-__device__ __forceinline__ double block_sum(double v, double *sh) {
-  sh[threadIdx.x] = v;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
-  }
-  const double r = sh[0];
-  __syncthreads();
-  return r;
-}
-
-// Stencil and vector kernels run on tiles of (32, 8) threads over columns and
-// rows; a tile strides over the rows of its instance's plane, grid.z is the
-// channel. Kernels that reduce write one partial per tile and channel.
+// Assembly, coarsening and output run on tiles of (32, 8) threads over columns
+// and rows; a tile strides over the rows of its instance's plane. The other
+// kernels run on strips (below), grid.z is the channel.
 constexpr int kTx = 32, kTy = 8;
 
-// One instance's plane as one launch tiles it. The blocks of a launch are the
-// instances' tiles one after another; bmap[blockIdx.x] names the entry.
+// One instance's plane as one launch cuts it. The blocks of a launch are the
+// instances' tiles, or their strips kStripWarps a block, one after another;
+// bmap[blockIdx.x] names the entry. Rows are P apart, a multiple of four.
 struct Geo {
-  int W, H;           // the tiled plane (restriction: the coarse one)
-  int gx, gy;         // tiles: gx across W (a half-sweep: across (W + 1) / 2), gy striding the rows
+  int W, H, P;        // the plane (coarsening: the coarse one)
+  int gx, gy;         // tiles across and striding the rows; strip columns and strips down a column
+  int rows;           // rows of a strip, a multiple of kBand
   int blk0;           // the instance's first block in the launch
   int C;              // its channels
   int unit0;          // its first (instance, channel) unit: CG scalars, scales, run flags, reductions
   int pad;
-  long long part0;    // its first partial sum (level-0 reductions): C * gx * gy of them, channel-major
+  long long part0;    // its first partial sum: C times one a band and strip column of level 0, channel-major
+  long long f;        // its first band flag of the level
   long long o, oc;    // the plane's first cell in its level's one-channel (interior flags) and C-channel arrays
   long long o2, oc2;  // the same for the other plane of a two-level kernel
-  int W2, H2;         // that plane (restriction: the fine level; prolongation: the coarse level)
-  float s, d;         // the level's 4^-k and diagonal 4^(1-k) + lambda (restriction: the fine level's)
+  int W2, H2, P2;     // that plane (coarsening: the fine level; else: the coarse level)
+  float s, d;         // the level's 4^-k and diagonal 4^(1-k) + lambda
   double lambda;
 };
 
@@ -105,21 +94,8 @@ __device__ __forceinline__ int4 entry_of(const int4 *__restrict__ bmap, const Ge
 // Which tile of its instance a block works on
 __device__ __forceinline__ int tile_b(const Geo &g) { return (int)blockIdx.x - g.blk0; }
 
-__device__ __forceinline__ double block_sum2(double v, double *sh) {
-  const int t = threadIdx.y * kTx + threadIdx.x;
-  sh[t] = v;
-  __syncthreads();
-  for (int o = kTx * kTy / 2; o > 0; o >>= 1) {
-    if (t < o) sh[t] += sh[t + o];
-    __syncthreads();
-  }
-  const double r = sh[0];
-  __syncthreads();
-  return r;
-}
-
-// Per-unit CG scalars: sc[unit] = {rho, rho_new, pq, rr, alpha, beta}
-enum { S_RHO, S_RHO_NEW, S_PQ, S_RR, S_ALPHA, S_BETA, S_N };
+// Per-unit CG scalars: sc[unit] = {rho, beta, p.q}
+enum { S_RHO, S_BETA, S_PQ, S_N };
 
 // The caller-side buffers of one instance (device memory: the caller's, or
 // the staged copies of host buffers)
@@ -142,16 +118,20 @@ __global__ void __launch_bounds__(kTx * kTy) k_mg_assemble(const Geo *__restrict
   const Geo g = bmap ? geo[gi] : one;
   const Io f = io[gi];
   const int C = g.C, W = g.W, H = g.H, b = tile_b(g), i = (b % g.gx) * kTx + threadIdx.x;
-  const size_t N = (size_t)W * H;
+  const size_t N = (size_t)g.P * H;
   uint8_t *a = act + g.o;
   double *u0 = u + g.oc, *b0 = bl + g.oc, *w0 = uw ? uw + g.oc : nullptr;
-  for (int j = (b / g.gx) * kTy + threadIdx.y; j < H && i < W; j += g.gy * kTy) {
-    const size_t q = (size_t)j * W + i;
+  for (int j = (b / g.gx) * kTy + threadIdx.y; j < H && i < g.P; j += g.gy * kTy) {
+    const size_t k = (size_t)j * g.P + i, q = (size_t)j * W + i;
+    if (i >= W) {  // padding
+      a[k] = 0;
+      continue;
+    }
     const bool in = W >= 3 && H >= 3 && i > 0 && j > 0 && i < W - 1 && j < H - 1 && f.mask[q] > 0.5f;
-    a[q] = in ? 1 : 0;
+    a[k] = in ? 1 : 0;
     for (int c = 0; c < C; ++c) {  // a thread's channels are adjacent in the interleaved inputs
       const double av = (double)f.anchor[q * C + c];
-      u0[c * N + q] = av;
+      u0[c * N + k] = av;
       double bv = 0.0;
       if (in) {
         // poisson.rs:364-373: L, R, U, D, then fma(4, -centre, sum)
@@ -161,102 +141,9 @@ __global__ void __launch_bounds__(kTx * kTy) k_mg_assemble(const Geo *__restrict
                          (double)gd[(q + W) * C + c];
         bv = fma(4.0, -ctr, s);
       }
-      b0[c * N + q] = in ? fma(g.lambda, -av, bv) : 0.0;
-      if (w0) w0[c * N + q] = (in && f.guess) ? (double)f.guess[q * C + c] : av;
+      b0[c * N + k] = in ? fma(g.lambda, -av, bv) : 0.0;
+      if (w0) w0[c * N + k] = (in && f.guess) ? (double)f.guess[q * C + c] : av;
     }
-  }
-}
-
-// r = fma(lambda + 4, -u, nsum) - b' at interior cells (0 elsewhere) and
-// per-tile partial sums of r^2.
-__global__ void __launch_bounds__(kTx * kTy) k_mg_residual64(const Geo *__restrict__ geo,
-                                                             const int4 *__restrict__ bmap, const Geo one,
-                                                             const uint8_t *__restrict__ act,
-                                                             const double *__restrict__ u,
-                                                             const double *__restrict__ bl, double *__restrict__ r64,
-                                                             double *__restrict__ part) {
-  __shared__ double sh[kTx * kTy];
-  const int4 bt = entry_of(bmap, one);
-  const Geo g = bmap ? geo[bt.x] : one;
-  const int c = blockIdx.z;
-  if (c >= bt.z) return;
-  const int W = g.W, H = g.H, gx = g.gx, gy = g.gy, b = tile_b(g), i = (b % gx) * kTx + threadIdx.x;
-  const size_t N = (size_t)W * H;
-  const uint8_t *a = act + g.o;
-  const double *uc = u + g.oc + c * N, *bc = bl + g.oc + c * N;
-  double *rc = r64 + g.oc + c * N;
-  const double lambda = g.lambda;
-  double acc = 0.0;
-  for (int j = (b / gx) * kTy + threadIdx.y; j < H && i < W; j += gy * kTy) {
-    const size_t q = (size_t)j * W + i;
-    double r = 0.0;
-    if (a[q]) {
-      const double nsum = uc[q - 1] + uc[q + 1] + uc[q - W] + uc[q + W];  // L, R, U, D (poisson.rs:275-298)
-      r = fma(lambda + 4.0, -uc[q], nsum) - bc[q];
-    }
-    rc[q] = r;
-    acc += r * r;
-  }
-  const double t = block_sum2(acc, sh);
-  if (threadIdx.x == 0 && threadIdx.y == 0) part[g.part0 + (long long)c * gx * gy + b] = t;
-}
-
-// A unit's partial sums: part[start .. start + n - 1]
-struct Red {
-  long long start, n;
-};
-
-// out[unit * stride] = fixed-order sum of the unit's partials; grid (units)
-__global__ void k_mg_reduce(const double *__restrict__ part, const Red *__restrict__ rtab, double *__restrict__ out,
-                            int stride) {
-  __shared__ double sh[kThreads];
-  const Red rt = rtab[blockIdx.x];
-  double acc = 0.0;
-  for (long long k = threadIdx.x; k < rt.n; k += blockDim.x) acc += part[rt.start + k];
-  const double s = block_sum(acc, sh);
-  if (threadIdx.x == 0) out[(long long)blockIdx.x * stride] = s;
-}
-
-// r32 = r64 / scale[unit] (0 where the unit is not being corrected)
-__global__ void __launch_bounds__(kTx * kTy) k_mg_scale(const Geo *__restrict__ geo,
-                                                        const int4 *__restrict__ bmap, const Geo one,
-                                                        const double *__restrict__ r64,
-                                                        const double *__restrict__ scale, float *__restrict__ r32) {
-  const int4 bt = entry_of(bmap, one);
-  const Geo g = bmap ? geo[bt.x] : one;
-  const int c = blockIdx.z;
-  if (c >= bt.z) return;
-  const int W = g.W, H = g.H, b = tile_b(g), i = (b % g.gx) * kTx + threadIdx.x;
-  const size_t N = (size_t)W * H;
-  const double s = scale[g.unit0 + c];
-  const double *rc = r64 + g.oc + c * N;
-  float *oc = r32 + g.oc + c * N;
-  for (int j = (b / g.gx) * kTy + threadIdx.y; j < H && i < W; j += g.gy * kTy) {
-    const size_t q = (size_t)j * W + i;
-    oc[q] = s > 0.0 ? (float)(rc[q] / s) : 0.0f;
-  }
-}
-
-// u += scale[unit] * x at interior cells; a unit with scale 0 (not being
-// corrected) is left as it is, bit for bit
-__global__ void __launch_bounds__(kTx * kTy) k_mg_update(const Geo *__restrict__ geo,
-                                                         const int4 *__restrict__ bmap, const Geo one,
-                                                         const uint8_t *__restrict__ act, const float *__restrict__ x,
-                                                         const double *__restrict__ scale, double *__restrict__ u) {
-  const int4 bt = entry_of(bmap, one);
-  const Geo g = bmap ? geo[bt.x] : one;
-  const int c = blockIdx.z;
-  if (c >= bt.z) return;
-  const double s = scale[g.unit0 + c];
-  if (s == 0.0) return;
-  const int W = g.W, H = g.H, b = tile_b(g), i = (b % g.gx) * kTx + threadIdx.x;
-  const size_t N = (size_t)W * H;
-  const uint8_t *a = act + g.o;
-  const float *xc = x + g.oc + c * N;
-  double *uc = u + g.oc + c * N;
-  for (int j = (b / g.gx) * kTy + threadIdx.y; j < H && i < W; j += g.gy * kTy) {
-    const size_t q = (size_t)j * W + i;
-    if (a[q]) uc[q] = fma(s, (double)xc[q], uc[q]);
   }
 }
 
@@ -281,405 +168,865 @@ __global__ void __launch_bounds__(kTx * kTy) k_mg_coarsen(const Geo *__restrict_
                                                           const uint8_t *__restrict__ af, uint8_t *__restrict__ ac) {
   const int4 bt = entry_of(bmap, one);
   const Geo g = bmap ? geo[bt.x] : one;
-  const int Wc = g.W, Hc = g.H, Wf = g.W2, Hf = g.H2, b = tile_b(g), I = (b % g.gx) * kTx + threadIdx.x;
+  const int Hc = g.H, Wf = g.W2, Hf = g.H2, b = tile_b(g), I = (b % g.gx) * kTx + threadIdx.x;
   const uint8_t *f = af + g.o2;
   uint8_t *cc = ac + g.o;
-  for (int J = (b / g.gx) * kTy + threadIdx.y; J < Hc && I < Wc; J += g.gy * kTy) {
+  for (int J = (b / g.gx) * kTy + threadIdx.y; J < Hc && I < g.P; J += g.gy * kTy) {  // (padding: 0)
     int n = 0;
     for (int dy = 0; dy < 2; ++dy)
       for (int dx = 0; dx < 2; ++dx) {
         const int i = 2 * I + dx, j = 2 * J + dy;
-        if (i < Wf && j < Hf) n += f[(size_t)j * Wf + i];
+        if (i < Wf && j < Hf) n += f[(size_t)j * g.P2 + i];
       }
-    cc[(size_t)J * Wc + I] = n >= kCoarseRule ? 1 : 0;
+    cc[(size_t)J * g.P + I] = n >= kCoarseRule ? 1 : 0;
   }
 }
 
-// V-cycle kernels return at once for a unit whose run flag is 0 (run null:
-// no unit is skipped).
+// ---- strips --------------------------------------------------------------------
+// The level and vector kernels give each warp a strip: 128 columns of which it
+// owns 112 (the first and last strips of a row more: there is no halo outside
+// the image), four a lane, and `rows` rows that it walks downwards, keeping
+// the last few rows in registers; horizontal neighbours come by shuffles. One
+// pass down a level (k_mg_down) runs four half-sweeps, the residual and its
+// restriction as stages on consecutive rows, one pass up (k_mg_up) the
+// prolongation and four half-sweeps, so a level's arrays cross the memory
+// system once each way instead of once a half-sweep, and no barrier is needed.
+// What a strip computes in its halo again, the strips beside it compute alike:
+// a cell's value does not depend on the strips.
 //
-// One colour of red-black Gauss-Seidel on A_k e = rhs: e = (rhs + s * sum of
-// neighbours) / d at active cells of that colour (inactive cells hold 0).
-// x threads index the cells of one colour in a row (half-sweep tiles).
-__global__ void __launch_bounds__(kTx * kTy) k_mg_smooth(const Geo *__restrict__ geo,
-                                                         const int4 *__restrict__ bmap, const Geo one,
-                                                         const uint8_t *__restrict__ act,
-                                                         const float *__restrict__ rhs, float *__restrict__ e,
-                                                         const double *__restrict__ run, int color) {
-  const int4 bt = entry_of(bmap, one);
-  const Geo g = bmap ? geo[bt.x] : one;
-  const int c = blockIdx.z;
-  if (c >= bt.z || (run && run[bt.y + c] == 0.0)) return;
-  const int W = g.W, H = g.H, b = tile_b(g), m = (b % g.gx) * kTx + threadIdx.x;
-  const float s = g.s, d = g.d;
-  const size_t N = (size_t)W * H;
-  const uint8_t *a = act + g.o;
-  float *ec = e + g.oc + c * N;
-  const float *rc = rhs + g.oc + c * N;
-  // Two of the tile's rows per pass, both rows' loads before either update:
-  // the neighbours read are of the other colour, which this half-sweep does
-  // not write, so the two rows' accesses are independent and the loads of the
-  // second row need not wait for the first row's store.
-  const int step = g.gy * kTy;
-  for (int j0 = (b / g.gx) * kTy + threadIdx.y; j0 < H; j0 += 2 * step) {
-    const int j1 = j0 + step;
-    const int i0 = 2 * m + ((j0 + color) & 1), i1 = 2 * m + ((j1 + color) & 1);
-    const size_t q0 = (size_t)j0 * W + i0, q1 = (size_t)j1 * W + i1;
-    const bool v0 = i0 < W && a[q0];
-    const bool v1 = j1 < H && i1 < W && a[q1];
-    float nb0 = 0.0f, e0 = 0.0f, r0 = 0.0f, nb1 = 0.0f, e1 = 0.0f, r1 = 0.0f;
-    if (v0) {
-      if (i0 > 0) nb0 += ec[q0 - 1];
-      if (i0 < W - 1) nb0 += ec[q0 + 1];
-      if (j0 > 0) nb0 += ec[q0 - W];
-      if (j0 < H - 1) nb0 += ec[q0 + W];
-      e0 = ec[q0];
-      r0 = rc[q0];
-    }
-    if (v1) {
-      if (i1 > 0) nb1 += ec[q1 - 1];
-      if (i1 < W - 1) nb1 += ec[q1 + 1];
-      if (j1 > 0) nb1 += ec[q1 - W];
-      if (j1 < H - 1) nb1 += ec[q1 + W];
-      e1 = ec[q1];
-      r1 = rc[q1];
-    }
-    if (v0) {
-      const float gs = (r0 + s * nb0) / d;
-      ec[q0] = e0 + kSmoothOmega * (gs - e0);
-    }
-    if (v1) {
-      const float gs = (r1 + s * nb1) / d;
-      ec[q1] = e1 + kSmoothOmega * (gs - e1);
-    }
-  }
+// Rows are padded to a multiple of four cells (pitch P), so that a lane moves
+// 16 bytes at once. Strips are skipped by bands of kBand rows without an active
+// cell (flags, one byte a band and strip column): their cells are never
+// written, and whoever reads them masks them with the interior flags -- or
+// reads zero: a level's correction is cleared before the first V-cycle.
+//
+// Border cells are inactive on every level (a coarse border cell has at most
+// two active children), so neighbours outside the image, which the edge lanes
+// replace by their own values, are never used.
+constexpr int kStripCols = 128, kStripStep = 112, kStripHalo = 8;
+constexpr int kStripWarps = 4;   // per block
+constexpr int kBand = 8;
+
+__host__ __device__ inline int strip_cols(int w) {
+  return w <= kStripCols ? 1 : 1 + (w - kStripCols + kStripStep - 1) / kStripStep;
 }
 
-// The first half-sweep of a V-cycle level, from e = 0: e = rhs / d at active
-// cells of colour 0 (red), 0 everywhere else, relaxed by kSmoothOmega -- what
-// zeroing e and one red half-sweep produce, bit for bit, in one pass that
-// writes every cell.
-__global__ void __launch_bounds__(kTx * kTy) k_mg_smooth_first(const Geo *__restrict__ geo,
+struct Strip {
+  int x0;        // the lane's first column
+  int y0, y1;    // rows, trimmed to bands with active cells
+  int sx;        // strip column
+  bool in, own;  // the lane's columns are inside the pitch; owned
+};
+
+// The warp's strip; false if there is none or no active cell in it.
+__device__ __forceinline__ bool strip_of(const Geo &g, const uint8_t *__restrict__ flags, Strip &t) {
+  const int lane = threadIdx.x & 31, s = tile_b(g) * kStripWarps + (threadIdx.x >> 5);
+  t.sx = s % g.gx;
+  const int sy = s / g.gx, b0 = sy * (g.rows / kBand), nb = (g.H + kBand - 1) / kBand;
+  if (sy >= g.gy) return false;
+  const int b = b0 + lane;  // (rows / kBand <= 32)
+  const bool f = lane < g.rows / kBand && b < nb && flags[g.f + (long long)b * g.gx + t.sx];
+  const unsigned m = __ballot_sync(0xffffffffu, f);
+  if (!m) return false;
+  t.y0 = (b0 + __ffs(m) - 1) * kBand;
+  t.y1 = min(g.H, (b0 + 32 - __clz(m)) * kBand);
+  t.x0 = kStripStep * t.sx + 4 * lane;
+  t.in = t.x0 < g.P;
+  const int lo = t.sx ? kStripStep * t.sx + kStripHalo : 0;
+  const int hi = t.sx + 1 == g.gx ? g.P : kStripStep * (t.sx + 1) + kStripHalo;
+  t.own = t.x0 >= lo && t.x0 < hi;
+  return true;
+}
+
+__device__ __forceinline__ unsigned nibble(uint32_t c) {  // four flag bytes -> four bits
+  return (c & 1u) | ((c >> 7) & 2u) | ((c >> 14) & 4u) | ((c >> 21) & 8u);
+}
+
+// Bands with active cells: one warp a band and strip column (its owned cells).
+__global__ void __launch_bounds__(kStripWarps * 32) k_mg_flags(const Geo *__restrict__ geo,
                                                                const int4 *__restrict__ bmap, const Geo one,
                                                                const uint8_t *__restrict__ act,
-                                                               const float *__restrict__ rhs, float *__restrict__ e,
-                                                               const double *__restrict__ run) {
+                                                               uint8_t *__restrict__ flags) {
   const int4 bt = entry_of(bmap, one);
   const Geo g = bmap ? geo[bt.x] : one;
-  const int c = blockIdx.z;
-  if (c >= bt.z || (run && run[bt.y + c] == 0.0)) return;
-  const int W = g.W, H = g.H, b = tile_b(g), i = (b % g.gx) * kTx + threadIdx.x;
-  const float s = g.s, d = g.d;
-  const size_t N = (size_t)W * H;
-  const uint8_t *a = act + g.o;
-  float *ec = e + g.oc + c * N;
-  const float *rc = rhs + g.oc + c * N;
-  for (int j = (b / g.gx) * kTy + threadIdx.y; j < H && i < W; j += g.gy * kTy) {
-    const size_t q = (size_t)j * W + i;
-    const float gs = (rc[q] + s * 0.0f) / d;
-    ec[q] = (a[q] && ((i + j) & 1) == 0) ? 0.0f + kSmoothOmega * (gs - 0.0f) : 0.0f;
+  const int lane = threadIdx.x & 31, s = tile_b(g) * kStripWarps + (threadIdx.x >> 5);
+  const int sx = s % g.gx, b = s / g.gx;
+  if (b >= g.gy) return;
+  const int x0 = kStripStep * sx + 4 * lane;
+  const int lo = sx ? kStripStep * sx + kStripHalo : 0, hi = sx + 1 == g.gx ? g.P : kStripStep * (sx + 1) + kStripHalo;
+  uint32_t any = 0;
+  if (x0 >= lo && x0 < hi)
+    for (int y = b * kBand; y < min(g.H, (b + 1) * kBand); ++y)
+      any |= *reinterpret_cast<const uint32_t *>(act + g.o + (long long)y * g.P + x0);
+  const unsigned m = __ballot_sync(0xffffffffu, any != 0);
+  if (lane == 0) flags[g.f + (long long)b * g.gx + sx] = m != 0;
+}
+
+// A lane's four cells of a row
+struct Row {
+  float v[4];
+};
+__device__ __forceinline__ Row row0() { return Row{{0.f, 0.f, 0.f, 0.f}}; }
+__device__ __forceinline__ Row ld_row(const float *p) {
+  const float4 q = *reinterpret_cast<const float4 *>(p);
+  return Row{{q.x, q.y, q.z, q.w}};
+}
+__device__ __forceinline__ void st_row(float *p, const Row &r) {
+  *reinterpret_cast<float4 *>(p) = make_float4(r.v[0], r.v[1], r.v[2], r.v[3]);
+}
+__device__ __forceinline__ float from_left(float x) { return __shfl_up_sync(0xffffffffu, x, 1); }
+__device__ __forceinline__ float from_right(float x) { return __shfl_down_sync(0xffffffffu, x, 1); }
+
+// v / d. With POW2 d is a power of two (lambda 0) and the product with its
+// reciprocal is the quotient, bit for bit.
+template <bool POW2>
+__device__ __forceinline__ float over(float v, float d, float inv) {
+  return POW2 ? v * inv : v / d;
+}
+
+// Red-black SOR on A_k e = rhs at cells F, F + 2 of the row: gs = (rhs + s *
+// sum of neighbours) / d, e += kSmoothOmega (gs - e), at active cells (inactive
+// cells hold 0).
+template <bool POW2, int F>
+__device__ __forceinline__ void relax_row(Row &e, const Row &up, const Row &dn, const Row &r, unsigned a, float s,
+                                          float d, float inv) {
+  float l0, r0, l1, r1;
+  if (F == 0) {
+    l0 = from_left(e.v[3]); r0 = e.v[1]; l1 = e.v[1]; r1 = e.v[3];
+  } else {
+    l0 = e.v[0]; r0 = e.v[2]; l1 = e.v[2]; r1 = from_right(e.v[0]);
+  }
+  const float n0 = ((l0 + r0) + up.v[F]) + dn.v[F], n1 = ((l1 + r1) + up.v[F + 2]) + dn.v[F + 2];
+  const float g0 = over<POW2>(r.v[F] + s * n0, d, inv), g1 = over<POW2>(r.v[F + 2] + s * n1, d, inv);
+  if (a & (1u << F)) e.v[F] = e.v[F] + kSmoothOmega * (g0 - e.v[F]);
+  if (a & (4u << F)) e.v[F + 2] = e.v[F + 2] + kSmoothOmega * (g1 - e.v[F + 2]);
+}
+
+// The per-band partial sums (part[start ..], the same places for every kernel:
+// a band without active cells is never written and stays 0), the blocks that
+// have finished (cleared again by the last), and the CG scalars.
+struct Sums {
+  double *part;
+  unsigned *done;
+  double *sc;
+};
+
+// A band's sum: lanes by an xor butterfly.
+__device__ __forceinline__ void band_sum(const Geo &g, const Strip &t, int c, int lane, int j, double v,
+                                         double *__restrict__ part) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) {
+    const int nb = (g.H + kBand - 1) / kBand;
+    part[g.part0 + ((long long)c * nb + j / kBand) * g.gx + t.sx] = v;
   }
 }
 
-// The coarsest level (at most kCoarseMax cells): `sweeps` red-black sweeps,
-// then as many in reverse colour order, from e = 0, in shared memory; one
-// block per instance (blockIdx.x = its entry) and channel (blockIdx.z).
-constexpr int kCoarseMax = 64;
-
-__global__ void k_mg_coarse(const Geo *__restrict__ geo, const uint8_t *__restrict__ act,
-                            const float *__restrict__ rhs, float *__restrict__ e, const double *__restrict__ run,
-                            int sweeps) {
-  __shared__ float se[kCoarseMax], sr[kCoarseMax];
-  __shared__ uint8_t sa[kCoarseMax];
-  const Geo &g = geo[blockIdx.x];
-  const int c = blockIdx.z;
-  if (c >= g.C || (run && run[g.unit0 + c] == 0.0)) return;
-  const int W = g.W, H = g.H, n = W * H, t = threadIdx.x;
-  const float s = g.s, d = g.d;
-  const float *rc = rhs + g.oc + (long long)c * n;
-  float *ecp = e + g.oc + (long long)c * n;
-  if (t < n) {
-    se[t] = 0.0f;
-    sr[t] = rc[t];
-    sa[t] = act[g.o + t];
+// By every thread of a strip block: true in one thread of the last block of the
+// unit to finish, with the unit's sum, its partials taken in a fixed order
+// (thread t takes t, t + 128, ..., then a tree).
+__device__ __forceinline__ bool unit_sum(const Geo &g, int c, const Sums &s, double *out) {
+  constexpr int T = kStripWarps * 32;
+  __shared__ bool last;
+  __shared__ double sh[T];
+  const int tid = threadIdx.x;
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    const unsigned blocks = (unsigned)((g.gx * g.gy + kStripWarps - 1) / kStripWarps);
+    last = atomicAdd(s.done + g.unit0 + c, 1u) == blocks - 1u;
+    __threadfence();
   }
   __syncthreads();
-  const int j = t / max(W, 1), i = t - j * W;
-  for (int k = 0; k < 4 * sweeps; ++k) {
-    // colour order R, B (first half) then B, R (second half)
-    const int half = k / (2 * sweeps), step = k & 1;
-    const int color = half == 0 ? step : 1 - step;
-    float v = 0.0f;
-    const bool mine = t < n && sa[t] && ((i + j) & 1) == color;
-    if (mine) {
-      float nb = 0.0f;
-      if (i > 0) nb += se[t - 1];
-      if (i < W - 1) nb += se[t + 1];
-      if (j > 0) nb += se[t - W];
-      if (j < H - 1) nb += se[t + W];
-      v = (sr[t] + s * nb) / d;
-    }
-    __syncthreads();
-    if (mine) se[t] = v;
+  if (!last) return false;
+  const long long n = (long long)((g.H + kBand - 1) / kBand) * g.gx, p0 = g.part0 + c * n;
+  double acc = 0.0;
+  for (long long k = tid; k < n; k += T) acc += __ldcg(s.part + p0 + k);
+  sh[tid] = acc;
+  __syncthreads();
+  for (int o = T / 2; o > 0; o >>= 1) {
+    if (tid < o) sh[tid] += sh[tid + o];
     __syncthreads();
   }
-  if (t < n) ecp[t] = se[t];
+  if (tid != 0) return false;
+  s.done[g.unit0 + c] = 0;
+  *out = sh[0];
+  return true;
 }
 
-__device__ __forceinline__ float pw(int a) { return (a == 0 || a == 1) ? 0.75f : 0.25f; }  // a = fine - 2 * coarse
+__device__ __forceinline__ void new_rho(double *sc, double rho, int first) {
+  sc[S_BETA] = first || sc[S_RHO] == 0.0 ? 0.0 : rho / sc[S_RHO];
+  sc[S_RHO] = rho;
+}
 
-// The restriction of the level's residual, rhs_c(I, J) = sum over fine
-// (2I + a, 2J + b), a, b in -1..2, of wx wy res_f / 4 with res_f = rhs - A e at
-// active fine cells (0 elsewhere), evaluated on the fly so the residual is
-// never stored. Tiles of the coarse plane; the fine plane is the second.
-__global__ void __launch_bounds__(kTx * kTy) k_mg_resid_restrict(const Geo *__restrict__ geo,
+// ---- the FP64 residual and update ------------------------------------------------
+// r = fma(lambda + 4, -u, nsum) - b' at interior cells (0 elsewhere); ||r||^2.
+struct Row64 {
+  double v[4];
+};
+__device__ __forceinline__ Row64 ld_row64(const double *p) {
+  const double2 a = *reinterpret_cast<const double2 *>(p), b = *reinterpret_cast<const double2 *>(p + 2);
+  return Row64{{a.x, a.y, b.x, b.y}};
+}
+__device__ __forceinline__ void st_row64(double *p, const Row64 &r) {
+  *reinterpret_cast<double2 *>(p) = make_double2(r.v[0], r.v[1]);
+  *reinterpret_cast<double2 *>(p + 2) = make_double2(r.v[2], r.v[3]);
+}
+__global__ void __launch_bounds__(kStripWarps * 32) k_mg_residual64(const Geo *__restrict__ geo,
+                                                                    const int4 *__restrict__ bmap, const Geo one,
+                                                                    const uint8_t *__restrict__ flags,
+                                                                    const uint8_t *__restrict__ act,
+                                                                    const double *__restrict__ u,
+                                                                    const double *__restrict__ bl,
+                                                                    double *__restrict__ r64, Sums sums,
+                                                                    double *__restrict__ rr) {
+  const int4 bt = entry_of(bmap, one);
+  const int c = blockIdx.z, lane = threadIdx.x & 31;
+  if (c >= bt.z) return;
+  const Geo g = bmap ? geo[bt.x] : one;
+  Strip t;
+  if (strip_of(g, flags, t)) {
+    const long long at = g.oc + (long long)c * g.P * g.H + t.x0;
+    const double lambda = g.lambda;
+    auto fetch = [&](int y) { return t.in && y >= 0 && y < g.H ? ld_row64(u + at + (long long)y * g.P) : Row64{}; };
+    Row64 m = fetch(t.y0 - 1), k = fetch(t.y0), n = fetch(t.y0 + 1);
+    double acc = 0.0;
+    for (int j = t.y0; j < t.y1; ++j) {
+      const Row64 next = fetch(j + 2);
+      const double l = __shfl_up_sync(0xffffffffu, k.v[3], 1), r = __shfl_down_sync(0xffffffffu, k.v[0], 1);
+      if (t.own) {
+        const unsigned a = nibble(*reinterpret_cast<const uint32_t *>(act + g.o + (long long)j * g.P + t.x0));
+        const Row64 b = ld_row64(bl + at + (long long)j * g.P);
+        Row64 res;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          // L, R, U, D (poisson.rs:275-298)
+          const double nsum = (((i ? k.v[i ? i - 1 : 0] : l) + (i < 3 ? k.v[i < 3 ? i + 1 : 3] : r)) + m.v[i]) + n.v[i];
+          res.v[i] = a & (1u << i) ? fma(lambda + 4.0, -k.v[i], nsum) - b.v[i] : 0.0;
+          acc += res.v[i] * res.v[i];
+        }
+        st_row64(r64 + at + (long long)j * g.P, res);
+      }
+      if ((j & (kBand - 1)) == kBand - 1 || j == t.y1 - 1) {
+        band_sum(g, t, c, lane, j, acc, sums.part);
+        acc = 0.0;
+      }
+      m = k;
+      k = n;
+      n = next;
+    }
+  }
+  double v;
+  if (unit_sum(g, c, sums, &v)) rr[g.unit0 + c] = v;
+}
+
+// r32 = r64 / scale[unit], x = 0; a unit that is not being corrected (scale 0) is left
+__global__ void __launch_bounds__(kStripWarps * 32) k_mg_scale(const Geo *__restrict__ geo,
+                                                               const int4 *__restrict__ bmap, const Geo one,
+                                                               const uint8_t *__restrict__ flags,
+                                                               const double *__restrict__ r64,
+                                                               const double *__restrict__ scale, float *__restrict__ r32,
+                                                               float *__restrict__ x) {
+  const int4 bt = entry_of(bmap, one);
+  const int c = blockIdx.z;
+  if (c >= bt.z) return;
+  const Geo g = bmap ? geo[bt.x] : one;
+  const double s = scale[g.unit0 + c];
+  if (!(s > 0.0)) return;
+  Strip t;
+  if (!strip_of(g, flags, t) || !t.own) return;
+  const long long at = g.oc + (long long)c * g.P * g.H + t.x0;
+#pragma unroll 4
+  for (int j = t.y0; j < t.y1; ++j) {
+    const long long o = at + (long long)j * g.P;
+    const Row64 r = ld_row64(r64 + o);
+    Row v;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v.v[i] = (float)(r.v[i] / s);
+    st_row(r32 + o, v);
+    st_row(x + o, row0());
+  }
+}
+
+// u += scale[unit] * x at interior cells; a unit with scale 0 (not being
+// corrected) is left as it is, bit for bit. x null: 0.
+__global__ void __launch_bounds__(kStripWarps * 32) k_mg_update(const Geo *__restrict__ geo,
+                                                                const int4 *__restrict__ bmap, const Geo one,
+                                                                const uint8_t *__restrict__ flags,
+                                                                const uint8_t *__restrict__ act,
+                                                                const float *__restrict__ x,
+                                                                const double *__restrict__ scale,
+                                                                double *__restrict__ u) {
+  const int4 bt = entry_of(bmap, one);
+  const int c = blockIdx.z;
+  if (c >= bt.z) return;
+  const Geo g = bmap ? geo[bt.x] : one;
+  const double s = scale[g.unit0 + c];
+  if (s == 0.0) return;
+  Strip t;
+  if (!strip_of(g, flags, t) || !t.own) return;
+  const long long at = g.oc + (long long)c * g.P * g.H + t.x0;
+#pragma unroll 4
+  for (int j = t.y0; j < t.y1; ++j) {
+    const long long o = at + (long long)j * g.P;
+    const unsigned a = nibble(*reinterpret_cast<const uint32_t *>(act + g.o + (long long)j * g.P + t.x0));
+    if (!a) continue;
+    const Row v = x ? ld_row(x + o) : row0();
+    Row64 w = ld_row64(u + o);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (a & (1u << i)) w.v[i] = fma(s, (double)v.v[i], w.v[i]);
+    st_row64(u + o, w);
+  }
+}
+
+// ---- the V-cycle -----------------------------------------------------------------
+// The products' roundings, spelled out: the residual and the prolongation are
+// the same bit for bit wherever they are evaluated.
+__device__ __forceinline__ float level_residual(float rhs, float d, float e, float s, float nb) {
+  return rhs - fmaf(d, e, -(s * nb));
+}
+// row + weight * x of a restriction's row sum, two roundings
+__device__ __forceinline__ float add_weighted(float row, float weight, float x) {
+  return __fadd_rn(row, __fmul_rn(weight, x));
+}
+// e(I0, J0), e(I1, J0), e(I0, J1), e(I1, J1): weights 9, 3, 3, 1 sixteenths
+__device__ __forceinline__ float bilinear(float a, float b, float c, float d) {
+  return fmaf(0.0625f, d, fmaf(0.1875f, b + c, 0.5625f * a));
+}
+
+// V-cycle kernels return at once for a unit whose run flag is 0.
+//
+// Down one level: from e = 0 the half-sweeps red, black, red, black, then the
+// restriction of the residual, rhs_c(I, J) = sum over fine (2I + a, 2J + b), a,
+// b in -1..2, of wx wy res / 4 (weights 1/4, 3/4, 3/4, 1/4; res = rhs - A e at
+// active cells, 0 elsewhere). Row y comes in as rows y - 1, y - 2, y - 3 get
+// their later half-sweeps, row y - 4 its residual.
+template <bool POW2>
+__device__ __forceinline__ void mg_down(const Geo &g, const Strip &t, int c, const uint8_t *__restrict__ act,
+                                        const float *__restrict__ rhs, float *__restrict__ e,
+                                        const uint8_t *__restrict__ actc, float *__restrict__ rhsc) {
+  const long long N = (long long)g.P * g.H, Nc = (long long)g.P2 * g.H2;
+  const uint8_t *a0 = act + g.o + t.x0;
+  const float *r0 = rhs + g.oc + c * N + t.x0;
+  float *e0 = e + g.oc + c * N + t.x0;
+  const int I = t.x0 >> 1;
+  const uint8_t *ca = actc + g.o2 + I;
+  float *rc = rhsc + g.oc2 + c * Nc + I;
+  const float s = g.s, d = g.d, inv = 1.0f / d;
+  const int J0 = t.y0 >> 1, J1 = (t.y1 + 1) >> 1, last = 2 * J1 + 4;
+  Row E[6], R[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) E[k] = R[k] = row0();
+  unsigned a = 0;  // active bits, the newest row's lowest
+  float vp0 = 0.f, vp1 = 0.f, vn0 = 0.f, vn1 = 0.f;
+  // the next two rows are on their way (rows after `last` are walked in vain)
+  const int y0 = t.y0 - 6;
+  auto fetch_r = [&](int y) { return t.in && y >= 0 && y < g.H ? ld_row(r0 + (long long)y * g.P) : row0(); };
+  auto fetch_a = [&](int y) {
+    return t.in && y >= 0 && y < g.H ? *reinterpret_cast<const uint32_t *>(a0 + (long long)y * g.P) : 0u;
+  };
+  Row pr0 = fetch_r(y0), pr1 = fetch_r(y0 + 1);
+  uint32_t pa0 = fetch_a(y0), pa1 = fetch_a(y0 + 1);
+  for (int yb = y0; yb <= last; yb += 6) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int y = yb + k;
+      constexpr auto at = [](int k, int i) { return (k + 6 - i) % 6; };
+      const int par = k & 1;  // y0 is even
+      R[k] = pr0;
+      a = (a << 4) | nibble(pa0);
+      pr0 = pr1; pa0 = pa1;
+      pr1 = fetch_r(y + 2); pa1 = fetch_a(y + 2);
+      Row &E0 = E[k], &E1 = E[at(k, 1)], &E2 = E[at(k, 2)], &E3 = E[at(k, 3)], &E4 = E[at(k, 4)], &E5 = E[at(k, 5)];
+      // red of row y from e = 0; black 0
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        E0.v[i] = ((i + par) & 1) == 0 && (a & (1u << i)) ? kSmoothOmega * over<POW2>(R[k].v[i], d, inv) : 0.0f;
+      if (par == 0) {  // rows y - 1 and y - 3 are odd, row y - 2 is even
+        relax_row<POW2, 0>(E1, E2, E0, R[at(k, 1)], a >> 4, s, d, inv);
+        relax_row<POW2, 0>(E2, E3, E1, R[at(k, 2)], a >> 8, s, d, inv);
+        relax_row<POW2, 0>(E3, E4, E2, R[at(k, 3)], a >> 12, s, d, inv);
+      } else {
+        relax_row<POW2, 1>(E1, E2, E0, R[at(k, 1)], a >> 4, s, d, inv);
+        relax_row<POW2, 1>(E2, E3, E1, R[at(k, 2)], a >> 8, s, d, inv);
+        relax_row<POW2, 1>(E3, E4, E2, R[at(k, 3)], a >> 12, s, d, inv);
+      }
+      if (t.own && y - 3 >= t.y0 && y - 3 < t.y1) st_row(e0 + (long long)(y - 3) * g.P, E3);
+      // residual of row j = y - 4
+      const int j = y - 4;
+      const float el = from_left(E4.v[3]), er = from_right(E4.v[0]);
+      float res[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float l = i ? E4.v[i ? i - 1 : 0] : el, r = i < 3 ? E4.v[i < 3 ? i + 1 : 3] : er;
+        const float nb = ((l + r) + E5.v[i]) + E3.v[i];
+        const float v = level_residual(R[at(k, 4)].v[i], d, E4.v[i], s, nb);
+        res[i] = (a >> 16) & (1u << i) ? v : 0.0f;
+      }
+      const float rl = from_left(res[3]), rr = from_right(res[0]);
+      float w0 = 0.25f * rl, w1 = 0.25f * res[1];
+      w0 = add_weighted(w0, 0.75f, res[0]); w1 = add_weighted(w1, 0.75f, res[2]);
+      w0 = add_weighted(w0, 0.75f, res[1]); w1 = add_weighted(w1, 0.75f, res[3]);
+      w0 = add_weighted(w0, 0.25f, res[2]); w1 = add_weighted(w1, 0.25f, rr);
+      if (par) {  // j = 2 J - 1
+        vp0 = fmaf(0.75f, w0, vp0); vp1 = fmaf(0.75f, w1, vp1);
+        vn0 = 0.25f * w0; vn1 = 0.25f * w1;
+      } else {    // j = 2 J: coarse row J - 1 is complete
+        vn0 = fmaf(0.75f, w0, vn0); vn1 = fmaf(0.75f, w1, vn1);
+        vp0 = fmaf(0.25f, w0, vp0); vp1 = fmaf(0.25f, w1, vp1);
+        const int J = (j >> 1) - 1;
+        if (t.own && I < g.P2 && J >= J0 && J < J1) {
+          const uchar2 q = *reinterpret_cast<const uchar2 *>(ca + (long long)J * g.P2);
+          *reinterpret_cast<float2 *>(rc + (long long)J * g.P2) = make_float2(q.x ? vp0 * 0.25f : 0.0f, q.y ? vp1 * 0.25f : 0.0f);
+        }
+        vp0 = vn0; vp1 = vn1;
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kStripWarps * 32, 4) k_mg_down(const Geo *__restrict__ geo,
                                                                  const int4 *__restrict__ bmap, const Geo one,
-                                                                 const uint8_t *__restrict__ af,
-                                                                 const float *__restrict__ rhsf,
-                                                                 const float *__restrict__ ef,
-                                                                 const uint8_t *__restrict__ ac,
+                                                                 const uint8_t *__restrict__ flags,
+                                                                 const uint8_t *__restrict__ act,
+                                                                 const float *__restrict__ rhs, float *__restrict__ e,
+                                                                 const uint8_t *__restrict__ actc,
                                                                  float *__restrict__ rhsc,
                                                                  const double *__restrict__ run) {
   const int4 bt = entry_of(bmap, one);
-  const Geo g = bmap ? geo[bt.x] : one;
-  const int c = blockIdx.z;
-  if (c >= bt.z || (run && run[bt.y + c] == 0.0)) return;
-  const int Wc = g.W, Hc = g.H, Wf = g.W2, Hf = g.H2, b = tile_b(g), I = (b % g.gx) * kTx + threadIdx.x;
-  const float s = g.s, d = g.d;
-  const size_t Nc = (size_t)Wc * Hc, Nf = (size_t)Wf * Hf;
-  const float *e = ef + g.oc2 + c * Nf, *rh = rhsf + g.oc2 + c * Nf;
-  const uint8_t *fa = af + g.o2, *ca = ac + g.o;
-  float *out = rhsc + g.oc + c * Nc;
-  for (int J = (b / g.gx) * kTy + threadIdx.y; J < Hc && I < Wc; J += g.gy * kTy) {
-    const size_t q = (size_t)J * Wc + I;
-    float v = 0.0f;
-    if (ca[q]) {
-      for (int bb = -1; bb <= 2; ++bb) {
-        const int j = 2 * J + bb;
-        if (j < 0 || j >= Hf) continue;
-        float row = 0.0f;
-        for (int aa = -1; aa <= 2; ++aa) {
-          const int i = 2 * I + aa;
-          if (i < 0 || i >= Wf) continue;
-          const size_t f = (size_t)j * Wf + i;
-          float r = 0.0f;
-          if (fa[f]) {
-            float nb = 0.0f;
-            if (i > 0) nb += e[f - 1];
-            if (i < Wf - 1) nb += e[f + 1];
-            if (j > 0) nb += e[f - Wf];
-            if (j < Hf - 1) nb += e[f + Wf];
-            r = rh[f] - (d * e[f] - s * nb);
-          }
-          row += pw(aa) * r;
-        }
-        v += pw(bb) * row;
-      }
-      v *= 0.25f;
-    }
-    out[q] = v;
-  }
-}
-
-// e_f += bilinear prolongation of e_c at active fine cells; tiles of the fine
-// plane, the coarse plane is the second.
-__global__ void __launch_bounds__(kTx * kTy) k_mg_prolong(const Geo *__restrict__ geo,
-                                                          const int4 *__restrict__ bmap, const Geo one,
-                                                          const uint8_t *__restrict__ af, float *__restrict__ ef,
-                                                          const float *__restrict__ ec,
-                                                          const double *__restrict__ run) {
-  const int4 bt = entry_of(bmap, one);
-  const Geo g = bmap ? geo[bt.x] : one;
-  const int c = blockIdx.z;
-  if (c >= bt.z || (run && run[bt.y + c] == 0.0)) return;
-  const int Wf = g.W, Hf = g.H, Wc = g.W2, Hc = g.H2, b = tile_b(g), i = (b % g.gx) * kTx + threadIdx.x;
-  const size_t Nc = (size_t)Wc * Hc, Nf = (size_t)Wf * Hf;
-  const float *e = ec + g.oc2 + c * Nc;
-  float *out = ef + g.oc + c * Nf;
-  const uint8_t *fa = af + g.o;
-  for (int j = (b / g.gx) * kTy + threadIdx.y; j < Hf && i < Wf; j += g.gy * kTy) {
-    const size_t q = (size_t)j * Wf + i;
-    if (!fa[q]) continue;
-    const int I0 = i >> 1, J0 = j >> 1;
-    const int I1 = (i & 1) ? I0 + 1 : I0 - 1, J1 = (j & 1) ? J0 + 1 : J0 - 1;
-    auto at = [&](int I, int J) -> float {
-      return (I >= 0 && I < Wc && J >= 0 && J < Hc) ? e[(size_t)J * Wc + I] : 0.0f;
-    };
-    const float v = 0.5625f * at(I0, J0) + 0.1875f * (at(I1, J0) + at(I0, J1)) + 0.0625f * at(I1, J1);
-    out[q] += v;
-  }
-}
-
-// ---- conjugate gradients (level-0 tiles) ---------------------------------------
-__device__ __forceinline__ void zero_partial(const Geo &g, int c, double *part) {
-  if (threadIdx.x == 0 && threadIdx.y == 0) part[g.part0 + (long long)c * g.gx * g.gy + tile_b(g)] = 0.0;
-}
-
-// q = A_0 p at active cells; partial sums of p.q
-__global__ void __launch_bounds__(kTx * kTy) k_cg_apply(const Geo *__restrict__ geo,
-                                                        const int4 *__restrict__ bmap, const Geo one,
-                                                        const uint8_t *__restrict__ act, const float *__restrict__ p,
-                                                        float *__restrict__ q, double *__restrict__ part,
-                                                        const double *__restrict__ run) {
-  __shared__ double sh[kTx * kTy];
-  const int4 bt = entry_of(bmap, one);
-  const Geo g = bmap ? geo[bt.x] : one;
-  const int c = blockIdx.z;
-  if (c >= bt.z) return;
-  if (run[bt.y + c] == 0.0) {  // a stopped unit: its p.q is never read
-    zero_partial(g, c, part);
-    return;
-  }
-  const int W = g.W, H = g.H, gx = g.gx, gy = g.gy, b = tile_b(g), i = (b % gx) * kTx + threadIdx.x;
-  const float d = g.d;
-  const size_t N = (size_t)W * H;
-  const uint8_t *a = act + g.o;
-  const float *pc = p + g.oc + c * N;
-  float *qc = q + g.oc + c * N;
-  double acc = 0.0;
-  // two of the tile's rows per pass, loads before stores (as in k_mg_smooth);
-  // the partial sum still takes the rows in order
-  const int step = gy * kTy;
-  for (int j0 = (b / gx) * kTy + threadIdx.y; j0 < H && i < W; j0 += 2 * step) {
-    const bool two = j0 + step < H;
-    const size_t k0 = (size_t)j0 * W + i, k1 = k0 + (size_t)step * W;
-    const bool a0 = a[k0] != 0, a1 = two && a[k1] != 0;
-    // interior cells are never on the border: all four neighbours exist
-    float c0 = 0.0f, s0 = 0.0f, c1 = 0.0f, s1 = 0.0f;
-    if (a0) {
-      c0 = pc[k0];
-      s0 = pc[k0 - 1] + pc[k0 + 1] + pc[k0 - W] + pc[k0 + W];
-    }
-    if (a1) {
-      c1 = pc[k1];
-      s1 = pc[k1 - 1] + pc[k1 + 1] + pc[k1 - W] + pc[k1 + W];
-    }
-    float v0 = 0.0f, v1 = 0.0f;
-    if (a0) {
-      v0 = d * c0 - s0;
-      acc += (double)c0 * (double)v0;
-    }
-    if (a1) {
-      v1 = d * c1 - s1;
-      acc += (double)c1 * (double)v1;
-    }
-    qc[k0] = v0;
-    if (two) qc[k1] = v1;
-  }
-  const double t = block_sum2(acc, sh);
-  if (threadIdx.x == 0 && threadIdx.y == 0) part[g.part0 + (long long)c * gx * gy + b] = t;
-}
-
-// partial sums of a.b
-__global__ void __launch_bounds__(kTx * kTy) k_cg_dot(const Geo *__restrict__ geo,
-                                                      const int4 *__restrict__ bmap, const Geo one,
-                                                      const float *__restrict__ x, const float *__restrict__ y,
-                                                      double *__restrict__ part, const double *__restrict__ run) {
-  __shared__ double sh[kTx * kTy];
-  const int4 bt = entry_of(bmap, one);
-  const Geo g = bmap ? geo[bt.x] : one;
-  const int c = blockIdx.z;
-  if (c >= bt.z) return;
-  if (run[bt.y + c] == 0.0) {  // a stopped unit: its rho is never read
-    zero_partial(g, c, part);
-    return;
-  }
-  const int W = g.W, H = g.H, gx = g.gx, gy = g.gy, b = tile_b(g), i = (b % gx) * kTx + threadIdx.x;
-  const size_t N = (size_t)W * H;
-  const float *xc = x + g.oc + c * N, *yc = y + g.oc + c * N;
-  double acc = 0.0;
-  const int step = gy * kTy;
-  for (int j0 = (b / gx) * kTy + threadIdx.y; j0 < H && i < W; j0 += 2 * step) {
-    const bool two = j0 + step < H;
-    const size_t o0 = (size_t)j0 * W + i, o1 = o0 + (size_t)step * W;
-    const float x0 = xc[o0], y0 = yc[o0];
-    const float x1 = two ? xc[o1] : 0.0f, y1 = two ? yc[o1] : 0.0f;
-    acc += (double)x0 * (double)y0;
-    if (two) acc += (double)x1 * (double)y1;
-  }
-  const double t = block_sum2(acc, sh);
-  if (threadIdx.x == 0 && threadIdx.y == 0) part[g.part0 + (long long)c * gx * gy + b] = t;
-}
-
-// p = z + beta p (beta = rho_new / rho; p = z on the first iteration)
-__global__ void __launch_bounds__(kTx * kTy) k_cg_direction(const Geo *__restrict__ geo,
-                                                            const int4 *__restrict__ bmap, const Geo one,
-                                                            const float *__restrict__ z, float *__restrict__ p,
-                                                            const double *__restrict__ sc,
-                                                            const double *__restrict__ run, int first) {
-  const int4 bt = entry_of(bmap, one);
-  const Geo g = bmap ? geo[bt.x] : one;
   const int c = blockIdx.z;
   if (c >= bt.z || run[bt.y + c] == 0.0) return;
-  const double *s = sc + (long long)(g.unit0 + c) * S_N;
-  const float beta = first ? 0.0f : (float)(s[S_RHO] != 0.0 ? s[S_RHO_NEW] / s[S_RHO] : 0.0);
-  const int W = g.W, H = g.H, b = tile_b(g), i = (b % g.gx) * kTx + threadIdx.x;
-  const size_t N = (size_t)W * H;
-  const float *zc = z + g.oc + c * N;
-  float *pc = p + g.oc + c * N;
-  // first: p is not read (it holds what the arena held); two rows per pass,
-  // loads before stores
-  const int step = g.gy * kTy;
-  for (int j0 = (b / g.gx) * kTy + threadIdx.y; j0 < H && i < W; j0 += 2 * step) {
-    const bool two = j0 + step < H;
-    const size_t o0 = (size_t)j0 * W + i, o1 = o0 + (size_t)step * W;
-    const float z0 = zc[o0], z1 = two ? zc[o1] : 0.0f;
-    const float p0 = first ? 0.0f : pc[o0], p1 = (first || !two) ? 0.0f : pc[o1];
-    pc[o0] = first ? z0 : z0 + beta * p0;
-    if (two) pc[o1] = first ? z1 : z1 + beta * p1;
-  }
-}
-
-__global__ void k_cg_scalars_after_dir(int U, double *__restrict__ sc) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < U; k += gridDim.x * blockDim.x)
-    sc[(long long)k * S_N + S_RHO] = sc[(long long)k * S_N + S_RHO_NEW];
-}
-
-// x += alpha p, r -= alpha q (alpha = rho / p.q); partial sums of r.r
-__global__ void __launch_bounds__(kTx * kTy) k_cg_step(const Geo *__restrict__ geo,
-                                                       const int4 *__restrict__ bmap, const Geo one,
-                                                       const float *__restrict__ p, const float *__restrict__ q,
-                                                       float *__restrict__ x, float *__restrict__ r,
-                                                       const double *__restrict__ sc, double *__restrict__ part,
-                                                       const double *__restrict__ run) {
-  __shared__ double sh[kTx * kTy];
-  const int4 bt = entry_of(bmap, one);
   const Geo g = bmap ? geo[bt.x] : one;
-  const int c = blockIdx.z;
-  if (c >= bt.z) return;
-  if (run[bt.y + c] == 0.0) {  // a stopped unit: x and r stay (p may never have been written)
-    zero_partial(g, c, part);
-    return;
-  }
-  const double *s = sc + (long long)(g.unit0 + c) * S_N;
-  const float alpha = s[S_PQ] > 0.0 ? (float)(s[S_RHO] / s[S_PQ]) : 0.0f;
-  const int W = g.W, H = g.H, gx = g.gx, gy = g.gy, b = tile_b(g), i = (b % gx) * kTx + threadIdx.x;
-  const size_t N = (size_t)W * H;
-  const float *pc = p + g.oc + c * N, *qc = q + g.oc + c * N;
-  float *xc = x + g.oc + c * N, *rc = r + g.oc + c * N;
+  Strip t;
+  if (!strip_of(g, flags, t)) return;
+  if (g.lambda == 0.0) mg_down<true>(g, t, c, act, rhs, e, actc, rhsc);
+  else mg_down<false>(g, t, c, act, rhs, e, actc, rhsc);
+}
+
+// Up one level: e += the bilinear prolongation of the coarse correction at
+// active cells, then the half-sweeps black, red, black, red; the result goes
+// to another array (the strips beside read e). DOT: also the partial sums of
+// rhs . result, one a band and strip column.
+template <bool POW2, bool DOT>
+__device__ __forceinline__ void mg_up(const Geo &g, const Strip &t, int c, const uint8_t *__restrict__ act,
+                                      const float *__restrict__ rhs, const float *__restrict__ e,
+                                      const float *__restrict__ ec, float *__restrict__ out,
+                                      double *__restrict__ part) {
+  const int lane = threadIdx.x & 31;
+  const long long N = (long long)g.P * g.H, Nc = (long long)g.P2 * g.H2;
+  const uint8_t *a0 = act + g.o + t.x0;
+  const float *r0 = rhs + g.oc + c * N + t.x0, *e0 = e + g.oc + c * N + t.x0;
+  float *o0 = out + g.oc + c * N + t.x0;
+  const int I = t.x0 >> 1;
+  const float *c0 = ec + g.oc2 + c * Nc + I;
+  const float s = g.s, d = g.d, inv = 1.0f / d;
+  const int last = t.y1 + 3;
+  Row E[6], R[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) E[k] = R[k] = row0();
+  unsigned a = 0;
   double acc = 0.0;
-  const int step = gy * kTy;  // two rows per pass, loads before stores
-  for (int j0 = (b / gx) * kTy + threadIdx.y; j0 < H && i < W; j0 += 2 * step) {
-    const bool two = j0 + step < H;
-    const size_t o0 = (size_t)j0 * W + i, o1 = o0 + (size_t)step * W;
-    const float p0 = pc[o0], q0 = qc[o0], x0 = xc[o0], r0 = rc[o0];
-    float p1 = 0.0f, q1 = 0.0f, x1 = 0.0f, r1 = 0.0f;
-    if (two) {
-      p1 = pc[o1]; q1 = qc[o1]; x1 = xc[o1]; r1 = rc[o1];
-    }
-    xc[o0] = x0 + alpha * p0;
-    const float rv0 = r0 - alpha * q0;
-    rc[o0] = rv0;
-    acc += (double)rv0 * (double)rv0;
-    if (two) {
-      xc[o1] = x1 + alpha * p1;
-      const float rv1 = r1 - alpha * q1;
-      rc[o1] = rv1;
-      acc += (double)rv1 * (double)rv1;
+  const int y0 = t.y0 - 4;
+  auto fetch = [&](const float *p, int y) { return t.in && y >= 0 && y < g.H ? ld_row(p + (long long)y * g.P) : row0(); };
+  auto fetch_a = [&](int y) {
+    return t.in && y >= 0 && y < g.H ? *reinterpret_cast<const uint32_t *>(a0 + (long long)y * g.P) : 0u;
+  };
+  auto fetch_c = [&](int J) {
+    return I < g.P2 && J >= 0 && J < g.H2 ? *reinterpret_cast<const float2 *>(c0 + (long long)J * g.P2) : make_float2(0.f, 0.f);
+  };
+  // four coarse values a row around the lane's four cells: columns I - 1 .. I + 2
+  auto wide = [&](float2 v) { return Row{{from_left(v.y), v.x, v.y, from_right(v.x)}}; };
+  Row pe0 = fetch(e0, y0), pr0 = fetch(r0, y0);
+  uint32_t pa0 = fetch_a(y0);
+  Row pe1 = fetch(e0, y0 + 1), pr1 = fetch(r0, y0 + 1);
+  uint32_t pa1 = fetch_a(y0 + 1);
+  // coarse rows J - 1, J (J = y / 2), and J + 1 on its way
+  Row cm = wide(fetch_c((y0 >> 1) - 1)), cj = wide(fetch_c(y0 >> 1));
+  float2 cn = fetch_c((y0 >> 1) + 1);
+  for (int yb = y0; yb <= last; yb += 6) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int y = yb + k;
+      constexpr auto at = [](int k, int i) { return (k + 6 - i) % 6; };
+      const int par = k & 1;  // y0 is even
+      Row &E0 = E[k], &E1 = E[at(k, 1)], &E2 = E[at(k, 2)], &E3 = E[at(k, 3)], &E4 = E[at(k, 4)], &E5 = E[at(k, 5)];
+      R[k] = pr0;
+      a = (a << 4) | nibble(pa0);
+      Row near;
+      if (par == 0) {
+        near = cm;
+      } else {
+        near = wide(cn);
+        cm = cj;
+        // (cj moves on after this row)
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        // columns: I0 = i / 2 (index 1 + i / 2), I1 beside it
+        const int m0 = 1 + (i >> 1), m1 = (i & 1) ? m0 + 1 : m0 - 1;
+        const Row &rj = par == 0 ? cj : cm;  // row J (cm holds it after the move)
+        const float v = bilinear(rj.v[m0], rj.v[m1], near.v[m0], near.v[m1]);
+        E0.v[i] = a & (1u << i) ? pe0.v[i] + v : 0.0f;
+      }
+      if (par) {
+        cj = near;
+        cn = fetch_c(((y + 1) >> 1) + 1);
+      }
+      pe0 = pe1; pr0 = pr1; pa0 = pa1;
+      pe1 = fetch(e0, y + 2); pr1 = fetch(r0, y + 2); pa1 = fetch_a(y + 2);
+      if (par == 0) {  // rows y - 1 and y - 3 are odd: black cells 0, 2; rows y - 2, y - 4 even: red 0, 2
+        relax_row<POW2, 0>(E1, E2, E0, R[at(k, 1)], a >> 4, s, d, inv);
+        relax_row<POW2, 0>(E2, E3, E1, R[at(k, 2)], a >> 8, s, d, inv);
+        relax_row<POW2, 0>(E3, E4, E2, R[at(k, 3)], a >> 12, s, d, inv);
+        relax_row<POW2, 0>(E4, E5, E3, R[at(k, 4)], a >> 16, s, d, inv);
+      } else {
+        relax_row<POW2, 1>(E1, E2, E0, R[at(k, 1)], a >> 4, s, d, inv);
+        relax_row<POW2, 1>(E2, E3, E1, R[at(k, 2)], a >> 8, s, d, inv);
+        relax_row<POW2, 1>(E3, E4, E2, R[at(k, 3)], a >> 12, s, d, inv);
+        relax_row<POW2, 1>(E4, E5, E3, R[at(k, 4)], a >> 16, s, d, inv);
+      }
+      const int j = y - 4;
+      if (j >= t.y0 && j < t.y1) {
+        if (t.own) {
+          st_row(o0 + (long long)j * g.P, E4);
+          if (DOT) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc = fma((double)R[at(k, 4)].v[i], (double)E4.v[i], acc);
+          }
+        }
+        if (DOT && ((j & (kBand - 1)) == kBand - 1 || j == t.y1 - 1)) {
+          band_sum(g, t, c, lane, j, acc, part);
+          acc = 0.0;
+        }
+      }
     }
   }
-  const double t = block_sum2(acc, sh);
-  if (threadIdx.x == 0 && threadIdx.y == 0) part[g.part0 + (long long)c * gx * gy + b] = t;
+}
+
+template <bool DOT>
+__global__ void __launch_bounds__(kStripWarps * 32, 4) k_mg_up(const Geo *__restrict__ geo,
+                                                               const int4 *__restrict__ bmap, const Geo one,
+                                                               const uint8_t *__restrict__ flags,
+                                                               const uint8_t *__restrict__ act,
+                                                               const float *__restrict__ rhs,
+                                                               const float *__restrict__ e,
+                                                               const float *__restrict__ ec, float *__restrict__ out,
+                                                               const double *__restrict__ run, Sums sums, int first) {
+  const int4 bt = entry_of(bmap, one);
+  const int c = blockIdx.z;
+  if (c >= bt.z || run[bt.y + c] == 0.0) return;
+  const Geo g = bmap ? geo[bt.x] : one;
+  Strip t;
+  if (strip_of(g, flags, t)) {
+    if (g.lambda == 0.0) mg_up<true, DOT>(g, t, c, act, rhs, e, ec, out, sums.part);
+    else mg_up<false, DOT>(g, t, c, act, rhs, e, ec, out, sums.part);
+  }
+  if (!DOT) return;
+  double rho;
+  if (unit_sum(g, c, sums, &rho)) new_rho(sums.sc + (long long)(g.unit0 + c) * S_N, rho, first);
+}
+
+// The levels of at most kTailCells cells, in one block's shared memory: the
+// V-cycle from level k0 of an instance down to its coarsest and up again; one
+// block per instance (blockIdx.x) and channel (blockIdx.z). The coarsest level
+// (at most kCoarseMax cells) takes kCoarseSweeps plain red-black Gauss-Seidel
+// sweeps and as many in reverse colour order.
+constexpr int kCoarseMax = 64, kTailCells = 4096, kTailLevels = 8, kCoarseSweeps = 24;
+constexpr int kTailX = 32, kTailY = 16;
+struct Tail {
+  int C, unit0, n;                   // channels, first unit, levels (from k0 to the coarsest)
+  int w[kTailLevels], h[kTailLevels], P[kTailLevels];
+  long long o[kTailLevels];          // the planes' first cells in the levels' flags
+  const uint8_t *act[kTailLevels];   // the levels' flags
+  const float *rhs;                  // level k0, C planes of P[0] * h[0]
+  float *e;
+  float s[kTailLevels], d[kTailLevels];
+};
+
+__global__ void __launch_bounds__(kTailX * kTailY) k_mg_tail(const Tail *__restrict__ tails,
+                                                             const double *__restrict__ run) {
+  extern __shared__ __align__(16) float tsm[];
+  __shared__ Tail T;
+  __shared__ int off[kTailLevels + 1];
+  const int c = blockIdx.z, tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTailX + tx;
+  {
+    const int *q = reinterpret_cast<const int *>(tails + blockIdx.x);
+    for (int k = tid; k < (int)(sizeof(Tail) / 4); k += kTailX * kTailY) reinterpret_cast<int *>(&T)[k] = q[k];
+  }
+  __syncthreads();
+  if (c >= T.C || run[T.unit0 + c] == 0.0) return;
+  if (tid == 0) {
+    off[0] = 0;
+    for (int l = 0; l < T.n; ++l) off[l + 1] = off[l] + T.w[l] * T.h[l];
+  }
+  __syncthreads();
+  const int all = off[T.n];
+  float *E = tsm, *R = tsm + all;
+  uint8_t *A = reinterpret_cast<uint8_t *>(R + all);
+  for (int l = 0; l < T.n; ++l)
+    for (int j = ty; j < T.h[l]; j += kTailY)
+      for (int i = tx; i < T.w[l]; i += kTailX) A[off[l] + j * T.w[l] + i] = T.act[l][T.o[l] + (long long)j * T.P[l] + i];
+  {
+    const float *r = T.rhs + (long long)c * T.P[0] * T.h[0];
+    for (int j = ty; j < T.h[0]; j += kTailY)
+      for (int i = tx; i < T.w[0]; i += kTailX) R[j * T.w[0] + i] = r[(long long)j * T.P[0] + i];
+  }
+  __syncthreads();
+  // one colour of level l (kSmoothOmega); with red from e = 0 first, as k_mg_down takes it
+  auto half = [&](int l, int color) {
+    const int w = T.w[l], h = T.h[l];
+    const float s = T.s[l], d = T.d[l];
+    float *e = E + off[l];
+    const float *r = R + off[l];
+    const uint8_t *a = A + off[l];
+    for (int j = ty; j < h; j += kTailY)
+      for (int i = 2 * tx + ((j + color) & 1); i < w; i += 2 * kTailX) {
+        const int q = j * w + i;
+        if (!a[q]) continue;  // (an active cell is never on the border)
+        const float nb = ((e[q - 1] + e[q + 1]) + e[q - w]) + e[q + w];
+        const float gs = (r[q] + s * nb) / d;
+        e[q] = e[q] + kSmoothOmega * (gs - e[q]);
+      }
+    __syncthreads();
+  };
+  for (int l = 0; l + 1 < T.n; ++l) {
+    const int w = T.w[l], h = T.h[l], W = T.w[l + 1], H = T.h[l + 1];
+    const float s = T.s[l], d = T.d[l];
+    float *e = E + off[l];
+    const float *r = R + off[l];
+    const uint8_t *a = A + off[l];
+    for (int j = ty; j < h; j += kTailY)
+      for (int i = tx; i < w; i += kTailX) {
+        const int q = j * w + i;
+        e[q] = a[q] && ((i + j) & 1) == 0 ? kSmoothOmega * (r[q] / d) : 0.0f;
+      }
+    __syncthreads();
+    half(l, 1);
+    half(l, 0);
+    half(l, 1);
+    for (int J = ty; J < H; J += kTailY)
+      for (int I = tx; I < W; I += kTailX) {
+        float v = 0.0f;
+        if (A[off[l + 1] + J * W + I]) {
+          for (int b = -1; b <= 2; ++b) {
+            const int j = 2 * J + b;
+            if (j < 0 || j >= h) continue;
+            float row = 0.0f;
+            for (int k = -1; k <= 2; ++k) {
+              const int i = 2 * I + k;
+              if (i < 0 || i >= w) continue;
+              const int f = j * w + i;
+              float x = 0.0f;
+              if (a[f]) x = level_residual(r[f], d, e[f], s, ((e[f - 1] + e[f + 1]) + e[f - w]) + e[f + w]);
+              row = add_weighted(row, (k == 0 || k == 1) ? 0.75f : 0.25f, x);
+            }
+            v = fmaf((b == 0 || b == 1) ? 0.75f : 0.25f, row, v);
+          }
+          v *= 0.25f;
+        }
+        R[off[l + 1] + J * W + I] = v;
+      }
+    __syncthreads();
+  }
+  {  // the coarsest level: two warps, a cell a thread
+    const int l = T.n - 1, w = T.w[l], n = w * T.h[l];
+    float *e = E + off[l];
+    if (tid < kCoarseMax) {
+      const bool mine = tid < n && A[off[l] + tid];
+      const int j = tid / max(w, 1), i = tid - j * w;
+      const float s = T.s[l], d = T.d[l], r = tid < n ? R[off[l] + tid] : 0.0f;
+      const int color = (i + j) & 1;
+      if (tid < n) e[tid] = 0.0f;
+      asm volatile("bar.sync 1, 64;" ::: "memory");
+      for (int k = 0; k < 4 * kCoarseSweeps; ++k) {
+        // colour order R, B (first half) then B, R (second half)
+        const int now = k < 2 * kCoarseSweeps ? (k & 1) : 1 - (k & 1);
+        if (mine && color == now) {
+          float nb = 0.0f;
+          if (i > 0) nb += e[tid - 1];
+          if (i < w - 1) nb += e[tid + 1];
+          if (tid >= w) nb += e[tid - w];
+          if (tid + w < n) nb += e[tid + w];
+          e[tid] = (r + s * nb) / d;
+        }
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+      }
+    }
+    __syncthreads();
+  }
+  for (int l = T.n - 2; l >= 0; --l) {
+    const int w = T.w[l], h = T.h[l], W = T.w[l + 1], H = T.h[l + 1];
+    float *e = E + off[l];
+    const float *x = E + off[l + 1];
+    const uint8_t *a = A + off[l];
+    auto at = [&](int I, int J) { return I >= 0 && I < W && J >= 0 && J < H ? x[J * W + I] : 0.0f; };
+    for (int j = ty; j < h; j += kTailY)
+      for (int i = tx; i < w; i += kTailX) {
+        if (!a[j * w + i]) continue;
+        const int I0 = i >> 1, J0 = j >> 1, I1 = (i & 1) ? I0 + 1 : I0 - 1, J1 = (j & 1) ? J0 + 1 : J0 - 1;
+        e[j * w + i] += bilinear(at(I0, J0), at(I1, J0), at(I0, J1), at(I1, J1));
+      }
+    __syncthreads();
+    half(l, 1);
+    half(l, 0);
+    half(l, 1);
+    half(l, 0);
+  }
+  float *out = T.e + (long long)c * T.P[0] * T.h[0];
+  for (int j = ty; j < T.h[0]; j += kTailY)
+    for (int i = tx; i < T.P[0]; i += kTailX) out[(long long)j * T.P[0] + i] = i < T.w[0] ? E[j * T.w[0] + i] : 0.0f;
+}
+
+// ---- conjugate gradients (level-0 strips) ---------------------------------------
+// rho = r.z of an instance whose finest level is its coarsest (k_mg_up sums the
+// others').
+__global__ void __launch_bounds__(kStripWarps * 32) k_cg_dot(const Geo *__restrict__ geo,
+                                                             const int4 *__restrict__ bmap, const Geo one,
+                                                             const uint8_t *__restrict__ flags,
+                                                             const float *__restrict__ x, const float *__restrict__ y,
+                                                             const double *__restrict__ run, Sums sums, int first) {
+  const int4 bt = entry_of(bmap, one);
+  const int c = blockIdx.z, lane = threadIdx.x & 31;
+  if (c >= bt.z || run[bt.y + c] == 0.0) return;
+  const Geo g = bmap ? geo[bt.x] : one;
+  Strip t;
+  if (strip_of(g, flags, t)) {
+    const long long at = g.oc + (long long)c * g.P * g.H + t.x0;
+    double acc = 0.0;
+    for (int j = t.y0; j < t.y1; ++j) {
+      if (t.own) {
+        const Row a = ld_row(x + at + (long long)j * g.P), b = ld_row(y + at + (long long)j * g.P);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc = fma((double)a.v[i], (double)b.v[i], acc);
+      }
+      if ((j & (kBand - 1)) == kBand - 1 || j == t.y1 - 1) {
+        band_sum(g, t, c, lane, j, acc, sums.part);
+        acc = 0.0;
+      }
+    }
+  }
+  double rho;
+  if (unit_sum(g, c, sums, &rho)) new_rho(sums.sc + (long long)(g.unit0 + c) * S_N, rho, first);
+}
+
+// p' = z + beta p (p' = z on the first iteration), q = A_0 p' at active cells,
+// p.q. The strips beside read p, so p' is another array.
+__global__ void __launch_bounds__(kStripWarps * 32) k_cg_apply(const Geo *__restrict__ geo,
+                                                               const int4 *__restrict__ bmap, const Geo one,
+                                                               const uint8_t *__restrict__ flags,
+                                                               const uint8_t *__restrict__ act,
+                                                               const float *__restrict__ z, const float *__restrict__ p,
+                                                               float *__restrict__ pn, float *__restrict__ q,
+                                                               const double *__restrict__ run, Sums sums, int first) {
+  const int4 bt = entry_of(bmap, one);
+  const int c = blockIdx.z, lane = threadIdx.x & 31;
+  if (c >= bt.z || run[bt.y + c] == 0.0) return;  // (a stopped unit's p may never have been written)
+  const Geo g = bmap ? geo[bt.x] : one;
+  double *sc = sums.sc + (long long)(g.unit0 + c) * S_N;
+  Strip t;
+  if (strip_of(g, flags, t)) {
+    const float beta = first ? 0.0f : (float)sc[S_BETA], d = g.d;
+    const long long at = g.oc + (long long)c * g.P * g.H + t.x0;
+    const uint8_t *a0 = act + g.o + t.x0;
+    auto fetch = [&](const float *v, int y) { return t.in && y >= 0 && y < g.H ? ld_row(v + at + (long long)y * g.P) : row0(); };
+    auto fetch_a = [&](int y) {
+      return t.in && y >= 0 && y < g.H ? *reinterpret_cast<const uint32_t *>(a0 + (long long)y * g.P) : 0u;
+    };
+    Row m = row0(), k = row0();  // rows y - 2, y - 1 of p'
+    unsigned ak = 0;
+    double acc = 0.0;
+    Row fz = fetch(z, t.y0 - 1), fp = first ? row0() : fetch(p, t.y0 - 1);
+    uint32_t fa = fetch_a(t.y0 - 1);
+#pragma unroll 3
+    for (int y = t.y0 - 1; y <= t.y1; ++y) {
+      const unsigned a = nibble(fa);
+      Row n;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) n.v[i] = a & (1u << i) ? (first ? fz.v[i] : fz.v[i] + beta * fp.v[i]) : 0.0f;
+      fz = fetch(z, y + 1);
+      if (!first) fp = fetch(p, y + 1);
+      fa = fetch_a(y + 1);
+      if (t.own && y >= t.y0 && y < t.y1) st_row(pn + at + (long long)y * g.P, n);
+      const int j = y - 1;
+      const float l = from_left(k.v[3]), r = from_right(k.v[0]);
+      if (j >= t.y0) {
+        Row v;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float sum = (((i ? k.v[i ? i - 1 : 0] : l) + (i < 3 ? k.v[i < 3 ? i + 1 : 3] : r)) + m.v[i]) + n.v[i];
+          v.v[i] = ak & (1u << i) ? d * k.v[i] - sum : 0.0f;
+        }
+        if (t.own) {
+          st_row(q + at + (long long)j * g.P, v);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc = fma((double)k.v[i], (double)v.v[i], acc);
+        }
+        if ((j & (kBand - 1)) == kBand - 1 || j == t.y1 - 1) {
+          band_sum(g, t, c, lane, j, acc, sums.part);
+          acc = 0.0;
+        }
+      }
+      m = k;
+      k = n;
+      ak = a;
+    }
+  }
+  double pq;
+  if (unit_sum(g, c, sums, &pq)) sc[S_PQ] = pq;
+}
+
+// x += alpha p, r -= alpha q (alpha = rho / p.q); ||r||^2
+__global__ void __launch_bounds__(kStripWarps * 32) k_cg_step(const Geo *__restrict__ geo,
+                                                              const int4 *__restrict__ bmap, const Geo one,
+                                                              const uint8_t *__restrict__ flags,
+                                                              const float *__restrict__ p, const float *__restrict__ q,
+                                                              float *__restrict__ x, float *__restrict__ r,
+                                                              const double *__restrict__ run, Sums sums,
+                                                              double *__restrict__ rr) {
+  const int4 bt = entry_of(bmap, one);
+  const int c = blockIdx.z, lane = threadIdx.x & 31;
+  if (c >= bt.z || run[bt.y + c] == 0.0) return;  // a stopped unit: x and r stay
+  const Geo g = bmap ? geo[bt.x] : one;
+  const double *sc = sums.sc + (long long)(g.unit0 + c) * S_N;
+  Strip t;
+  if (strip_of(g, flags, t)) {
+    const float alpha = sc[S_PQ] > 0.0 ? (float)(sc[S_RHO] / sc[S_PQ]) : 0.0f;
+    const long long at = g.oc + (long long)c * g.P * g.H + t.x0;
+    double acc = 0.0;
+    // the rows of a band in two halves, each half's loads before its stores
+    for (int j0 = t.y0; j0 < t.y1; j0 += kBand / 2) {
+      const int n = min(kBand / 2, t.y1 - j0);
+      if (t.own) {
+        Row P[kBand / 2], Q[kBand / 2], X[kBand / 2], S[kBand / 2];
+#pragma unroll
+        for (int k = 0; k < kBand / 2; ++k) {
+          const long long o = at + (long long)(j0 + min(k, n - 1)) * g.P;
+          P[k] = ld_row(p + o); Q[k] = ld_row(q + o); X[k] = ld_row(x + o); S[k] = ld_row(r + o);
+        }
+#pragma unroll
+        for (int k = 0; k < kBand / 2; ++k) {
+          if (k >= n) break;
+          const long long o = at + (long long)(j0 + k) * g.P;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            X[k].v[i] = X[k].v[i] + alpha * P[k].v[i];
+            S[k].v[i] = S[k].v[i] - alpha * Q[k].v[i];
+            acc = fma((double)S[k].v[i], (double)S[k].v[i], acc);
+          }
+          st_row(x + o, X[k]);
+          st_row(r + o, S[k]);
+        }
+      }
+      const int j = j0 + n - 1;
+      if ((j & (kBand - 1)) == kBand - 1 || j == t.y1 - 1) {
+        band_sum(g, t, c, lane, j, acc, sums.part);
+        acc = 0.0;
+      }
+    }
+  }
+  double v;
+  if (unit_sum(g, c, sums, &v)) rr[g.unit0 + c] = v;
 }
 
 // out = interleave(u) at interior cells, the anchor elsewhere (bit for bit);
@@ -693,14 +1040,14 @@ __global__ void __launch_bounds__(kTx * kTy) k_mg_emit(const Geo *__restrict__ g
   const Geo g = bmap ? geo[gi] : one;
   const Io f = io[gi];
   const int C = g.C, W = g.W, H = g.H, b = tile_b(g), i = (b % g.gx) * kTx + threadIdx.x;
-  const size_t N = (size_t)W * H;
+  const size_t N = (size_t)g.P * H;
   const uint8_t *a = act + g.o;
   const double *u0 = u + g.oc;
   for (int j = (b / g.gx) * kTy + threadIdx.y; j < H && i < W; j += g.gy * kTy) {
-    const size_t q = (size_t)j * W + i;
-    const bool in = a[q] != 0;
+    const size_t q = (size_t)j * W + i, k = (size_t)j * g.P + i;
+    const bool in = a[k] != 0;
     for (int c = 0; c < C; ++c)  // a warp writes 32 whole pixels: C * 32 adjacent floats
-      f.out[q * C + c] = in ? (float)u0[c * N + q] : f.anchor[q * C + c];
+      f.out[q * C + c] = in ? (float)u0[c * N + k] : f.anchor[q * C + c];
   }
 }
 
@@ -708,34 +1055,25 @@ __global__ void __launch_bounds__(kTx * kTy) k_mg_emit(const Geo *__restrict__ g
 size_t aup(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // (32, 8)-thread tiles over w columns and h rows of one instance: at most
-// about 8 tiles per SM per channel, at least min_bands bands of 8 rows per
-// tile where the instance has them (a tile's first loads -- its table entry,
-// geometry and run flag -- then serve several bands), at most 65535 rows of
-// tiles.
-//
-// Level-0 launches, whose tiles write the partial sums, take kMinBands: a
-// choice that depends on the instance alone, so its partial sums and their
-// order are the same in any batch. A V-cycle launch reduces nothing and its
-// result does not depend on the tiling; it takes kMinBands only when its
-// instances have many tiles (more than kManyWaves waves of 8 per SM at one
-// band each), and one band otherwise, so that the small launches of a single
-// image's coarse levels keep their parallelism.
-constexpr int kMinBands = 4;
-constexpr long long kManyWaves = 4;
-void tiles2(int w, int h, int sms, int min_bands, int &gx, int &gy) {
+// about 8 tiles per SM per channel.
+void tiles2(int w, int h, int sms, int &gx, int &gy) {
   gx = std::max(1, (w + kTx - 1) / kTx);
-  const int bands = std::max(1, (h + kTy - 1) / kTy);
-  gy = std::min(bands, std::max(1, sms * 8 / gx));
-  gy = std::min(gy, (bands + min_bands - 1) / min_bands);
+  gy = std::min(std::max(1, (h + kTy - 1) / kTy), std::max(1, sms * 8 / gx));
   gy = std::min(gy, 65535);
 }
-const dim3 kBlock2(kTx, kTy);
+const dim3 kBlock2(kTx, kTy), kStrip(kStripWarps * 32);
+
+int pitch(int w) { return (w + 3) / 4 * 4; }
+long long bands(int w, int h) { return (long long)strip_cols(w) * ((h + kBand - 1) / kBand); }
 
 float level_s(int k) { return 1.0f / (float)(1u << (2 * std::min(k, 15))); }
 
-// A call is cut into groups of at most this many level-0 tiles (and units);
+// A call is cut into groups of at most this many level-0 bands (and units);
 // every launch of a group then has fewer blocks.
 constexpr long long kGroupTiles = 1ll << 22;
+
+// Strips: at most kMostRows rows, fewer until a launch has kFewStrips an SM.
+constexpr int kMostRows = 64, kFewStrips = 16;
 
 // One instance (a problem with channels) of a group
 struct Inst {
@@ -743,10 +1081,10 @@ struct Inst {
   int W, H, C, L;                // extent, channels, levels
   double lambda;
   std::vector<int> w, h;         // level extents
-  std::vector<long long> o, oc;  // level offsets in the one-channel and C-channel arrays
+  std::vector<long long> o, oc, f;  // level offsets in the one-channel, C-channel and flag arrays
+  int k0 = 0;                    // the first level of the one-block tail
   int unit0 = 0;                 // first (instance, channel) unit
   long long part0 = 0;           // first level-0 partial sum
-  int gx = 1, gy = 1;            // level-0 tiles
   bool dev = false, warm = false;
   size_t in = 0, mask = 0, guess = 0, out = 0;  // staged copies of host buffers
 };
@@ -759,8 +1097,10 @@ struct Launch {
   Geo one{};                 // the entry of a launch over one instance (passed by value)
 };
 
+// A level's arrays: interior flags, band flags, the correction after the pass
+// down and after the pass up, the right-hand side
 struct LevelArr {
-  size_t act = 0, e = 0, rhs = 0;
+  size_t act = 0, flags = 0, e = 0, eu = 0, rhs = 0;
 };
 
 // Tables built on the host and uploaded in one copy
@@ -774,13 +1114,18 @@ struct Blob {
   }
 };
 
-Launch make_launch(Blob &blob, std::vector<Geo> &gs) {
+// Strip launches (strips true) have kStripWarps strips a block.
+Launch make_launch(Blob &blob, std::vector<Geo> &gs, bool strips) {
+  auto count = [&](const Geo &g) {
+    const long long n = (long long)g.gx * g.gy;
+    return strips ? (n + kStripWarps - 1) / kStripWarps : n;
+  };
   Launch l;
   l.n = (int)gs.size();
   if (gs.size() == 1) {  // one instance: its geometry goes by value, no block map
     gs[0].blk0 = 0;
     l.one = gs[0];
-    l.blocks = (long long)gs[0].gx * gs[0].gy;
+    l.blocks = count(gs[0]);
     l.geo = blob.put(gs.data(), sizeof(Geo));
     return l;
   }
@@ -788,7 +1133,7 @@ Launch make_launch(Blob &blob, std::vector<Geo> &gs) {
   long long blk = 0;
   for (size_t k = 0; k < gs.size(); ++k) {
     gs[k].blk0 = (int)blk;
-    const long long nb = (long long)gs[k].gx * gs[k].gy;
+    const long long nb = count(gs[k]);
     bm.insert(bm.end(), (size_t)nb, make_int4((int)k, gs[k].unit0, gs[k].C, 0));
     blk += nb;
   }
@@ -806,11 +1151,15 @@ struct Mg {
   int U = 0;
   std::vector<Inst> in;
   std::vector<LevelArr> lv;
-  Launch all0;
-  std::vector<Launch> full, half, restr, coarse;  // per level
-  size_t tab = 0, rtab = 0, io = 0;
-  size_t u = 0, bl = 0, uw = 0, r64 = 0, part = 0, red = 0, sc = 0, scale = 0, run = 0, x = 0, r = 0, z = 0, p = 0,
+  Launch tiles0, strips0, dot0;  // level 0: tiles; strips; strips of instances without a finer level than the coarsest
+  std::vector<Launch> strips, flags, coarsen;  // per level
+  size_t tails = 0;              // table of the tails, in the table area
+  int ntails = 0;
+  size_t tail_smem = 0;
+  size_t tab = 0, io = 0;
+  size_t u = 0, bl = 0, uw = 0, r64 = 0, part = 0, done = 0, red = 0, sc = 0, scale = 0, run = 0, x = 0, r = 0, z = 0,
          q = 0;
+  size_t p[2] = {0, 0};          // the search direction's two arrays (k_cg_apply)
   long long launches = 0;
   template <class T> T *at(size_t off) { return reinterpret_cast<T *>(base + off); }
   const Geo *geo(const Launch &l) { return at<Geo>(tab + l.geo); }
@@ -818,46 +1167,45 @@ struct Mg {
   dim3 grid(const Launch &l, unsigned z) { return dim3((unsigned)l.blocks, 1, z); }
 };
 
-void vcycle(Mg &m, float *rhs0, float *e0) {
-  const int L = (int)m.lv.size();
-  // Units whose run has stopped skip the V-cycle in a batch; a single image's
-  // channels do the work regardless (their z is not read) and so spare every
-  // block a load before its first data.
-  const double *run = m.in.size() > 1 ? m.at<double>(m.run) : nullptr;
+// One V-cycle z = M r (level 0's correction on the way is the vector q), and
+// with its last pass rho = r.z and beta.
+void vcycle(Mg &m, int first) {
+  const int L = (int)m.strips.size();
   const unsigned Cz = m.Cmax;
+  const double *run = m.at<double>(m.run);
+  const Sums sums{m.at<double>(m.part), m.at<unsigned>(m.done), m.at<double>(m.sc)};
+  auto rhs = [&](int k) { return k ? m.at<float>(m.lv[k].rhs) : m.at<float>(m.r); };
+  auto down = [&](int k) { return k ? m.at<float>(m.lv[k].e) : m.at<float>(m.q); };
   for (int k = 0; k < L; ++k) {
-    const LevelArr &v = m.lv[k];
-    float *rhs = k == 0 ? rhs0 : m.at<float>(v.rhs), *e = k == 0 ? e0 : m.at<float>(v.e);
-    const uint8_t *act = m.at<uint8_t>(v.act);
-    const Launch &K = m.coarse[k];
-    if (K.n) {  // instances whose coarsest level this is: symmetric sweeps in one block per channel
-      k_mg_coarse<<<dim3((unsigned)K.n, 1, Cz), kCoarseMax, 0, m.st>>>(m.geo(K), act, rhs, e, run, 24);
-      ++m.launches;
-    }
-    const Launch &F = m.full[k], &Hh = m.half[k], &R = m.restr[k];
-    if (!F.n) continue;
-    // red, black, red, black from e = 0 (the first red half-sweep writes all of e)
-    k_mg_smooth_first<<<m.grid(F, Cz), kBlock2, 0, m.st>>>(m.geo(F), m.bmap(F), F.one, act, rhs, e, run);
-    k_mg_smooth<<<m.grid(Hh, Cz), kBlock2, 0, m.st>>>(m.geo(Hh), m.bmap(Hh), Hh.one, act, rhs, e, run, 1);
-    k_mg_smooth<<<m.grid(Hh, Cz), kBlock2, 0, m.st>>>(m.geo(Hh), m.bmap(Hh), Hh.one, act, rhs, e, run, 0);
-    k_mg_smooth<<<m.grid(Hh, Cz), kBlock2, 0, m.st>>>(m.geo(Hh), m.bmap(Hh), Hh.one, act, rhs, e, run, 1);
-    const LevelArr &cl = m.lv[k + 1];
-    k_mg_resid_restrict<<<m.grid(R, Cz), kBlock2, 0, m.st>>>(m.geo(R), m.bmap(R), R.one, act, rhs, e,
-                                                              m.at<uint8_t>(cl.act), m.at<float>(cl.rhs), run);
-    m.launches += 5;
+    const Launch &S = m.strips[k];
+    if (!S.n) continue;
+    k_mg_down<<<m.grid(S, Cz), kStrip, 0, m.st>>>(m.geo(S), m.bmap(S), S.one, m.at<uint8_t>(m.lv[k].flags),
+                                                  m.at<uint8_t>(m.lv[k].act), rhs(k), down(k),
+                                                  m.at<uint8_t>(m.lv[k + 1].act), rhs(k + 1), run);
+    ++m.launches;
   }
-  for (int k = L - 2; k >= 0; --k) {
-    const Launch &F = m.full[k], &Hh = m.half[k];
-    if (!F.n) continue;
-    const LevelArr &v = m.lv[k], &cl = m.lv[k + 1];
-    float *rhs = k == 0 ? rhs0 : m.at<float>(v.rhs), *e = k == 0 ? e0 : m.at<float>(v.e);
-    const uint8_t *act = m.at<uint8_t>(v.act);
-    k_mg_prolong<<<m.grid(F, Cz), kBlock2, 0, m.st>>>(m.geo(F), m.bmap(F), F.one, act, e, m.at<float>(cl.e), run);
-    for (int t = 0; t < 2; ++t) {
-      k_mg_smooth<<<m.grid(Hh, Cz), kBlock2, 0, m.st>>>(m.geo(Hh), m.bmap(Hh), Hh.one, act, rhs, e, run, 1);
-      k_mg_smooth<<<m.grid(Hh, Cz), kBlock2, 0, m.st>>>(m.geo(Hh), m.bmap(Hh), Hh.one, act, rhs, e, run, 0);
-    }
-    m.launches += 5;
+  k_mg_tail<<<dim3((unsigned)m.ntails, 1, Cz), dim3(kTailX, kTailY), m.tail_smem, m.st>>>(
+      m.at<Tail>(m.tab + m.tails), run);
+  ++m.launches;
+  for (int k = L - 1; k >= 0; --k) {
+    const Launch &S = m.strips[k];
+    if (!S.n) continue;
+    float *out = k ? m.at<float>(m.lv[k].eu) : m.at<float>(m.z);
+    if (k == 0)
+      k_mg_up<true><<<m.grid(S, Cz), kStrip, 0, m.st>>>(m.geo(S), m.bmap(S), S.one, m.at<uint8_t>(m.lv[k].flags),
+                                                        m.at<uint8_t>(m.lv[k].act), rhs(k), down(k),
+                                                        m.at<float>(m.lv[k + 1].eu), out, run, sums, first);
+    else
+      k_mg_up<false><<<m.grid(S, Cz), kStrip, 0, m.st>>>(m.geo(S), m.bmap(S), S.one, m.at<uint8_t>(m.lv[k].flags),
+                                                         m.at<uint8_t>(m.lv[k].act), rhs(k), down(k),
+                                                         m.at<float>(m.lv[k + 1].eu), out, run, sums, first);
+    ++m.launches;
+  }
+  if (m.dot0.n) {
+    k_cg_dot<<<m.grid(m.dot0, Cz), kStrip, 0, m.st>>>(m.geo(m.dot0), m.bmap(m.dot0), m.dot0.one,
+                                                      m.at<uint8_t>(m.lv[0].flags), m.at<float>(m.r), m.at<float>(m.z),
+                                                      run, sums, first);
+    ++m.launches;
   }
 }
 
@@ -893,104 +1241,128 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
       w = (w + 1) / 2; h = (h + 1) / 2; ++k;
     }
     I.L = (int)I.w.size();
-    tiles2(I.W, I.H, sms, kMinBands, I.gx, I.gy);
+    // the tail: the levels of few cells, and at least the coarsest
+    while (I.k0 < I.L - 1 && (I.k0 == 0 || (long long)I.w[I.k0] * I.h[I.k0] > kTailCells)) ++I.k0;
     I.unit0 = m.U;
     m.U += I.C;
     I.part0 = P;
-    P += (long long)I.C * I.gx * I.gy;
+    P += (long long)I.C * bands(I.W, I.H);
     Lmax = std::max(Lmax, I.L);
     m.Cmax = std::max(m.Cmax, (unsigned)I.C);
     any_warm |= I.warm;
     m.in.push_back(std::move(I));
   }
   const int U = m.U;
-  std::vector<long long> cells(Lmax, 0), ccells(Lmax, 0);
+  std::vector<long long> cells(Lmax, 0), ccells(Lmax, 0), nflags(Lmax, 0);
   for (Inst &I : m.in)
     for (int k = 0; k < I.L; ++k) {
       I.o.push_back(cells[k]);
       I.oc.push_back(ccells[k]);
-      cells[k] += (long long)I.w[k] * I.h[k];
-      ccells[k] += (long long)I.C * I.w[k] * I.h[k];
+      I.f.push_back(nflags[k]);
+      const long long n = (long long)pitch(I.w[k]) * I.h[k];
+      cells[k] += n;
+      ccells[k] += I.C * n;
+      nflags[k] += bands(I.w[k], I.h[k]);
     }
 
   // launch tables
   Blob blob;
-  auto geo_at = [&](const Inst &I, int k, int tw, int th, int mb) {
+  auto geo_at = [&](const Inst &I, int k) {
     Geo g{};
-    g.W = I.w[k]; g.H = I.h[k];
-    tiles2(tw, th, sms, mb, g.gx, g.gy);
+    g.W = I.w[k]; g.H = I.h[k]; g.P = pitch(g.W);
     g.C = I.C; g.unit0 = I.unit0; g.part0 = I.part0;
-    g.o = I.o[k]; g.oc = I.oc[k];
+    g.o = I.o[k]; g.oc = I.oc[k]; g.f = I.f[k];
     g.s = level_s(k);
     g.d = 4.0f * g.s + (float)I.lambda;
     g.lambda = I.lambda;
     return g;
   };
   auto second = [](Geo &g, const Inst &I, int k) {
-    g.W2 = I.w[k]; g.H2 = I.h[k]; g.o2 = I.o[k]; g.oc2 = I.oc[k];
+    g.W2 = I.w[k]; g.H2 = I.h[k]; g.P2 = pitch(g.W2); g.o2 = I.o[k]; g.oc2 = I.oc[k];
+  };
+  auto tiled = [&](Geo g) {
+    tiles2(g.P, g.H, sms, g.gx, g.gy);
+    return g;
+  };
+  auto stripped = [&](Geo g, int rows) {
+    g.rows = rows;
+    g.gx = strip_cols(g.W);
+    g.gy = (g.H + rows - 1) / rows;
+    return g;
+  };
+  // Rows a strip: as many as leave the launch kFewStrips strips. A strip walks
+  // about ten rows more than it owns (five halo rows either side), so long ones
+  // do less twice; short ones fill the GPU on small levels.
+  auto rows_for = [&](int k, bool all) {
+    for (int rows = kMostRows; rows > kBand; rows /= 2) {
+      long long n = 0;
+      for (const Inst &I : m.in)
+        if (all || k < I.k0) n += (long long)I.C * strip_cols(I.w[std::min(k, I.L - 1)]) * ((I.h[std::min(k, I.L - 1)] + rows - 1) / rows);
+      if (n >= (long long)kFewStrips * sms) return rows;
+    }
+    return kBand;
   };
   {
-    std::vector<Geo> g0;
-    for (const Inst &I : m.in) g0.push_back(geo_at(I, 0, I.W, I.H, kMinBands));
-    m.all0 = make_launch(blob, g0);
-  }
-  m.full.resize(Lmax); m.half.resize(Lmax); m.restr.resize(Lmax); m.coarse.resize(Lmax);
-  for (int k = 0; k < Lmax; ++k) {
-    long long many = 0;  // the level's tiles at one band each, all channels
-    for (const Inst &I : m.in)
-      if (k < I.L - 1) {
-        int gx, gy;
-        tiles2(I.w[k], I.h[k], sms, 1, gx, gy);
-        many += (long long)I.C * gx * gy;
-      }
-    const int mb = many > kManyWaves * 8 * sms ? kMinBands : 1;
-    std::vector<Geo> gf, gh, gr, gk;
+    std::vector<Geo> gt, gs, gd;
+    const int rows = rows_for(0, true);
     for (const Inst &I : m.in) {
-      if (k == I.L - 1) {
-        gk.push_back(geo_at(I, k, 1, 1, 1));
-      } else if (k < I.L - 1) {
-        Geo f = geo_at(I, k, I.w[k], I.h[k], mb);
-        second(f, I, k + 1);
-        gf.push_back(f);
-        gh.push_back(geo_at(I, k, (I.w[k] + 1) / 2, I.h[k], mb));
-        Geo r = geo_at(I, k + 1, I.w[k + 1], I.h[k + 1], mb);  // coarse tiles, the fine level's operator
-        r.s = level_s(k);
-        r.d = 4.0f * r.s + (float)I.lambda;
-        second(r, I, k);
-        gr.push_back(r);
+      Geo g = geo_at(I, 0);
+      gt.push_back(tiled(g));
+      gs.push_back(stripped(g, rows));
+      if (I.k0 == 0) gd.push_back(stripped(g, rows));
+    }
+    m.tiles0 = make_launch(blob, gt, false);
+    m.strips0 = make_launch(blob, gs, true);
+    m.dot0 = make_launch(blob, gd, true);
+  }
+  m.strips.resize(Lmax); m.flags.resize(Lmax); m.coarsen.resize(Lmax);
+  for (int k = 0; k < Lmax; ++k) {
+    std::vector<Geo> gs, gf, gc;
+    const int rows = rows_for(k, k == 0);
+    for (const Inst &I : m.in) {
+      if (k < I.L) gf.push_back(stripped(geo_at(I, k), kBand));
+      if (k < I.k0) {
+        Geo g = geo_at(I, k);
+        second(g, I, k + 1);
+        gs.push_back(stripped(g, rows));
+      }
+      if (k + 1 < I.L) {
+        Geo g = geo_at(I, k + 1);
+        second(g, I, k);
+        gc.push_back(tiled(g));
       }
     }
-    m.full[k] = make_launch(blob, gf);
-    m.half[k] = make_launch(blob, gh);
-    m.restr[k] = make_launch(blob, gr);
-    m.coarse[k] = make_launch(blob, gk);
-  }
-  {
-    std::vector<Red> rt;
-    for (const Inst &I : m.in)
-      for (int c = 0; c < I.C; ++c)
-        rt.push_back(Red{I.part0 + (long long)c * I.gx * I.gy, (long long)I.gx * I.gy});
-    m.rtab = blob.put(rt.data(), rt.size() * sizeof(Red));
+    m.strips[k] = make_launch(blob, gs, true);
+    m.flags[k] = make_launch(blob, gf, true);
+    m.coarsen[k] = make_launch(blob, gc, false);
   }
 
   // arena: tables, levels, level-0 vectors, then the staged host buffers
   size_t o = 0;
   auto take = [&](size_t b) { size_t r = o; o = aup(o + std::max<size_t>(b, 1)); return r; };
-  m.tab = take(blob.b.size());
+  m.tails = blob.b.size() + 64;  // (the tails' table follows: it holds arena addresses)
+  m.ntails = (int)m.in.size();
+  m.tails = (m.tails + 15) & ~(size_t)15;
+  m.tab = take(m.tails + m.in.size() * sizeof(Tail));
   m.io = take(m.in.size() * sizeof(Io));
   m.lv.resize(Lmax);
   for (int k = 0; k < Lmax; ++k) {
     m.lv[k].act = take((size_t)cells[k]);
+    m.lv[k].flags = take((size_t)nflags[k]);
     if (k > 0) {
       m.lv[k].e = take((size_t)ccells[k] * sizeof(float));
       m.lv[k].rhs = take((size_t)ccells[k] * sizeof(float));
     }
   }
+  const size_t up0 = o;  // the corrections after the passes up, cleared once
+  for (int k = 1; k < Lmax; ++k) m.lv[k].eu = take((size_t)ccells[k] * sizeof(float));
+  const size_t up1 = o;
   const size_t NC = (size_t)ccells[0];
   m.u = take(NC * 8); m.bl = take(NC * 8); m.uw = any_warm ? take(NC * 8) : 0; m.r64 = take(NC * 8);
-  m.part = take((size_t)P * 8); m.red = take((size_t)U * 8); m.sc = take((size_t)U * S_N * 8);
+  m.part = take((size_t)P * 8); m.done = take((size_t)U * sizeof(unsigned)); m.red = take((size_t)U * 8); m.sc = take((size_t)U * S_N * 8);
   m.scale = take((size_t)U * 8); m.run = take((size_t)U * 8);
-  m.x = take(NC * 4); m.r = take(NC * 4); m.z = take(NC * 4); m.p = take(NC * 4); m.q = take(NC * 4);
+  m.x = take(NC * 4); m.r = take(NC * 4); m.z = take(NC * 4); m.q = take(NC * 4);
+  m.p[0] = take(NC * 4); m.p[1] = take(NC * 4);
   for (Inst &I : m.in) {
     if (I.dev) continue;
     const size_t n = (size_t)I.W * I.H, nc = n * I.C;
@@ -1000,8 +1372,35 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
   m.base = static_cast<char *>(ctx->arena);
   cudaEventRecord(ctx->ev[0], m.st);
 
+  // the tails (they hold addresses in the arena)
+  blob.b.resize(m.tails);
+  for (const Inst &I : m.in) {
+    Tail T{};
+    T.C = I.C; T.unit0 = I.unit0; T.n = I.L - I.k0;
+    size_t cells_all = 0;
+    for (int l = 0; l < T.n; ++l) {
+      const int k = I.k0 + l;
+      T.w[l] = I.w[k]; T.h[l] = I.h[k]; T.P[l] = pitch(I.w[k]);
+      T.o[l] = I.o[k];
+      T.act[l] = m.at<uint8_t>(m.lv[k].act);
+      T.s[l] = level_s(k);
+      T.d[l] = 4.0f * T.s[l] + (float)I.lambda;
+      cells_all += (size_t)I.w[k] * I.h[k];
+    }
+    T.rhs = (I.k0 ? m.at<float>(m.lv[I.k0].rhs) : m.at<float>(m.r)) + I.oc[I.k0];
+    T.e = (I.k0 ? m.at<float>(m.lv[I.k0].eu) : m.at<float>(m.z)) + I.oc[I.k0];
+    blob.put(&T, sizeof(T));
+    m.tail_smem = std::max(m.tail_smem, cells_all * 9);
+  }
+  static_assert(sizeof(Tail) % 16 == 0, "the tails lie one after another");
+
   // tables and inputs
-  cudaError_t ce = cudaMemcpyAsync(m.base + m.tab, blob.b.data(), blob.b.size(), cudaMemcpyHostToDevice, m.st);
+  cudaError_t ce = cudaFuncSetAttribute(k_mg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kTailCells * 9);
+  if (ce == cudaSuccess)
+    ce = cudaMemcpyAsync(m.base + m.tab, blob.b.data(), blob.b.size(), cudaMemcpyHostToDevice, m.st);
+  if (ce == cudaSuccess) ce = cudaMemsetAsync(m.base + m.part, 0, (size_t)P * 8, m.st);
+  if (ce == cudaSuccess) ce = cudaMemsetAsync(m.base + m.done, 0, (size_t)U * sizeof(unsigned), m.st);
+  if (ce == cudaSuccess && up1 > up0) ce = cudaMemsetAsync(m.base + up0, 0, up1 - up0, m.st);
   std::vector<Io> io(m.in.size());
   for (size_t k = 0; k < m.in.size() && ce == cudaSuccess; ++k) {
     const Inst &I = m.in[k];
@@ -1024,24 +1423,27 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
   if (ce != cudaSuccess) return mfail(ctx, PT_LAUNCH_FAILED, std::string("input upload: ") + cudaGetErrorString(ce));
 
   const Io *iod = m.at<Io>(m.io);
-  const Launch &A = m.all0;
-  const Geo *g0 = m.geo(A);
-  const int4 *b0 = m.bmap(A);
-  const dim3 ga = m.grid(A, m.Cmax);
-  const Red *rtab = m.at<Red>(m.tab + m.rtab);
+  const Launch &A = m.tiles0, &S0 = m.strips0;
+  const Geo *g0 = m.geo(S0);
+  const int4 *b0 = m.bmap(S0);
+  const dim3 gs = m.grid(S0, m.Cmax);
   uint8_t *act0 = m.at<uint8_t>(m.lv[0].act);
-  double *u = m.at<double>(m.u), *bl = m.at<double>(m.bl), *r64 = m.at<double>(m.r64), *part = m.at<double>(m.part),
-         *red = m.at<double>(m.red), *sc = m.at<double>(m.sc), *scale = m.at<double>(m.scale),
-         *run = m.at<double>(m.run);
-  float *x = m.at<float>(m.x), *r = m.at<float>(m.r), *z = m.at<float>(m.z), *pp = m.at<float>(m.p),
-        *q = m.at<float>(m.q);
-  k_mg_assemble<<<m.grid(A, 1), kBlock2, 0, m.st>>>(g0, b0, A.one, iod, act0, u, bl,
+  const uint8_t *fl0 = m.at<uint8_t>(m.lv[0].flags);
+  double *u = m.at<double>(m.u), *bl = m.at<double>(m.bl), *r64 = m.at<double>(m.r64), *red = m.at<double>(m.red),
+         *sc = m.at<double>(m.sc), *scale = m.at<double>(m.scale), *run = m.at<double>(m.run);
+  float *x = m.at<float>(m.x), *r = m.at<float>(m.r), *z = m.at<float>(m.z), *q = m.at<float>(m.q);
+  float *pp[2] = {m.at<float>(m.p[0]), m.at<float>(m.p[1])};
+  const Sums sums{m.at<double>(m.part), m.at<unsigned>(m.done), sc};
+  k_mg_assemble<<<m.grid(A, 1), kBlock2, 0, m.st>>>(m.geo(A), m.bmap(A), A.one, iod, act0, u, bl,
                                                      any_warm ? m.at<double>(m.uw) : nullptr);
   m.launches = 1;
-  for (int k = 0; k + 1 < Lmax; ++k) {
-    const Launch &R = m.restr[k];
-    if (!R.n) continue;
-    k_mg_coarsen<<<m.grid(R, 1), kBlock2, 0, m.st>>>(m.geo(R), m.bmap(R), R.one, m.at<uint8_t>(m.lv[k].act),
+  for (int k = 0; k < Lmax; ++k) {
+    const Launch &F = m.flags[k], &K = m.coarsen[k];
+    k_mg_flags<<<m.grid(F, 1), kStrip, 0, m.st>>>(m.geo(F), m.bmap(F), F.one, m.at<uint8_t>(m.lv[k].act),
+                                                  m.at<uint8_t>(m.lv[k].flags));
+    ++m.launches;
+    if (!K.n) continue;
+    k_mg_coarsen<<<m.grid(K, 1), kBlock2, 0, m.st>>>(m.geo(K), m.bmap(K), K.one, m.at<uint8_t>(m.lv[k].act),
                                                      m.at<uint8_t>(m.lv[k + 1].act));
     ++m.launches;
   }
@@ -1061,9 +1463,9 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
   // FP64 residual norms per unit of the current u -> host
   std::vector<double> nrm(U);
   auto residual = [&](const double *uu) -> cudaError_t {
-    k_mg_residual64<<<ga, kBlock2, 0, m.st>>>(g0, b0, A.one, act0, uu, bl, r64, part);
-    k_mg_reduce<<<U, kThreads, 0, m.st>>>(part, rtab, red, 1);
-    m.launches += 2;
+    cudaMemsetAsync(red, 0, (size_t)U * 8, m.st);  // (a unit without active cells has no strips)
+    k_mg_residual64<<<gs, kStrip, 0, m.st>>>(g0, b0, S0.one, fl0, act0, uu, bl, r64, sums, red);
+    ++m.launches;
     cudaError_t e = cudaMemcpyAsync(nrm.data(), red, (size_t)U * 8, cudaMemcpyDeviceToHost, m.st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m.st);
     for (double &v : nrm) v = std::sqrt(v);
@@ -1082,7 +1484,7 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
       const Inst &I = m.in[uinst[un]];
       if (!I.warm || !(std::isfinite(nrm[un]) && nrm[un] < r0[un])) continue;
       warm_used[un] = 1;
-      const size_t n = (size_t)I.W * I.H, off = (size_t)I.oc[0] + (size_t)(un - I.unit0) * n;
+      const size_t n = (size_t)pitch(I.W) * I.H, off = (size_t)I.oc[0] + (size_t)(un - I.unit0) * n;
       cudaMemcpyAsync(u + off, uw + off, n * 8, cudaMemcpyDeviceToDevice, m.st);
     }
     ce = residual(u);
@@ -1109,51 +1511,47 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
   }
   if (poisoned) {  // u = fma(NaN, 0, u) = NaN at interior cells of those units
     cudaMemcpyAsync(scale, hscale.data(), (size_t)U * 8, cudaMemcpyHostToDevice, m.st);
-    cudaMemsetAsync(x, 0, NC * 4, m.st);
-    k_mg_update<<<ga, kBlock2, 0, m.st>>>(g0, b0, A.one, act0, x, scale, u);
+    k_mg_update<<<gs, kStrip, 0, m.st>>>(g0, b0, S0.one, fl0, act0, nullptr, scale, u);
     ++m.launches;
     std::fill(hscale.begin(), hscale.end(), 0.0);
   }
   // One CG iteration: V-cycle z = M r, rho = r.z, p = z + beta p, q = A p,
   // alpha = rho / p.q, x += alpha p, r -= alpha q, ||r||^2 (to `red`). Its
   // launches depend only on the group's shapes and the arena, so they are
-  // captured once into two CUDA graphs (first iteration, later ones) cached on
-  // the context and replayed while shapes and arena stay the same.
+  // captured once into three CUDA graphs (first iteration, later odd and even
+  // ones) cached on the context and replayed while shapes and arena stay the same.
   long long per_iteration = 0;
-  const unsigned gsc = (unsigned)std::max(1, std::min((U + kThreads - 1) / kThreads, sms * 4));
-  auto enqueue_iteration = [&](bool first) -> cudaError_t {
+  // kind 0: the first iteration; 1, 2: the later ones, which take p from one
+  // array to the other
+  auto enqueue_iteration = [&](int kind) -> cudaError_t {
     const long long l0 = m.launches;
-    vcycle(m, r, z);
-    k_cg_dot<<<ga, kBlock2, 0, m.st>>>(g0, b0, A.one, r, z, part, run);
-    k_mg_reduce<<<U, kThreads, 0, m.st>>>(part, rtab, sc + S_RHO_NEW, S_N);
-    k_cg_direction<<<ga, kBlock2, 0, m.st>>>(g0, b0, A.one, z, pp, sc, run, first ? 1 : 0);
-    k_cg_scalars_after_dir<<<gsc, kThreads, 0, m.st>>>(U, sc);
-    k_cg_apply<<<ga, kBlock2, 0, m.st>>>(g0, b0, A.one, act0, pp, q, part, run);
-    k_mg_reduce<<<U, kThreads, 0, m.st>>>(part, rtab, sc + S_PQ, S_N);
-    k_cg_step<<<ga, kBlock2, 0, m.st>>>(g0, b0, A.one, pp, q, x, r, sc, part, run);
-    k_mg_reduce<<<U, kThreads, 0, m.st>>>(part, rtab, red, 1);
-    m.launches += 8;
+    float *p = pp[kind == 1 ? 0 : 1], *pn = pp[kind == 1 ? 1 : 0];
+    const int first = kind == 0;
+    vcycle(m, first);
+    k_cg_apply<<<gs, kStrip, 0, m.st>>>(g0, b0, S0.one, fl0, act0, z, p, pn, q, run, sums, first);
+    k_cg_step<<<gs, kStrip, 0, m.st>>>(g0, b0, S0.one, fl0, pn, q, x, r, run, sums, red);
+    m.launches += 2;
     per_iteration = m.launches - l0;
     return cudaGetLastError();
   };
   if (ctx->graphs) {
     // the graphs' arguments are arena offsets and the tables' contents
     std::string key(reinterpret_cast<const char *>(&m.base), sizeof(m.base));
-    std::vector<size_t> offs = {o, m.tab, m.rtab, m.part, m.red, m.sc, m.run, m.x, m.r, m.z, m.p, m.q,
+    std::vector<size_t> offs = {o, m.tab, m.tails, m.part, m.done, m.red, m.sc, m.run, m.x, m.r, m.z, m.p[0], m.p[1], m.q,
                                 (size_t)m.Cmax, (size_t)U};
-    for (const LevelArr &v : m.lv) offs.insert(offs.end(), {v.act, v.e, v.rhs});
+    for (const LevelArr &v : m.lv) offs.insert(offs.end(), {v.act, v.flags, v.e, v.eu, v.rhs});
     key.append(reinterpret_cast<const char *>(offs.data()), offs.size() * sizeof(size_t));
     key.append(reinterpret_cast<const char *>(blob.b.data()), blob.b.size());
-    if (key != ctx->mgkey || !ctx->mgexec[0] || !ctx->mgexec[1]) {
+    if (key != ctx->mgkey || !ctx->mgexec[0] || !ctx->mgexec[1] || !ctx->mgexec[2]) {
       for (auto &ge : ctx->mgexec)
         if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
       ctx->mgkey.clear();
       const long long saved = m.launches;
-      for (int g = 0; g < 2 && ce == cudaSuccess; ++g) {
+      for (int g = 0; g < 3 && ce == cudaSuccess; ++g) {
         cudaGraph_t graph = nullptr;
         ce = cudaStreamBeginCapture(m.st, cudaStreamCaptureModeThreadLocal);
         if (ce == cudaSuccess) {
-          const cudaError_t e1 = enqueue_iteration(g == 0);
+          const cudaError_t e1 = enqueue_iteration(g);
           ce = cudaStreamEndCapture(m.st, &graph);
           if (e1 != cudaSuccess) ce = e1;
         }
@@ -1180,8 +1578,7 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
     cudaMemcpyAsync(scale, hscale.data(), (size_t)U * 8, cudaMemcpyHostToDevice, m.st);
     cudaMemcpyAsync(run, hrun.data(), (size_t)U * 8, cudaMemcpyHostToDevice, m.st);
     cudaMemsetAsync(sc, 0, (size_t)U * S_N * 8, m.st);
-    k_mg_scale<<<ga, kBlock2, 0, m.st>>>(g0, b0, A.one, r64, scale, r);
-    cudaMemsetAsync(x, 0, NC * 4, m.st);
+    k_mg_scale<<<gs, kStrip, 0, m.st>>>(g0, b0, S0.one, fl0, r64, scale, r, x);
     m.launches += 1;
     // inner target: a quarter of the remaining bar, at most as deep as FP32
     // goes from a unit residual; a run whose residual stops falling (less than
@@ -1194,12 +1591,12 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
       target[un] = going[un] ? std::max(0.25 * tol[un] * r0[un] / cur[un], kInnerFloor) : 1.0;
     }
     for (int it = 0;; ++it) {
-      const int g = it == 0 ? 0 : 1;
+      const int g = it == 0 ? 0 : 2 - (it & 1);
       if (ctx->mgexec[g]) {
         ce = cudaGraphLaunch(ctx->mgexec[g], m.st);
         m.launches += ctx->mgnodes;
       } else {
-        ce = enqueue_iteration(it == 0);
+        ce = enqueue_iteration(g);
       }
       if (ce != cudaSuccess) return mfail(ctx, PT_LAUNCH_FAILED, std::string("cg: ") + cudaGetErrorString(ce));
       ce = cudaMemcpyAsync(rr.data(), red, (size_t)U * 8, cudaMemcpyDeviceToHost, m.st);
@@ -1225,7 +1622,7 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
       if (changed) cudaMemcpyAsync(run, hrun.data(), (size_t)U * 8, cudaMemcpyHostToDevice, m.st);
     }
     // u += scale * x, then the FP64 residual decides
-    k_mg_update<<<ga, kBlock2, 0, m.st>>>(g0, b0, A.one, act0, x, scale, u);
+    k_mg_update<<<gs, kStrip, 0, m.st>>>(g0, b0, S0.one, fl0, act0, x, scale, u);
     ++m.launches;
     const std::vector<double> prev = cur;
     ce = residual(u);
@@ -1242,7 +1639,7 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
     ++outer;
   }
   cudaEventRecord(ctx->ev[2], m.st);
-  k_mg_emit<<<m.grid(A, 1), kBlock2, 0, m.st>>>(g0, b0, A.one, iod, act0, u);
+  k_mg_emit<<<m.grid(A, 1), kBlock2, 0, m.st>>>(m.geo(A), m.bmap(A), A.one, iod, act0, u);
   ++m.launches;
   ce = cudaSuccess;
   for (size_t k = 0; k < m.in.size() && ce == cudaSuccess; ++k) {
@@ -1338,9 +1735,7 @@ pt_status ptk_solve_mg_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, floa
       reports[i][0] = r;
       continue;
     }
-    int gx, gy;
-    tiles2((int)p.width, (int)p.height, ctx->sms, kMinBands, gx, gy);
-    const long long t = (long long)gx * gy;
+    const long long t = bands((int)p.width, (int)p.height);
     if (!ids.empty() && (tiles + t > kGroupTiles || units + p.channels > kGroupTiles)) {
       const pt_status s = flush();
       if (s != PT_OK) return s;
