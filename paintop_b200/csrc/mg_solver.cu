@@ -277,6 +277,34 @@ __device__ __forceinline__ void st_row(float *p, const Row &r) {
 __device__ __forceinline__ float from_left(float x) { return __shfl_up_sync(0xffffffffu, x, 1); }
 __device__ __forceinline__ float from_right(float x) { return __shfl_down_sync(0xffffffffu, x, 1); }
 
+// Rows on their way: each lane's 16 bytes (and its four flags) of the next
+// kRing - 1 rows, copied asynchronously into a ring in shared memory that only
+// the lane itself reads. With two rows held ahead in registers instead, a third
+// of the passes' time went by waiting for loads.
+constexpr int kRing = 6;
+struct RowRing {
+  float4 v[kRing][32];
+};
+struct FlagRing {
+  uint32_t v[kRing][32];
+};
+__device__ __forceinline__ void ring_put(void *dst, const void *src, int bytes, bool in) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if (bytes == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(in ? 16 : 0) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void ring_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void ring_wait() {  // all but the newest kRing - 2 rows have arrived
+  asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 2) : "memory");
+}
+__device__ __forceinline__ void ring_drain() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ Row ring_row(const RowRing &q, int k) {
+  const float4 x = q.v[k][threadIdx.x & 31];
+  return Row{{x.x, x.y, x.z, x.w}};
+}
+
 // v / d. With POW2 d is a power of two (lambda 0) and the product with its
 // reciprocal is the quotient, bit for bit.
 template <bool POW2>
@@ -505,7 +533,8 @@ __device__ __forceinline__ float bilinear(float a, float b, float c, float d) {
 template <bool POW2>
 __device__ __forceinline__ void mg_down(const Geo &g, const Strip &t, int c, const uint8_t *__restrict__ act,
                                         const float *__restrict__ rhs, float *__restrict__ e,
-                                        const uint8_t *__restrict__ actc, float *__restrict__ rhsc) {
+                                        const uint8_t *__restrict__ actc, float *__restrict__ rhsc, RowRing &rr,
+                                        FlagRing &ra) {
   const long long N = (long long)g.P * g.H, Nc = (long long)g.P2 * g.H2;
   const uint8_t *a0 = act + g.o + t.x0;
   const float *r0 = rhs + g.oc + c * N + t.x0;
@@ -520,24 +549,26 @@ __device__ __forceinline__ void mg_down(const Geo &g, const Strip &t, int c, con
   for (int k = 0; k < 6; ++k) E[k] = R[k] = row0();
   unsigned a = 0;  // active bits, the newest row's lowest
   float vp0 = 0.f, vp1 = 0.f, vn0 = 0.f, vn1 = 0.f;
-  // the next two rows are on their way (rows after `last` are walked in vain)
-  const int y0 = t.y0 - 6;
-  auto fetch_r = [&](int y) { return t.in && y >= 0 && y < g.H ? ld_row(r0 + (long long)y * g.P) : row0(); };
-  auto fetch_a = [&](int y) {
-    return t.in && y >= 0 && y < g.H ? *reinterpret_cast<const uint32_t *>(a0 + (long long)y * g.P) : 0u;
+  const int y0 = t.y0 - 6, lane = threadIdx.x & 31;  // (rows after `last` are walked in vain)
+  auto fetch = [&](int y, int k) {
+    const bool in = t.in && y >= 0 && y < g.H;
+    const long long o = in ? (long long)y * g.P : -(long long)t.x0;  // (the plane's first cell: not read)
+    ring_put(&rr.v[k][lane], r0 + o, 16, in);
+    ring_put(&ra.v[k][lane], a0 + o, 4, in);
+    ring_commit();
   };
-  Row pr0 = fetch_r(y0), pr1 = fetch_r(y0 + 1);
-  uint32_t pa0 = fetch_a(y0), pa1 = fetch_a(y0 + 1);
+#pragma unroll
+  for (int k = 0; k < kRing - 1; ++k) fetch(y0 + k, k);
   for (int yb = y0; yb <= last; yb += 6) {
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
       const int y = yb + k;
       constexpr auto at = [](int k, int i) { return (k + 6 - i) % 6; };
       const int par = k & 1;  // y0 is even
-      R[k] = pr0;
-      a = (a << 4) | nibble(pa0);
-      pr0 = pr1; pa0 = pa1;
-      pr1 = fetch_r(y + 2); pa1 = fetch_a(y + 2);
+      ring_wait();
+      R[k] = ring_row(rr, k);
+      a = (a << 4) | nibble(ra.v[k][lane]);
+      fetch(y + kRing - 1, at(k, 1));
       Row &E0 = E[k], &E1 = E[at(k, 1)], &E2 = E[at(k, 2)], &E3 = E[at(k, 3)], &E4 = E[at(k, 4)], &E5 = E[at(k, 5)];
       // red of row y from e = 0; black 0
 #pragma unroll
@@ -584,6 +615,7 @@ __device__ __forceinline__ void mg_down(const Geo &g, const Strip &t, int c, con
       }
     }
   }
+  ring_drain();
 }
 
 __global__ void __launch_bounds__(kStripWarps * 32, 4) k_mg_down(const Geo *__restrict__ geo,
@@ -598,10 +630,13 @@ __global__ void __launch_bounds__(kStripWarps * 32, 4) k_mg_down(const Geo *__re
   const int c = blockIdx.z;
   if (c >= bt.z || run[bt.y + c] == 0.0) return;
   const Geo g = bmap ? geo[bt.x] : one;
+  __shared__ RowRing rr[kStripWarps];
+  __shared__ FlagRing ra[kStripWarps];
+  const int w = threadIdx.x >> 5;
   Strip t;
   if (!strip_of(g, flags, t)) return;
-  if (g.lambda == 0.0) mg_down<true>(g, t, c, act, rhs, e, actc, rhsc);
-  else mg_down<false>(g, t, c, act, rhs, e, actc, rhsc);
+  if (g.lambda == 0.0) mg_down<true>(g, t, c, act, rhs, e, actc, rhsc, rr[w], ra[w]);
+  else mg_down<false>(g, t, c, act, rhs, e, actc, rhsc, rr[w], ra[w]);
 }
 
 // Up one level: e += the bilinear prolongation of the coarse correction at
@@ -612,7 +647,7 @@ template <bool POW2, bool DOT>
 __device__ __forceinline__ void mg_up(const Geo &g, const Strip &t, int c, const uint8_t *__restrict__ act,
                                       const float *__restrict__ rhs, const float *__restrict__ e,
                                       const float *__restrict__ ec, float *__restrict__ out,
-                                      double *__restrict__ part) {
+                                      double *__restrict__ part, RowRing &re, RowRing &rr, FlagRing &ra) {
   const int lane = threadIdx.x & 31;
   const long long N = (long long)g.P * g.H, Nc = (long long)g.P2 * g.H2;
   const uint8_t *a0 = act + g.o + t.x0;
@@ -628,22 +663,24 @@ __device__ __forceinline__ void mg_up(const Geo &g, const Strip &t, int c, const
   unsigned a = 0;
   double acc = 0.0;
   const int y0 = t.y0 - 4;
-  auto fetch = [&](const float *p, int y) { return t.in && y >= 0 && y < g.H ? ld_row(p + (long long)y * g.P) : row0(); };
-  auto fetch_a = [&](int y) {
-    return t.in && y >= 0 && y < g.H ? *reinterpret_cast<const uint32_t *>(a0 + (long long)y * g.P) : 0u;
+  auto fetch = [&](int y, int k) {
+    const bool in = t.in && y >= 0 && y < g.H;
+    const long long o = in ? (long long)y * g.P : -(long long)t.x0;  // (the plane's first cell: not read)
+    ring_put(&re.v[k][lane], e0 + o, 16, in);
+    ring_put(&rr.v[k][lane], r0 + o, 16, in);
+    ring_put(&ra.v[k][lane], a0 + o, 4, in);
+    ring_commit();
   };
   auto fetch_c = [&](int J) {
     return I < g.P2 && J >= 0 && J < g.H2 ? *reinterpret_cast<const float2 *>(c0 + (long long)J * g.P2) : make_float2(0.f, 0.f);
   };
   // four coarse values a row around the lane's four cells: columns I - 1 .. I + 2
   auto wide = [&](float2 v) { return Row{{from_left(v.y), v.x, v.y, from_right(v.x)}}; };
-  Row pe0 = fetch(e0, y0), pr0 = fetch(r0, y0);
-  uint32_t pa0 = fetch_a(y0);
-  Row pe1 = fetch(e0, y0 + 1), pr1 = fetch(r0, y0 + 1);
-  uint32_t pa1 = fetch_a(y0 + 1);
-  // coarse rows J - 1, J (J = y / 2), and J + 1 on its way
+#pragma unroll
+  for (int k = 0; k < kRing - 1; ++k) fetch(y0 + k, k);
+  // coarse rows J - 1, J (J = y / 2), and J + 1, J + 2 on their way
   Row cm = wide(fetch_c((y0 >> 1) - 1)), cj = wide(fetch_c(y0 >> 1));
-  float2 cn = fetch_c((y0 >> 1) + 1);
+  float2 cn = fetch_c((y0 >> 1) + 1), cnn = fetch_c((y0 >> 1) + 2);
   for (int yb = y0; yb <= last; yb += 6) {
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -651,8 +688,11 @@ __device__ __forceinline__ void mg_up(const Geo &g, const Strip &t, int c, const
       constexpr auto at = [](int k, int i) { return (k + 6 - i) % 6; };
       const int par = k & 1;  // y0 is even
       Row &E0 = E[k], &E1 = E[at(k, 1)], &E2 = E[at(k, 2)], &E3 = E[at(k, 3)], &E4 = E[at(k, 4)], &E5 = E[at(k, 5)];
-      R[k] = pr0;
-      a = (a << 4) | nibble(pa0);
+      ring_wait();
+      R[k] = ring_row(rr, k);
+      const Row pe = ring_row(re, k);
+      a = (a << 4) | nibble(ra.v[k][lane]);
+      fetch(y + kRing - 1, at(k, 1));
       Row near;
       if (par == 0) {
         near = cm;
@@ -667,14 +707,13 @@ __device__ __forceinline__ void mg_up(const Geo &g, const Strip &t, int c, const
         const int m0 = 1 + (i >> 1), m1 = (i & 1) ? m0 + 1 : m0 - 1;
         const Row &rj = par == 0 ? cj : cm;  // row J (cm holds it after the move)
         const float v = bilinear(rj.v[m0], rj.v[m1], near.v[m0], near.v[m1]);
-        E0.v[i] = a & (1u << i) ? pe0.v[i] + v : 0.0f;
+        E0.v[i] = a & (1u << i) ? pe.v[i] + v : 0.0f;
       }
       if (par) {
         cj = near;
-        cn = fetch_c(((y + 1) >> 1) + 1);
+        cn = cnn;
+        cnn = fetch_c(((y + 1) >> 1) + 2);
       }
-      pe0 = pe1; pr0 = pr1; pa0 = pa1;
-      pe1 = fetch(e0, y + 2); pr1 = fetch(r0, y + 2); pa1 = fetch_a(y + 2);
       if (par == 0) {  // rows y - 1 and y - 3 are odd: black cells 0, 2; rows y - 2, y - 4 even: red 0, 2
         relax_row<POW2, 0>(E1, E2, E0, R[at(k, 1)], a >> 4, s, d, inv);
         relax_row<POW2, 0>(E2, E3, E1, R[at(k, 2)], a >> 8, s, d, inv);
@@ -702,6 +741,7 @@ __device__ __forceinline__ void mg_up(const Geo &g, const Strip &t, int c, const
       }
     }
   }
+  ring_drain();
 }
 
 template <bool DOT>
@@ -717,10 +757,13 @@ __global__ void __launch_bounds__(kStripWarps * 32, 4) k_mg_up(const Geo *__rest
   const int c = blockIdx.z;
   if (c >= bt.z || run[bt.y + c] == 0.0) return;
   const Geo g = bmap ? geo[bt.x] : one;
+  __shared__ RowRing re[kStripWarps], rr[kStripWarps];
+  __shared__ FlagRing ra[kStripWarps];
+  const int w = threadIdx.x >> 5;
   Strip t;
   if (strip_of(g, flags, t)) {
-    if (g.lambda == 0.0) mg_up<true, DOT>(g, t, c, act, rhs, e, ec, out, sums.part);
-    else mg_up<false, DOT>(g, t, c, act, rhs, e, ec, out, sums.part);
+    if (g.lambda == 0.0) mg_up<true, DOT>(g, t, c, act, rhs, e, ec, out, sums.part, re[w], rr[w], ra[w]);
+    else mg_up<false, DOT>(g, t, c, act, rhs, e, ec, out, sums.part, re[w], rr[w], ra[w]);
   }
   if (!DOT) return;
   double rho;
@@ -731,11 +774,16 @@ __global__ void __launch_bounds__(kStripWarps * 32, 4) k_mg_up(const Geo *__rest
 // V-cycle from level k0 of an instance down to its coarsest and up again; one
 // block per instance (blockIdx.x) and channel (blockIdx.z). The coarsest level
 // (at most kCoarseMax cells) takes kCoarseSweeps plain red-black Gauss-Seidel
-// sweeps and as many in reverse colour order.
-constexpr int kCoarseMax = 64, kTailCells = 4096, kTailLevels = 8, kCoarseSweeps = 24;
-constexpr int kTailX = 32, kTailY = 16;
-struct Tail {
+// sweeps and as many in reverse colour order. Bound by the latency of its
+// phases, a barrier each, and beyond a few thousand cells by one SM's shared
+// memory: a level of 119 x 91 cells cost 20 us more here than its two strip
+// launches, one of 60 x 46 about 10 us less (per pass over 237 x 181: 849 us
+// a solve with 12288 cells in the tail, 797 with 4096, 816 with 1100).
+constexpr int kCoarseMax = 64, kTailCells = 4096, kTailLevels = 10, kCoarseSweeps = 24;
+constexpr int kTailX = 32, kTailY = 32;
+struct alignas(16) Tail {
   int C, unit0, n;                   // channels, first unit, levels (from k0 to the coarsest)
+  int pow2;                          // lambda is 0: every level's d is a power of two (over)
   int w[kTailLevels], h[kTailLevels], P[kTailLevels];
   long long o[kTailLevels];          // the planes' first cells in the levels' flags
   const uint8_t *act[kTailLevels];   // the levels' flags
@@ -743,19 +791,21 @@ struct Tail {
   float *e;
   float s[kTailLevels], d[kTailLevels];
 };
+// Shared memory: e, rhs and flags of every level; the first level's residual.
+constexpr int kTailSmem = 224 * 1024;
+size_t tail_bytes(size_t all, size_t first) { return all * 9 + 16 + first * 4; }
 
-__global__ void __launch_bounds__(kTailX * kTailY) k_mg_tail(const Tail *__restrict__ tails,
-                                                             const double *__restrict__ run) {
+__global__ void __launch_bounds__(kTailX * kTailY, 1) k_mg_tail(const Tail *__restrict__ tails,
+                                                                const double *__restrict__ run) {
   extern __shared__ __align__(16) float tsm[];
   __shared__ Tail T;
-  __shared__ int off[kTailLevels + 1];
+  __shared__ int off[kTailLevels + 1], table[kCoarseMax];
   const int c = blockIdx.z, tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTailX + tx;
-  {
-    const int *q = reinterpret_cast<const int *>(tails + blockIdx.x);
-    for (int k = tid; k < (int)(sizeof(Tail) / 4); k += kTailX * kTailY) reinterpret_cast<int *>(&T)[k] = q[k];
-  }
+  for (int k = tid; k < (int)(sizeof(Tail) / 4); k += kTailX * kTailY)
+    reinterpret_cast<int *>(&T)[k] = reinterpret_cast<const int *>(tails + blockIdx.x)[k];
   __syncthreads();
   if (c >= T.C || run[T.unit0 + c] == 0.0) return;
+  if (tid < kCoarseMax) table[tid] = -1;
   if (tid == 0) {
     off[0] = 0;
     for (int l = 0; l < T.n; ++l) off[l + 1] = off[l] + T.w[l] * T.h[l];
@@ -763,64 +813,84 @@ __global__ void __launch_bounds__(kTailX * kTailY) k_mg_tail(const Tail *__restr
   __syncthreads();
   const int all = off[T.n];
   float *E = tsm, *R = tsm + all;
-  uint8_t *A = reinterpret_cast<uint8_t *>(R + all);
-  for (int l = 0; l < T.n; ++l)
-    for (int j = ty; j < T.h[l]; j += kTailY)
-      for (int i = tx; i < T.w[l]; i += kTailX) A[off[l] + j * T.w[l] + i] = T.act[l][T.o[l] + (long long)j * T.P[l] + i];
+  float *X = R + all;  // the residual of the level on the way down
+  uint8_t *A = reinterpret_cast<uint8_t *>(X + T.w[0] * T.h[0]);
   {
     const float *r = T.rhs + (long long)c * T.P[0] * T.h[0];
+    const int w = T.w[0];
+#pragma unroll 4
     for (int j = ty; j < T.h[0]; j += kTailY)
-      for (int i = tx; i < T.w[0]; i += kTailX) R[j * T.w[0] + i] = r[(long long)j * T.P[0] + i];
+      for (int i = tx; i < w; i += kTailX) R[j * w + i] = r[(long long)j * T.P[0] + i];
+  }
+  for (int l = 0; l < T.n; ++l) {
+    const uint8_t *f = T.act[l] + T.o[l];
+    const int w = T.w[l];
+#pragma unroll 4
+    for (int j = ty; j < T.h[l]; j += kTailY)
+      for (int i = tx; i < w; i += kTailX) A[off[l] + j * w + i] = f[(long long)j * T.P[l] + i];
   }
   __syncthreads();
-  // one colour of level l (kSmoothOmega); with red from e = 0 first, as k_mg_down takes it
+  const bool pow2 = T.pow2;
+  auto quotient = [&](float v, float d, float inv) { return pow2 ? v * inv : v / d; };
+  // one colour of level l (kSmoothOmega); two rows at once, loads first: the
+  // neighbours are of the other colour
   auto half = [&](int l, int color) {
     const int w = T.w[l], h = T.h[l];
-    const float s = T.s[l], d = T.d[l];
+    const float s = T.s[l], d = T.d[l], inv = 1.0f / d;
     float *e = E + off[l];
     const float *r = R + off[l];
     const uint8_t *a = A + off[l];
-    for (int j = ty; j < h; j += kTailY)
-      for (int i = 2 * tx + ((j + color) & 1); i < w; i += 2 * kTailX) {
-        const int q = j * w + i;
-        if (!a[q]) continue;  // (an active cell is never on the border)
-        const float nb = ((e[q - 1] + e[q + 1]) + e[q - w]) + e[q + w];
-        const float gs = (r[q] + s * nb) / d;
-        e[q] = e[q] + kSmoothOmega * (gs - e[q]);
+    // (kTailY is even: a thread's rows have one parity)
+    for (int i = 2 * tx + ((ty + color) & 1); i < w; i += 2 * kTailX)
+      for (int j = ty, q = ty * w + i; j < h; j += 2 * kTailY, q += 2 * kTailY * w) {
+        const int q1 = q + kTailY * w;
+        const bool on0 = a[q], on1 = j + kTailY < h && a[q1];  // (an active cell is never on the border)
+        float n0, n1, r0, r1, e0, e1;
+        if (on0) {
+          n0 = ((e[q - 1] + e[q + 1]) + e[q - w]) + e[q + w];
+          r0 = r[q];
+          e0 = e[q];
+        }
+        if (on1) {
+          n1 = ((e[q1 - 1] + e[q1 + 1]) + e[q1 - w]) + e[q1 + w];
+          r1 = r[q1];
+          e1 = e[q1];
+        }
+        if (on0) e[q] = e0 + kSmoothOmega * (quotient(r0 + s * n0, d, inv) - e0);
+        if (on1) e[q1] = e1 + kSmoothOmega * (quotient(r1 + s * n1, d, inv) - e1);
       }
     __syncthreads();
   };
   for (int l = 0; l + 1 < T.n; ++l) {
     const int w = T.w[l], h = T.h[l], W = T.w[l + 1], H = T.h[l + 1];
-    const float s = T.s[l], d = T.d[l];
+    const float s = T.s[l], d = T.d[l], inv = 1.0f / d;
     float *e = E + off[l];
     const float *r = R + off[l];
     const uint8_t *a = A + off[l];
-    for (int j = ty; j < h; j += kTailY)
-      for (int i = tx; i < w; i += kTailX) {
-        const int q = j * w + i;
-        e[q] = a[q] && ((i + j) & 1) == 0 ? kSmoothOmega * (r[q] / d) : 0.0f;
-      }
+    for (int i = tx; i < w; i += kTailX)
+#pragma unroll 2
+      for (int j = ty, q = ty * w + i; j < h; j += kTailY, q += kTailY * w)
+        e[q] = a[q] && ((i + ty) & 1) == 0 ? kSmoothOmega * quotient(r[q], d, inv) : 0.0f;
     __syncthreads();
     half(l, 1);
     half(l, 0);
     half(l, 1);
+    for (int i = tx; i < w; i += kTailX)
+#pragma unroll 2
+      for (int j = ty, q = ty * w + i; j < h; j += kTailY, q += kTailY * w) {
+        X[q] = a[q] ? level_residual(r[q], d, e[q], s, ((e[q - 1] + e[q + 1]) + e[q - w]) + e[q + w]) : 0.0f;
+      }
+    __syncthreads();
     for (int J = ty; J < H; J += kTailY)
       for (int I = tx; I < W; I += kTailX) {
         float v = 0.0f;
-        if (A[off[l + 1] + J * W + I]) {
+        if (A[off[l + 1] + J * W + I]) {  // (not on the border: all its 4 x 4 fine cells exist)
+#pragma unroll
           for (int b = -1; b <= 2; ++b) {
-            const int j = 2 * J + b;
-            if (j < 0 || j >= h) continue;
+            const float *x = X + (2 * J + b) * w + 2 * I;
             float row = 0.0f;
-            for (int k = -1; k <= 2; ++k) {
-              const int i = 2 * I + k;
-              if (i < 0 || i >= w) continue;
-              const int f = j * w + i;
-              float x = 0.0f;
-              if (a[f]) x = level_residual(r[f], d, e[f], s, ((e[f - 1] + e[f + 1]) + e[f - w]) + e[f + w]);
-              row = add_weighted(row, (k == 0 || k == 1) ? 0.75f : 0.25f, x);
-            }
+#pragma unroll
+            for (int k = -1; k <= 2; ++k) row = add_weighted(row, (k == 0 || k == 1) ? 0.75f : 0.25f, x[k]);
             v = fmaf((b == 0 || b == 1) ? 0.75f : 0.25f, row, v);
           }
           v *= 0.25f;
@@ -829,44 +899,69 @@ __global__ void __launch_bounds__(kTailX * kTailY) k_mg_tail(const Tail *__restr
       }
     __syncthreads();
   }
-  {  // the coarsest level: two warps, a cell a thread
-    const int l = T.n - 1, w = T.w[l], n = w * T.h[l];
-    float *e = E + off[l];
-    if (tid < kCoarseMax) {
-      const bool mine = tid < n && A[off[l] + tid];
-      const int j = tid / max(w, 1), i = tid - j * w;
-      const float s = T.s[l], d = T.d[l], r = tid < n ? R[off[l] + tid] : 0.0f;
-      const int color = (i + j) & 1;
-      if (tid < n) e[tid] = 0.0f;
-      asm volatile("bar.sync 1, 64;" ::: "memory");
-      for (int k = 0; k < 4 * kCoarseSweeps; ++k) {
-        // colour order R, B (first half) then B, R (second half)
-        const int now = k < 2 * kCoarseSweeps ? (k & 1) : 1 - (k & 1);
-        if (mine && color == now) {
-          float nb = 0.0f;
-          if (i > 0) nb += e[tid - 1];
-          if (i < w - 1) nb += e[tid + 1];
-          if (tid >= w) nb += e[tid - w];
-          if (tid + w < n) nb += e[tid + w];
-          e[tid] = (r + s * nb) / d;
-        }
-        asm volatile("bar.sync 1, 64;" ::: "memory");
-      }
-    }
-    __syncthreads();
+  // lane of a cell of the coarsest level: the cells of its colour before it, row-major
+  auto lane_of = [&](int w, int q) {
+    const int j = q / w, i = q - j * w, color = (i + j) & 1;
+    const int even = (w + 1 - color) / 2, odd = (w + color) / 2;  // of this colour in even rows, in odd rows
+    return ((j + 1) >> 1) * even + (j >> 1) * odd + (i >> 1);
+  };
+  if (tid < kCoarseMax) {
+    const int w = T.w[T.n - 1], n = w * T.h[T.n - 1];
+    if (tid < n) table[((tid % w + tid / w) & 1) * 32 + lane_of(w, tid)] = tid;
+    asm volatile("bar.sync 1, 64;" ::: "memory");
   }
+  if (tid < 32) {
+    // the coarsest level: one warp, a red and a black cell a lane (64 cells have
+    // 32 of each), neighbours by shuffles from the lanes that hold them
+    const int l = T.n - 1, w = T.w[l];
+    const float s = T.s[l], d = T.d[l], inv = 1.0f / d;
+    float v[2] = {0.0f, 0.0f}, r[2] = {0.0f, 0.0f};
+    const int cell[2] = {table[tid], table[32 + tid]};
+    int at[2][4];
+    bool on[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int q = cell[k];
+      on[k] = q >= 0 && A[off[l] + q];  // (never on the border)
+      if (on[k]) r[k] = R[off[l] + q];
+      at[k][0] = on[k] ? lane_of(w, q - 1) : 0;
+      at[k][1] = on[k] ? lane_of(w, q + 1) : 0;
+      at[k][2] = on[k] ? lane_of(w, q - w) : 0;
+      at[k][3] = on[k] ? lane_of(w, q + w) : 0;
+    }
+    auto step = [&](int k) {
+      const float x0 = __shfl_sync(0xffffffffu, v[1 - k], at[k][0]), x1 = __shfl_sync(0xffffffffu, v[1 - k], at[k][1]);
+      const float x2 = __shfl_sync(0xffffffffu, v[1 - k], at[k][2]), x3 = __shfl_sync(0xffffffffu, v[1 - k], at[k][3]);
+      const float nb = ((x0 + x1) + x2) + x3;
+      if (on[k]) v[k] = quotient(r[k] + s * nb, d, inv);
+    };
+    for (int k = 0; k < kCoarseSweeps; ++k) {
+      step(0);
+      step(1);
+    }
+    for (int k = 0; k < kCoarseSweeps; ++k) {
+      step(1);
+      step(0);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      if (cell[k] >= 0) E[off[l] + cell[k]] = v[k];
+  }
+  __syncthreads();
   for (int l = T.n - 2; l >= 0; --l) {
-    const int w = T.w[l], h = T.h[l], W = T.w[l + 1], H = T.h[l + 1];
+    const int w = T.w[l], h = T.h[l], W = T.w[l + 1];
     float *e = E + off[l];
     const float *x = E + off[l + 1];
     const uint8_t *a = A + off[l];
-    auto at = [&](int I, int J) { return I >= 0 && I < W && J >= 0 && J < H ? x[J * W + I] : 0.0f; };
-    for (int j = ty; j < h; j += kTailY)
-      for (int i = tx; i < w; i += kTailX) {
-        if (!a[j * w + i]) continue;
-        const int I0 = i >> 1, J0 = j >> 1, I1 = (i & 1) ? I0 + 1 : I0 - 1, J1 = (j & 1) ? J0 + 1 : J0 - 1;
-        e[j * w + i] += bilinear(at(I0, J0), at(I1, J0), at(I0, J1), at(I1, J1));
+    for (int i = tx; i < w; i += kTailX) {
+      const int I0 = i >> 1, I1 = (i & 1) ? I0 + 1 : I0 - 1;
+#pragma unroll 2
+      for (int j = ty, q = ty * w + i; j < h; j += kTailY, q += kTailY * w) {
+        if (!a[q]) continue;  // (an active cell's coarse neighbours exist)
+        const float *x0 = x + (j >> 1) * W, *x1 = (j & 1) ? x0 + W : x0 - W;
+        e[q] += bilinear(x0[I0], x0[I1], x1[I0], x1[I1]);
       }
+    }
     __syncthreads();
     half(l, 1);
     half(l, 0);
@@ -1242,7 +1337,13 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
     }
     I.L = (int)I.w.size();
     // the tail: the levels of few cells, and at least the coarsest
-    while (I.k0 < I.L - 1 && (I.k0 == 0 || (long long)I.w[I.k0] * I.h[I.k0] > kTailCells)) ++I.k0;
+    auto in_tail = [&](int k) {
+      size_t all = 0;
+      for (int l = k; l < I.L; ++l) all += (size_t)I.w[l] * I.h[l];
+      const size_t first = (size_t)I.w[k] * I.h[k];
+      return first <= (size_t)kTailCells && I.L - k <= kTailLevels && tail_bytes(all, first) <= (size_t)kTailSmem;
+    };
+    while (I.k0 < I.L - 1 && (I.k0 == 0 || !in_tail(I.k0))) ++I.k0;
     I.unit0 = m.U;
     m.U += I.C;
     I.part0 = P;
@@ -1377,6 +1478,7 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
   for (const Inst &I : m.in) {
     Tail T{};
     T.C = I.C; T.unit0 = I.unit0; T.n = I.L - I.k0;
+    T.pow2 = I.lambda == 0.0;
     size_t cells_all = 0;
     for (int l = 0; l < T.n; ++l) {
       const int k = I.k0 + l;
@@ -1390,12 +1492,12 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
     T.rhs = (I.k0 ? m.at<float>(m.lv[I.k0].rhs) : m.at<float>(m.r)) + I.oc[I.k0];
     T.e = (I.k0 ? m.at<float>(m.lv[I.k0].eu) : m.at<float>(m.z)) + I.oc[I.k0];
     blob.put(&T, sizeof(T));
-    m.tail_smem = std::max(m.tail_smem, cells_all * 9);
+    m.tail_smem = std::max(m.tail_smem, tail_bytes(cells_all, (size_t)I.w[I.k0] * I.h[I.k0]));
   }
   static_assert(sizeof(Tail) % 16 == 0, "the tails lie one after another");
 
   // tables and inputs
-  cudaError_t ce = cudaFuncSetAttribute(k_mg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kTailCells * 9);
+  cudaError_t ce = cudaFuncSetAttribute(k_mg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
   if (ce == cudaSuccess)
     ce = cudaMemcpyAsync(m.base + m.tab, blob.b.data(), blob.b.size(), cudaMemcpyHostToDevice, m.st);
   if (ce == cudaSuccess) ce = cudaMemsetAsync(m.base + m.part, 0, (size_t)P * 8, m.st);
