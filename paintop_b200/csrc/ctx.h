@@ -24,6 +24,9 @@ struct pt_ctx {
   double last_call_ms = 0.0;   // whole call from first upload to last download
   long long last_launches = 0; // kernels launched by the last call
   unsigned long long last_h2d = 0, last_d2h = 0;  // bytes the last solve moved each way
+  void *pin = nullptr;         // page-locked staging of plans and results, grown to a high-water mark
+  size_t pin_cap = 0;
+  int solve_grid[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // blocks of k_solve that fit the device, by tile configuration
   bool graphs = true;          // capture device-pointer solves into a CUDA graph
   cudaGraphExec_t gexec = nullptr;
   std::string gkey;            // the plan the cached graph was captured for
@@ -63,8 +66,27 @@ struct pt_ctx {
     return true;
   }
 
+  // Staging for at least `bytes`; the calls wait for their copies before they
+  // return, so what is there is free.
+  bool reserve_pin(size_t bytes) {
+    if (bytes <= pin_cap) return true;
+    if (pin) cudaFreeHost(pin);
+    pin = nullptr;
+    pin_cap = 0;
+    if (cudaMallocHost(&pin, bytes + bytes / 4) != cudaSuccess) {
+      cudaGetLastError();
+      pin = nullptr;
+      return false;
+    }
+    pin_cap = bytes + bytes / 4;
+    return true;
+  }
+
   void release() {
     drop_graphs();
+    if (pin) cudaFreeHost(pin);
+    pin = nullptr;
+    pin_cap = 0;
     for (auto &e : ev)
       if (e) { cudaEventDestroy(e); e = nullptr; }
     if (arena) cudaFree(arena);

@@ -217,7 +217,7 @@ extern "C" pt_status pt_poisson_solve_noalloc(const pt_problem *p, float *out_ca
     if (e == cudaSuccess) e = launch_assembly(P, tc, st);
     int grid = 0;
     if (e == cudaSuccess) e = launch_solve(P, cfg, sms, st, &grid);
-    if (e == cudaSuccess) e = launch_emit(P, 0, tc, (long long)W * H, st);
+    if (e == cudaSuccess) e = launch_emit(P, nullptr, 1, tc, (long long)W * H, st);
     SysState states[kMaxChannels];
     int kerr = 0;
     if (e == cudaSuccess)

@@ -19,6 +19,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <algorithm>
+#include <limits>
 #include <string>
 #include <vector>
 
@@ -681,9 +683,15 @@ extern "C" pt_status pt_op_compute_ex(pt_ctx *ctx, const char *op_id, const pt_p
       std::memcpy(residual_history, hist.data() + (size_t)w.channel * p.max_iterations, m * sizeof(double));
     }
     if (all_finite) {
+      // a run at a time, so that the test of a run needs no branch: one value at
+      // a time took 4 ms on 6.3 million
       int32_t f = 1;
-      for (size_t k = 0; k < count; ++k)
-        if (!std::isfinite(candidate[k])) { f = 0; break; }
+      for (size_t k0 = 0; k0 < count && f; k0 += 4096) {
+        const size_t k1 = std::min(count, k0 + 4096);
+        int bad = 0;
+        for (size_t k = k0; k < k1; ++k) bad |= !(std::fabs(candidate[k]) <= std::numeric_limits<float>::max());
+        f = !bad;
+      }
       *all_finite = f;
     }
     return PT_OK;

@@ -431,41 +431,45 @@ __global__ void k_compact(KParams P) {
 
 // Interleave the result: interior cells take (float)u (the reference's `as f32`,
 // poisson_blend.rs:211-219); every other pixel copies the target bit for bit.
-__global__ void k_emit(KParams P, int sys0, int TW, int TH) {
-  const SysDesc d0 = P.sys[sys0];
-  const long long npx = (long long)d0.W * d0.H;
-  const int C = d0.C;
-  // four channels with 16-byte aligned images: one vector load and store per pixel
-  const bool vec4 = C == 4 && ((reinterpret_cast<uintptr_t>(d0.tgt) | reinterpret_cast<uintptr_t>(d0.out)) & 15) == 0;
-  for (long long px = blockIdx.x * (long long)blockDim.x + threadIdx.x; px < npx;
-       px += (long long)gridDim.x * blockDim.x) {
-    const int y = (int)(px / d0.W), x = (int)(px - (long long)y * d0.W);
-    const int tx = x / TW, ty = y / TH;
-    const int c = (x + y) & 1, i = x >> 1;
-    // the channels share the tile counts (k_tile_count stores one per channel)
-    const bool active = P.tcount[d0.tile0 + ty * d0.ntx + tx] > 0;
-    if (vec4) {
-      float4 v = *reinterpret_cast<const float4 *>(d0.tgt + px * 4);
-      if (active) {
-        float *vv = reinterpret_cast<float *>(&v);
+__global__ void k_emit(KParams P, const int *__restrict__ imgs, int nimg, int TW, int TH) {
+  // image by image (blockIdx.y)
+  for (int img = blockIdx.y; img < nimg; img += gridDim.y) {
+    const int sys0 = imgs ? imgs[img] : 0;
+    const SysDesc d0 = P.sys[sys0];
+    const long long npx = (long long)d0.W * d0.H;
+    const int C = d0.C;
+    // four channels with 16-byte aligned images: one vector load and store per pixel
+    const bool vec4 = C == 4 && ((reinterpret_cast<uintptr_t>(d0.tgt) | reinterpret_cast<uintptr_t>(d0.out)) & 15) == 0;
+    for (long long px = blockIdx.x * (long long)blockDim.x + threadIdx.x; px < npx;
+         px += (long long)gridDim.x * blockDim.x) {
+      const int y = (int)(px / d0.W), x = (int)(px - (long long)y * d0.W);
+      const int tx = x / TW, ty = y / TH;
+      const int c = (x + y) & 1, i = x >> 1;
+      // the channels share the tile counts (k_tile_count stores one per channel)
+      const bool active = P.tcount[d0.tile0 + ty * d0.ntx + tx] > 0;
+      if (vec4) {
+        float4 v = *reinterpret_cast<const float4 *>(d0.tgt + px * 4);
+        if (active) {
+          float *vv = reinterpret_cast<float *>(&v);
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
-          if (P.st[sys0 + ch].out_anchor) continue;
-          const long long o = plane_index(P.sys[sys0 + ch], c, y, i);
-          if (P.cell[o]) vv[ch] = (float)P.u[o];
+          for (int ch = 0; ch < 4; ++ch) {
+            if (P.st[sys0 + ch].out_anchor) continue;
+            const long long o = plane_index(P.sys[sys0 + ch], c, y, i);
+            if (P.cell[o]) vv[ch] = (float)P.u[o];
+          }
         }
+        *reinterpret_cast<float4 *>(d0.out + px * 4) = v;
+        continue;
       }
-      *reinterpret_cast<float4 *>(d0.out + px * 4) = v;
-      continue;
-    }
-    for (int ch = 0; ch < C; ++ch) {
-      const SysDesc &d = P.sys[sys0 + ch];
-      float v = d.tgt[px * C + ch];
-      if (active && !P.st[sys0 + ch].out_anchor) {
-        const long long o = plane_index(d, c, y, i);
-        if (P.cell[o]) v = (float)P.u[o];
+      for (int ch = 0; ch < C; ++ch) {
+        const SysDesc &d = P.sys[sys0 + ch];
+        float v = d.tgt[px * C + ch];
+        if (active && !P.st[sys0 + ch].out_anchor) {
+          const long long o = plane_index(d, c, y, i);
+          if (P.cell[o]) v = (float)P.u[o];
+        }
+        d.out[px * C + ch] = v;
       }
-      d.out[px * C + ch] = v;
     }
   }
 }
@@ -993,12 +997,15 @@ cudaError_t launch_band_flags(const KParams &P, int sys0, int *spans, cudaStream
   return cudaGetLastError();
 }
 
-cudaError_t launch_emit(const KParams &P, int sys0, const TileConfig &tc, long long npx,
+cudaError_t launch_emit(const KParams &P, const int *imgs, int nimg, const TileConfig &tc, long long npx,
                         cudaStream_t stream) {
-  if (npx <= 0) return cudaSuccess;
+  if (npx <= 0 || nimg <= 0) return cudaSuccess;
   long long blocks = (npx + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  k_emit<<<(int)blocks, 256, 0, stream>>>(P, sys0, tc.tw, tc.th);
+  // one launch for all images; their blocks fill the GPU a few times over
+  const long long each = 148 * 32 / nimg > 16 ? 148 * 32 / nimg : 16;
+  if (nimg > 1 && blocks > each) blocks = each;
+  k_emit<<<dim3((unsigned)blocks, (unsigned)(nimg < 65535 ? nimg : 65535)), 256, 0, stream>>>(P, imgs, nimg, tc.tw, tc.th);
   return cudaGetLastError();
 }
 

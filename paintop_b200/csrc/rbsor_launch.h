@@ -44,8 +44,10 @@ cudaError_t launch_tile_count(const KParams &P, const TileConfig &tc, cudaStream
 // of image sys0 that hold interior cells, or -1, -1 (the solve reads the
 // image only there, one pixel around).
 cudaError_t launch_band_flags(const KParams &P, int sys0, int *spans, cudaStream_t stream);
-// Interleave one image's channels sys0 .. sys0+C-1 into its output.
-cudaError_t launch_emit(const KParams &P, int sys0, const TileConfig &tc, long long npx,
+// Interleave the images' channels into their outputs: image k's are the systems
+// imgs[k] .. (imgs on the device; null: one image, from system 0); npx: the
+// largest image's pixels.
+cudaError_t launch_emit(const KParams &P, const int *imgs, int nimg, const TileConfig &tc, long long npx,
                         cudaStream_t stream);
 
 }  // namespace ptk

@@ -91,6 +91,8 @@ struct Plan {
   long long out_floats = 0;
   std::vector<RegionDesc> regions;  // images labelled for the automatic omega
   long long rpix = 0;               // their pixels
+  std::vector<int> imgs;            // the first system of each image
+  long long largest = 0;            // the largest image's pixels
   std::vector<int> clist;           // the systems by cluster class
   std::vector<ClusterClass> classes;
 };
@@ -98,7 +100,7 @@ struct Plan {
 // Arena layout (byte offsets) for one call.
 struct Layout {
   size_t sys, st, claim, arrive, tiles, tcount, tbox, act, e0, e1, g, cell, u, bp, partial, fpart, hist, bar, err, in,
-      mask, out, regions, label, rsize, rmax, bands, route, clist, total;
+      mask, out, regions, label, rsize, rmax, bands, route, clist, imgs, plan_end, results_end, total;
 };
 
 // Row bands of every image (host-buffer solves: two ints each, the band's
@@ -115,11 +117,19 @@ Layout layout(const Plan &pl, bool stage) {
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t r = o; o = align_up(o + std::max<size_t>(bytes, 1), kAlign); return r; };
   const size_t nt = pl.tiles.size(), ns = pl.sys.size();
+  // the plan, in one piece: what a call uploads
   L.sys = take(ns * sizeof(SysDesc));
+  L.tiles = take(nt * sizeof(Tile));
+  L.regions = take(pl.regions.size() * sizeof(RegionDesc));
+  L.clist = take(pl.clist.size() * sizeof(int));
+  L.imgs = take(pl.imgs.size() * sizeof(int));
+  L.plan_end = o;
+  // the states and the error word, in one piece: what it downloads
   L.st = take(ns * sizeof(SysState));
+  L.err = take(sizeof(int));
+  L.results_end = o;
   L.claim = take(ns * sizeof(unsigned long long));
   L.arrive = take(ns * sizeof(unsigned));
-  L.tiles = take(nt * sizeof(Tile));
   L.tcount = take(nt * sizeof(int));
   L.tbox = take(nt * sizeof(int4));
   L.act = take(nt * sizeof(int));
@@ -133,17 +143,14 @@ Layout layout(const Plan &pl, bool stage) {
   L.fpart = take(2 * nt * sizeof(double));
   L.hist = take(pl.hist * sizeof(double));
   L.bar = take(kBarWords * sizeof(unsigned));
-  L.err = take(sizeof(int));
   L.in = stage ? take(pl.in_floats * sizeof(float)) : 0;
   L.mask = stage ? take(pl.mask_floats * sizeof(float)) : 0;
   L.out = stage ? take(pl.out_floats * sizeof(float)) : 0;
-  L.regions = take(pl.regions.size() * sizeof(RegionDesc));
   L.label = take((size_t)pl.rpix * sizeof(int));
   L.rsize = take((size_t)pl.rpix * sizeof(int));
   L.rmax = take(pl.regions.size() * sizeof(int));
   L.bands = stage ? take(2 * band_count(pl) * sizeof(int)) : 0;
   L.route = take(ns * sizeof(Route));
-  L.clist = take(pl.clist.size() * sizeof(int));
   L.total = o;
   return L;
 }
@@ -287,6 +294,8 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
       pl.sys.push_back(d);
     }
     if (C > 0) {
+      pl.imgs.push_back(sys0[i]);
+      pl.largest = std::max(pl.largest, img);
       pl.in_floats += img * C * (1 + 1 + ((p.flags & PT_FLAG_WARM_START) ? 1 : 0));
       pl.mask_floats += img;
       pl.out_floats += img * C;
@@ -310,7 +319,8 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
   if (ce != cudaSuccess) return cuda_fail(ctx, ce, "cudaSetDevice");
   const Layout L = layout(pl, !devptr);
   if (!ctx->reserve(L.total)) return fail(ctx, PT_OOM, "device arena allocation failed");
-  char *base = static_cast<char *>(ctx->arena);
+  if (!ctx->reserve_pin(std::max(L.plan_end, L.results_end - L.st))) return fail(ctx, PT_OOM, "host staging allocation failed");
+  char *base = static_cast<char *>(ctx->arena), *pin = static_cast<char *>(ctx->pin);
   cudaStream_t st = ctx->stream;
   for (auto &e : ctx->ev)
     if (!e && cudaEventCreate(&e) != cudaSuccess) return fail(ctx, PT_LAUNCH_FAILED, "event create");
@@ -349,18 +359,24 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
       }
     }
   }
-  h2d += pl.sys.size() * sizeof(SysDesc) + pl.tiles.size() * sizeof(Tile) + pl.regions.size() * sizeof(RegionDesc) +
-         pl.clist.size() * sizeof(int);
-  ce = cudaMemcpyAsync(base + L.sys, pl.sys.data(), pl.sys.size() * sizeof(SysDesc),
-                       cudaMemcpyHostToDevice, st);
-  if (ce == cudaSuccess)
-    ce = cudaMemcpyAsync(base + L.tiles, pl.tiles.data(), pl.tiles.size() * sizeof(Tile),
-                         cudaMemcpyHostToDevice, st);
-  if (ce == cudaSuccess && !pl.regions.empty())
-    ce = cudaMemcpyAsync(base + L.regions, pl.regions.data(), pl.regions.size() * sizeof(RegionDesc),
-                         cudaMemcpyHostToDevice, st);
-  if (ce == cudaSuccess && !pl.clist.empty())
-    ce = cudaMemcpyAsync(base + L.clist, pl.clist.data(), pl.clist.size() * sizeof(int), cudaMemcpyHostToDevice, st);
+  h2d += L.plan_end;
+  // (a call that fails below leaves the staging only when its copies are done)
+  struct Settle {
+    cudaStream_t st;
+    bool done = false;
+    ~Settle() {
+      if (!done) cudaStreamSynchronize(st);
+    }
+  } settle{st};
+  auto stage = [&](size_t at, const void *from, size_t bytes) {
+    if (bytes) std::memcpy(pin + at, from, bytes);
+  };
+  stage(L.sys, pl.sys.data(), pl.sys.size() * sizeof(SysDesc));
+  stage(L.tiles, pl.tiles.data(), pl.tiles.size() * sizeof(Tile));
+  stage(L.regions, pl.regions.data(), pl.regions.size() * sizeof(RegionDesc));
+  stage(L.clist, pl.clist.data(), pl.clist.size() * sizeof(int));
+  stage(L.imgs, pl.imgs.data(), pl.imgs.size() * sizeof(int));
+  ce = cudaMemcpyAsync(base, pin, L.plan_end, cudaMemcpyHostToDevice, st);
   if (ce != cudaSuccess) return cuda_fail(ctx, ce, "plan upload");
 
   KParams P{};
@@ -522,16 +538,21 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
   }
 
   int grid = 0;
-  ce = prepare_cluster();
-  if (ce == cudaSuccess) ce = prepare_solve(P, pl.cfg, ctx->sms, &grid);
-  if (ce != cudaSuccess) return cuda_fail(ctx, ce, "solve prepare");
+  if (!ctx->solve_grid[pl.cfg]) {  // once a context and configuration
+    KParams all = P;
+    all.ntiles = INT32_MAX;
+    ce = prepare_cluster();
+    if (ce == cudaSuccess) ce = prepare_solve(all, pl.cfg, ctx->sms, &ctx->solve_grid[pl.cfg]);
+    if (ce != cudaSuccess) return cuda_fail(ctx, ce, "solve prepare");
+  }
+  grid = std::max(1, std::min(ctx->solve_grid[pl.cfg], P.ntiles));
   ctx->last_grid = grid;
   ctx->last_cfg = pl.cfg;
   long long cluster_launches = 0;
   for (const ClusterClass &k : pl.classes) cluster_launches += k.rows4 ? 2 : 1;
   long long launches = 5 + cluster_launches;  // tile count, compaction, assembly, init, solves
-  for (uint32_t i = 0; i < n; ++i) launches += ps[i].channels > 0 ? (devptr ? 1 : 2) : 0;  // emits, band flags
-  if (!devptr) launches += 1;  // the first tile count
+  launches += 1;                                                 // emit
+  if (!devptr) launches += 1 + (long long)pl.imgs.size();        // the first tile count, band flags
 
   // Everything from here to the results is stream work on the device: with
   // device pointers it is captured once into a CUDA graph and replayed while
@@ -552,26 +573,22 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
       if (e == cudaSuccess) e = launch_cluster(P, pl.tc, k, reinterpret_cast<const int *>(base + L.clist), st);
     if (e == cudaSuccess) e = launch_prepared(P, pl.cfg, grid, st);
     if (e == cudaSuccess) e = record(ctx->ev[2], capturing);
-    for (uint32_t i = 0; i < n && e == cudaSuccess; ++i)
-      if (ps[i].channels > 0)
-        e = launch_emit(P, sys0[i], pl.tc, (long long)ps[i].width * ps[i].height, st);
-    if (devptr && histories)
-      for (uint32_t i = 0; i < n && e == cudaSuccess; ++i) {
-        if (!histories[i] || !ps[i].max_iterations) continue;
-        for (uint32_t c = 0; c < ps[i].channels && e == cudaSuccess; ++c)
-          e = cudaMemcpyAsync(histories[i] + (size_t)c * ps[i].max_iterations,
-                              reinterpret_cast<double *>(base + L.hist) + pl.sys[sys0[i] + c].hist_off,
-                              ps[i].max_iterations * sizeof(double), cudaMemcpyDeviceToDevice, st);
-      }
+    if (e == cudaSuccess)
+      e = launch_emit(P, reinterpret_cast<const int *>(base + L.imgs), (int)pl.imgs.size(), pl.tc, pl.largest, st);
     return e;
   };
   if (devptr && ctx->graphs) {
-    std::string key(reinterpret_cast<const char *>(pl.sys.data()), pl.sys.size() * sizeof(SysDesc));
+    // the kernels read the images' addresses from the descriptors, so the
+    // graph serves any buffers: they are no part of its key
+    std::vector<SysDesc> shapes = pl.sys;
+    for (SysDesc &d : shapes) {
+      d.src = d.tgt = d.guess = d.mask = nullptr;
+      d.out = nullptr;
+    }
+    std::string key(reinterpret_cast<const char *>(shapes.data()), shapes.size() * sizeof(SysDesc));
     const long long extra[6] = {pl.cfg, grid, (long long)(uintptr_t)base, (long long)L.total,
-                                (long long)pl.tiles.size(), (long long)(histories != nullptr)};
+                                (long long)pl.tiles.size(), (long long)P.budget_ns};
     key.append(reinterpret_cast<const char *>(extra), sizeof(extra));
-    if (histories)
-      for (uint32_t i = 0; i < n; ++i) key.append(reinterpret_cast<const char *>(&histories[i]), sizeof(void *));
     if (!ctx->gexec || key != ctx->gkey) {
       if (ctx->gexec) { cudaGraphExecDestroy(ctx->gexec); ctx->gexec = nullptr; }
       cudaGraph_t g = nullptr;
@@ -594,11 +611,9 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
   }
 
   // ---- download
-  std::vector<SysState> states(nsys);
-  int kerr = 0;
-  d2h += nsys * sizeof(SysState) + sizeof(int);
-  ce = cudaMemcpyAsync(states.data(), base + L.st, nsys * sizeof(SysState), cudaMemcpyDeviceToHost, st);
-  if (ce == cudaSuccess) ce = cudaMemcpyAsync(&kerr, base + L.err, sizeof(int), cudaMemcpyDeviceToHost, st);
+  const SysState *states = reinterpret_cast<const SysState *>(pin);
+  d2h += L.results_end - L.st;
+  ce = cudaMemcpyAsync(pin, base + L.st, L.results_end - L.st, cudaMemcpyDeviceToHost, st);
   // host buffers: each band's span of interior tiles comes down after the
   // emit (the rest of the output is being filled on the host)
   if (!devptr && ce == cudaSuccess) {
@@ -620,23 +635,24 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
       boff += (size_t)d0.nty;
     }
   }
-  if (histories && !devptr && ce == cudaSuccess) {
+  if (histories && ce == cudaSuccess) {
     for (uint32_t i = 0; i < n && ce == cudaSuccess; ++i) {
       if (!histories[i]) continue;
       for (uint32_t c = 0; c < ps[i].channels && ce == cudaSuccess; ++c) {
         const SysDesc &d = pl.sys[sys0[i] + c];
         const size_t cnt = ps[i].max_iterations;
         if (!cnt) continue;
-        d2h += cnt * sizeof(double);
+        if (!devptr) d2h += cnt * sizeof(double);
         ce = cudaMemcpyAsync(histories[i] + (size_t)c * cnt,
                              reinterpret_cast<double *>(base + L.hist) + d.hist_off, cnt * sizeof(double),
-                             cudaMemcpyDeviceToHost, st);
+                             devptr ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st);
       }
     }
   }
   if (ce != cudaSuccess) return cuda_fail(ctx, ce, "result download");
   cudaEventRecord(ctx->ev[3], st);
   ce = cudaStreamSynchronize(st);
+  settle.done = true;
   if (ce != cudaSuccess) return cuda_fail(ctx, ce, "stream synchronize");
   {
     float a = 0.f, b = 0.f;
@@ -649,6 +665,8 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
     ctx->last_h2d = h2d;
     ctx->last_d2h = d2h;
   }
+  int kerr = 0;
+  std::memcpy(&kerr, pin + (L.err - L.st), sizeof(int));
   if (kerr != KERR_NONE)
     return fail(ctx, PT_TIMEOUT, kerr == KERR_DEADLINE ? "solve exceeded its wall budget"
                                                        : "wait for work gave up (no progress)");
