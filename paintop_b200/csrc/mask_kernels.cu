@@ -12,19 +12,29 @@
 // the device. Only hypot may differ from the host's in the last bit (the op is
 // declared tolerance-bounded for exactly that reason).
 //
+// Most pixels lie far from the edge, where the feather saturates: a bound on the
+// signed distance from (u/rx)^2 + (v/ry)^2 alone settles those without the
+// square roots and divisions (4096 x 4096: 168 us with them for every pixel, 54 without).
+//
 // Polygon: the reference tests every edge at every one of the 16 subsamples of
 // every pixel. A subsample row's crossing abscissa t = (y - y0) / (y1 - y0),
 // c = fma(t, x1 - x0, x0) depends on the row and the edge only, and a
 // subsample column x_q = (q + 0.5) / 4 lies left of c exactly when
-// q < ceil(4c - 0.5), an integer computed exactly from c. So a block owns a
-// span of 1024 pixels of one pixel row; per subsample row it computes each
-// edge's crossing once (edges in chunks of 256, one per thread), turns it into
-// that integer, adds crossings right of the whole span to a span-wide winding,
-// drops those left of it, and keeps the few inside the span; each thread then
-// resolves its 4 pixels' 16 subsamples with integer compares. The arithmetic
-// of every crossing is the reference's and winding sums and parities do not
-// depend on the order crossings are visited in, so the mask is bit-identical
-// to the reference's rasterize().
+// q < ceil(4c - 0.5), an integer computed exactly from c. So a warp owns a
+// span of 2048 pixels of one pixel row: its lanes compute each (edge, subsample
+// row)'s crossing once, turn it into that integer, add crossings right of the
+// whole span to a span-wide winding, drop those left of it and keep the few
+// inside it. Then each lane sums up one 128-pixel run of the span; a run without
+// a crossing inside has one coverage and is stored as such, the others resolve
+// their pixels' 16 subsamples with integer compares. The arithmetic of every
+// crossing is the reference's and winding sums and parities do not depend on
+// the order crossings are visited in, so the mask is bit-identical to the
+// reference's rasterize(). More than 256 edges: a block a span, edges in chunks.
+//
+// Bound by the stores of the plane (4096 x 4096: 67 MB). A block a span with a
+// barrier a row, every thread visiting every crossing, took 50 us for the
+// 12-vertex star; a warp a span takes 25 (19 in the
+// profiler, at 65% of the issue slots; writing the plane alone is 10).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -53,21 +63,31 @@ __device__ __forceinline__ double feather(double sd, double half_width_px) {
   return __dsub_rn(1.0, smoothstep);
 }
 
+// far2: (u/rx)^2 + (v/ry)^2 above which the coverage is 0, near2: below which it
+// is 1. The signed distance (f - 1) f / |grad| is at least |f - 1| min(rx, ry)
+// in size, f = sqrt of that sum, so beyond half_width_px of the edge the feather
+// is saturated; the limits keep a margin of 1e-9 for the rounding of both.
 __global__ void k_mask_ellipse(int W, int H, double cx, double cy, double rx, double ry, double sn, double cs,
-                               double half_width_px, float *out) {
+                               double half_width_px, double far2, double near2, float *out) {
+  const double irx = 1.0 / rx, iry = 1.0 / ry;
   const long long n = (long long)W * H;
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n;
-       p += (long long)gridDim.x * blockDim.x) {
+  const long long step = (long long)gridDim.x * blockDim.x;
+  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += step) {
     const int j = (int)(p / W), i = (int)(p - (long long)j * W);
     const double off_x = ((double)i + 0.5) - cx, off_y = ((double)j + 0.5) - cy;
     const double local_u = fma(sn, off_y, cs * off_x);
     const double local_v = fma(cs, off_y, -sn * off_x);
-    const double norm_x = local_u / rx, norm_y = local_v / ry;
-    const double f = sqrt(fma(norm_x, norm_x, norm_y * norm_y));
+    const double ax = local_u * irx, ay = local_v * iry, f2 = fma(ax, ax, ay * ay);
     double cov = 1.0;
-    if (f != 0.0) {
-      const double grad = hypot(local_u / (rx * rx), local_v / (ry * ry));
-      if (grad != 0.0) cov = feather((f - 1.0) * f / grad, half_width_px);
+    if (f2 > far2 && f2 < 1e200) {
+      cov = 0.0;
+    } else if (!(f2 < near2)) {
+      const double norm_x = local_u / rx, norm_y = local_v / ry;
+      const double f = sqrt(fma(norm_x, norm_x, norm_y * norm_y));
+      if (f != 0.0) {
+        const double grad = hypot(local_u / (rx * rx), local_v / (ry * ry));
+        if (grad != 0.0) cov = feather((f - 1.0) * f / grad, half_width_px);
+      }
     }
     out[p] = (float)cov;
   }
@@ -83,9 +103,9 @@ __device__ __forceinline__ int columns_left_of(double c, int W) {
   return (int)fmin(fmax(z, 0.0), 4.0 * (double)W);
 }
 
-// Winding of this thread's 4 x kPix subsamples of one subsample row, applied
-// to the fill rule and added to inside[]: wt is shared by all its columns,
-// w[l] holds crossings that fall inside its columns.
+// (k_mask_polygon_chunked) Winding of this thread's 4 x kPix subsamples of one
+// subsample row, applied to the fill rule and added to inside[]: wt is shared by
+// all its columns, w[l] holds crossings that fall inside its columns.
 __device__ __forceinline__ void add_row(int wt, const int (&w)[kPix * kSub], bool partial, int even_odd,
                                         int (&inside)[kPix]) {
   if (!partial) {
@@ -100,99 +120,147 @@ __device__ __forceinline__ void add_row(int wt, const int (&w)[kPix * kSub], boo
   }
 }
 
-// Polygons of at most 256 edges: a block loops over rows of its span. The
-// (edge, subsample row) pairs are spread over all threads, crossings of a row
-// land in one of three shared buffers (the row's position in the block's
-// sequence, modulo 3), so one barrier per row orders them: the buffer written
-// for the next row was last read two rows ago, and is cleared between the two
-// barriers that follow that read.
 // edges[k] = (x0, y0, x1, y1) of the edge from vertex k to vertex (k + 1) % n.
-__device__ __forceinline__ void store_row(float *out, int W, int j, int px, int vec4, const int (&inside)[kPix]) {
-  float cov[kPix];
-  for (int p = 0; p < kPix; ++p) cov[p] = (float)inside[p] * (1.0f / (float)(kSub * kSub));  // k / 16, exact
-  float *row = out + (long long)j * W;
+__device__ __forceinline__ void store_row(float *out, int W, int j, int px, int vec4, float c0, float c1, float c2,
+                                          float c3) {
+  float *row = out + (long long)j * W + px;
   if (vec4 && px + kPix <= W) {
-    *reinterpret_cast<float4 *>(row + px) = make_float4(cov[0], cov[1], cov[2], cov[3]);
+    *reinterpret_cast<float4 *>(row) = make_float4(c0, c1, c2, c3);
   } else {
-    for (int p = 0; p < kPix; ++p)
-      if (px + p < W) row[px + p] = cov[p];
+    if (px < W) row[0] = c0;
+    if (px + 1 < W) row[1] = c1;
+    if (px + 2 < W) row[2] = c2;
+    if (px + 3 < W) row[3] = c3;
   }
 }
 
-__global__ void __launch_bounds__(kRowThreads, 4) k_mask_polygon_rows(int W, int H,
-                                                                     const double4 *__restrict__ edges, int nedges,
-                                                                     int even_odd, double ymin, double ymax,
-                                                                     int vec4, float *__restrict__ out) {
-  __shared__ double4 sedge[kRowThreads];
-  __shared__ int cross_q[3][kSub][kRowThreads];
-  __shared__ signed char cross_dir[3][kSub][kRowThreads];
-  __shared__ int count[3][kSub];
-  __shared__ int span_base[3][kSub];
-  const int x0 = blockIdx.x * kSpan;
-  const int q0 = 4 * x0, q1 = 4 * min(x0 + kSpan, W);
-  const int px = x0 + threadIdx.x * kPix;
-  const int qp = 4 * px;
+// Polygons of at most kRowThreads edges: a warp a unit of one row and one span of
+// kRuns runs; crossings inside the span by subsample row in shared memory
+// (room for nedges each).
+constexpr int kRun = 32 * kPix;               // pixels of a run: a float4 a lane
+constexpr int kRuns = 16;                     // runs of a span
+constexpr int kUnitWarps = kRowThreads / 32;  // warps per block
+size_t rows_smem(int nedges) { return (size_t)nedges * (sizeof(double4) + kUnitWarps * kSub * sizeof(int2)); }
+
+__global__ void __launch_bounds__(kRowThreads) k_mask_polygon_rows(int W, int H, const double4 *__restrict__ edges,
+                                                                  int nedges, int even_odd, double ymin, double ymax,
+                                                                  int vec4, int spans, float *__restrict__ out) {
+  extern __shared__ __align__(32) unsigned char smem[];
+  double4 *sedge = reinterpret_cast<double4 *>(smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int2 *cross = reinterpret_cast<int2 *>(sedge + nedges) + warp * kSub * nedges;  // [kSub][nedges] (column, direction)
   const double step = 1.0 / (double)kSub;
-  if (threadIdx.x < 3 * kSub) {
-    (&count[0][0])[threadIdx.x] = 0;
-    (&span_base[0][0])[threadIdx.x] = 0;
-  }
-  if ((int)threadIdx.x < nedges) sedge[threadIdx.x] = edges[threadIdx.x];
+  for (int k = threadIdx.x; k < nedges; k += kRowThreads) sedge[k] = edges[k];
   __syncthreads();
-  int it = 0;
-  for (int j = blockIdx.y; j < H; j += gridDim.y) {
+  const long long units = (long long)H * spans;
+  for (long long u = blockIdx.x * (long long)kUnitWarps + warp; u < units; u += (long long)gridDim.x * kUnitWarps) {
+    const int j = (int)(u / spans), x0 = (int)(u - (long long)j * spans) * (kRuns * kRun);
+    const int q0 = 4 * x0, q1 = 4 * min(x0 + kRuns * kRun, W);
+    int count[kSub], base[kSub];
+#pragma unroll
+    for (int t = 0; t < kSub; ++t) count[t] = base[t] = 0;
     const double ylo = fma(0.5, step, (double)j), yhi = fma((double)kSub - 0.5, step, (double)j);
-    int inside[kPix];
-    for (int p = 0; p < kPix; ++p) inside[p] = 0;
     // a scanline below every vertex or at/above the highest one straddles no
     // edge (the half-open test compares y0 <= y and y1 <= y): coverage 0
     if (!(yhi < ymin || ylo >= ymax)) {
-      const int b = it % 3;
-      for (int task = threadIdx.x; task < nedges * kSub; task += kRowThreads) {
-        const int e = task >> 2, t = task & 3;
-        const double sy = fma((double)t + 0.5, step, (double)j);
-        const double4 E = sedge[e];
-        const bool below0 = E.y <= sy, below1 = E.w <= sy;
-        if (below0 == below1) continue;
-        const double tt = (sy - E.y) / (E.w - E.y);
-        const int qc = columns_left_of(fma(tt, E.z - E.x, E.x), W);
-        const int d = below0 ? 1 : -1;
-        if (qc >= q1) {
-          atomicAdd(&span_base[b][t], d);
-        } else if (qc > q0) {  // (qc <= q0: no column of the span is left of it)
-          const int k = atomicAdd(&count[b][t], 1);
-          cross_q[b][t][k] = qc;
-          cross_dir[b][t][k] = (signed char)d;
+      __syncwarp();  // the last unit's crossings have been read
+      for (int e0 = 0; e0 < nedges; e0 += 32) {
+        const bool have = e0 + lane < nedges;
+        const double4 E = have ? sedge[e0 + lane] : make_double4(0., 0., 0., 0.);
+#pragma unroll
+        for (int t = 0; t < kSub; ++t) {
+          const double sy = fma((double)t + 0.5, step, (double)j);
+          const bool below0 = E.y <= sy, below1 = E.w <= sy;
+          int qc = 0, d = 0;
+          if (have && below0 != below1) {
+            const double tt = (sy - E.y) / (E.w - E.y);
+            qc = columns_left_of(fma(tt, E.z - E.x, E.x), W);
+            d = below0 ? 1 : -1;
+          }
+          const bool right = d && qc >= q1, in = d && !right && qc > q0;  // (qc <= q0: no column of the span is left of it)
+          base[t] += __popc(__ballot_sync(0xffffffffu, right && d > 0)) - __popc(__ballot_sync(0xffffffffu, right && d < 0));
+          const unsigned m = __ballot_sync(0xffffffffu, in);
+          if (in) cross[t * nedges + count[t] + __popc(m & ((1u << lane) - 1u))] = make_int2(qc, d);
+          count[t] += __popc(m);
         }
       }
-      __syncthreads();
-      if (threadIdx.x < kSub) {
-        const int c = (b + 2) % 3;  // last read two rows ago (before this barrier); next written for the next row
-        count[c][threadIdx.x] = 0;
-        span_base[c][threadIdx.x] = 0;
-      }
+      __syncwarp();
+    }
+    // lane r: run r's coverage, or -1 where a crossing lies inside it
+    float run = 0.0f;
+    if (lane < kRuns) {
+      const int r0 = q0 + lane * 4 * kRun, r1 = r0 + 4 * kRun;
+      int n = 0;
+      bool crossed = false;
+#pragma unroll
       for (int t = 0; t < kSub; ++t) {
-        int wt = span_base[b][t];
-        int w[kPix * kSub];
-        bool partial = false;
-        const int m = count[b][t];
-        for (int k = 0; k < m; ++k) {
-          const int qc = cross_q[b][t][k];
-          const int d = cross_dir[b][t][k];
-          if (qc >= qp + kPix * kSub) {
-            wt += d;
-          } else if (qc > qp) {  // rare: a crossing among this thread's own columns
-            if (!partial)
-              for (int l = 0; l < kPix * kSub; ++l) w[l] = 0;
-            partial = true;
-            for (int l = 0; l < kPix * kSub; ++l) w[l] += qp + l < qc ? d : 0;
+        int wt = base[t];
+        for (int k = 0; k < count[t]; ++k) {
+          const int2 c = cross[t * nedges + k];
+          if (c.x >= r1) wt += c.y;
+          else if (c.x > r0) crossed = true;
+        }
+        n += kSub * (even_odd ? (wt & 1) : (wt != 0));
+      }
+      run = crossed ? -1.0f : (float)n * (1.0f / (float)(kSub * kSub));  // k / 16, exact
+    }
+    const int runs = (min(x0 + kRuns * kRun, W) - x0 + kRun - 1) / kRun;
+    for (int r = 0; r < runs; ++r) {
+      const float n = __shfl_sync(0xffffffffu, run, r);
+      const int px = x0 + r * kRun + lane * kPix;
+      if (n >= 0.0f) {
+        store_row(out, W, j, px, vec4, n, n, n, n);
+      } else {
+        const int qp = 4 * px;
+        int inside[kPix] = {0, 0, 0, 0};
+#pragma unroll
+        for (int t = 0; t < kSub; ++t) {
+          int wt = base[t];
+          const int m = count[t];
+          // the 16 columns' windings in a nibble each, 8 more than they are:
+          // up to seven crossings among them leave every nibble in 1 .. 15
+          constexpr unsigned long long kOnes = 0x1111111111111111ull;
+          unsigned long long w = 8 * kOnes;
+          int own = 0;
+          for (int k = 0; k < m; ++k) {
+            const int2 c = cross[t * nedges + k];
+            if (c.x >= qp + kPix * kSub) {
+              wt += c.y;
+            } else if (c.x > qp) {  // columns qp .. c.x - 1 are left of it
+              const unsigned long long left = kOnes >> (4 * (kPix * kSub - (c.x - qp)));
+              w += c.y > 0 ? left : 0ull - left;
+              ++own;
+            }
+          }
+          if (own <= 7) {
+            unsigned long long in;  // a one in each covered column's nibble
+            if (even_odd) {
+              in = (w & kOnes) ^ ((wt & 1) ? kOnes : 0ull);
+            } else if (wt > 7 || wt < -7) {
+              in = kOnes;
+            } else {
+              const unsigned long long x = w ^ (kOnes * (unsigned long long)(8 - wt));  // 0 where the winding is 0
+              in = (x | (x >> 1) | (x >> 2) | (x >> 3)) & kOnes;
+            }
+#pragma unroll
+            for (int p = 0; p < kPix; ++p) inside[p] += __popc((unsigned)(in >> (16 * p)) & 0xffffu);
+          } else {  // column by column
+#pragma unroll
+            for (int p = 0; p < kPix; ++p)
+              for (int l = p * kSub; l < (p + 1) * kSub; ++l) {
+                int v = wt;
+                for (int k = 0; k < m; ++k) {
+                  const int2 c = cross[t * nedges + k];
+                  if (c.x > qp && c.x < qp + kPix * kSub && qp + l < c.x) v += c.y;
+                }
+                inside[p] += even_odd ? (v & 1) : (v != 0);
+              }
           }
         }
-        add_row(wt, w, partial, even_odd, inside);
+        constexpr float u = 1.0f / (float)(kSub * kSub);  // k / 16, exact
+        store_row(out, W, j, px, vec4, (float)inside[0] * u, (float)inside[1] * u, (float)inside[2] * u, (float)inside[3] * u);
       }
-      ++it;
     }
-    store_row(out, W, j, px, vec4, inside);
   }
 }
 
@@ -267,7 +335,8 @@ __global__ void __launch_bounds__(kRowThreads) k_mask_polygon_chunked(int W, int
       for (int t = 0; t < kSub; ++t) add_row(wt[t] + span_base[t], w[t], partial[t], even_odd, inside);
       __syncthreads();  // span_base is reset for the next row only after every read
     }
-    store_row(out, W, j, px, vec4, inside);
+    constexpr float u = 1.0f / (float)(kSub * kSub);  // k / 16, exact
+    store_row(out, W, j, px, vec4, (float)inside[0] * u, (float)inside[1] * u, (float)inside[2] * u, (float)inside[3] * u);
   }
 }
 
@@ -346,9 +415,14 @@ extern "C" pt_status pt_mask_ellipse(pt_ctx *ctx, uint32_t width, uint32_t heigh
     if ((st = mask_begin(ctx)) != PT_OK) return st;
     const double sn = std::sin(angle_rad), cs = std::cos(angle_rad);
     const long long blocks = std::min<long long>(((long long)npx + 255) / 256, (long long)ctx->sms * 16);
+    // (radii whose squares leave the range of doubles take the formula everywhere)
+    const double rmin = std::min(radius_x, radius_y), band = half_width_px / rmin;
+    const bool plain = rmin >= 1e-100 && std::max(radius_x, radius_y) <= 1e100;
+    const double far2 = plain ? (1.0 + band) * (1.0 + band) * (1.0 + 1e-9) : INFINITY;
+    const double near2 = plain && band < 1.0 ? (1.0 - band) * (1.0 - band) * (1.0 - 1e-9) : -1.0;
     cudaEventRecord(ctx->ev[1], ctx->stream);
     k_mask_ellipse<<<(unsigned)blocks, 256, 0, ctx->stream>>>((int)width, (int)height, center_x, center_y,
-                                                             radius_x, radius_y, sn, cs, half_width_px, out);
+                                                             radius_x, radius_y, sn, cs, half_width_px, far2, near2, out);
     cudaEventRecord(ctx->ev[2], ctx->stream);
     return mask_finish(ctx, npx, dev, mask, out, 1);
   });
@@ -404,11 +478,14 @@ extern "C" pt_status pt_mask_polygon(pt_ctx *ctx, uint32_t width, uint32_t heigh
       k_mask_polygon_chunked<<<grid, kRowThreads, 0, ctx->stream>>>((int)width, (int)height, dedges,
                                                                     (int)n_points, even_odd, ymin, ymax, vec4, out);
     } else {
-      // two waves of 4 resident blocks per SM, each block looping over rows of its span
-      const uint32_t rows = std::max<uint32_t>(1u, (uint32_t)(ctx->sms * 8) / spans);
-      const dim3 grid(spans, std::min<uint32_t>(std::min<uint32_t>(height, rows), 65535u));
-      k_mask_polygon_rows<<<grid, kRowThreads, 0, ctx->stream>>>((int)width, (int)height, dedges, (int)n_points,
-                                                                 even_odd, ymin, ymax, vec4, out);
+      // a unit a warp, at most eight blocks an SM
+      const int spans = (int)((width + kRuns * kRun - 1) / (kRuns * kRun));
+      const long long units = (long long)height * spans;
+      const unsigned blocks = (unsigned)std::min<long long>((units + kUnitWarps - 1) / kUnitWarps, (long long)ctx->sms * 8);
+      ce = cudaFuncSetAttribute(k_mask_polygon_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem(kRowThreads));
+      if (ce != cudaSuccess) return mfail(ctx, PT_LAUNCH_FAILED, cudaGetErrorString(ce));
+      k_mask_polygon_rows<<<blocks, kRowThreads, rows_smem((int)n_points), ctx->stream>>>(
+          (int)width, (int)height, dedges, (int)n_points, even_odd, ymin, ymax, vec4, spans, out);
     }
     cudaEventRecord(ctx->ev[2], ctx->stream);
     return mask_finish(ctx, npx, dev, mask, out, 1);
