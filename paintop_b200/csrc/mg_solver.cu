@@ -127,8 +127,14 @@ __global__ void __launch_bounds__(kTx * kTy) k_mg_assemble(const Geo *__restrict
       a[k] = 0;
       continue;
     }
-    const bool in = W >= 3 && H >= 3 && i > 0 && j > 0 && i < W - 1 && j < H - 1 && f.mask[q] > 0.5f;
+    auto interior = [&](int x, int y) {
+      return W >= 3 && H >= 3 && x > 0 && y > 0 && x < W - 1 && y < H - 1 && f.mask[(size_t)y * W + x] > 0.5f;
+    };
+    const bool in = interior(i, j);
     a[k] = in ? 1 : 0;
+    // u is read at interior cells and their neighbours, b' at interior cells:
+    // elsewhere neither is written (all cells of 4096 x 4096 took 285 us)
+    if (!in && !interior(i - 1, j) && !interior(i + 1, j) && !interior(i, j - 1) && !interior(i, j + 1)) continue;
     for (int c = 0; c < C; ++c) {  // a thread's channels are adjacent in the interleaved inputs
       const double av = (double)f.anchor[q * C + c];
       u0[c * N + k] = av;
@@ -141,7 +147,7 @@ __global__ void __launch_bounds__(kTx * kTy) k_mg_assemble(const Geo *__restrict
                          (double)gd[(q + W) * C + c];
         bv = fma(4.0, -ctr, s);
       }
-      b0[c * N + k] = in ? fma(g.lambda, -av, bv) : 0.0;
+      if (in) b0[c * N + k] = fma(g.lambda, -av, bv);
       if (w0) w0[c * N + k] = (in && f.guess) ? (double)f.guess[q * C + c] : av;
     }
   }
@@ -498,12 +504,10 @@ __global__ void __launch_bounds__(kStripWarps * 32) k_mg_update(const Geo *__res
   for (int j = t.y0; j < t.y1; ++j) {
     const long long o = at + (long long)j * g.P;
     const unsigned a = nibble(*reinterpret_cast<const uint32_t *>(act + g.o + (long long)j * g.P + t.x0));
-    if (!a) continue;
     const Row v = x ? ld_row(x + o) : row0();
     Row64 w = ld_row64(u + o);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (a & (1u << i)) w.v[i] = fma(s, (double)v.v[i], w.v[i]);
+    for (int i = 0; i < 4; ++i) w.v[i] = a & (1u << i) ? fma(s, (double)v.v[i], w.v[i]) : w.v[i];
     st_row64(u + o, w);
   }
 }
@@ -1005,14 +1009,28 @@ __global__ void __launch_bounds__(kStripWarps * 32) k_cg_dot(const Geo *__restri
   if (unit_sum(g, c, sums, &rho)) new_rho(sums.sc + (long long)(g.unit0 + c) * S_N, rho, first);
 }
 
-// p' = z + beta p (p' = z on the first iteration), q = A_0 p' at active cells,
-// p.q. The strips beside read p, so p' is another array.
+// A_0 p at a row's active cells: d p - (left + right + up + down)
+__device__ __forceinline__ Row apply_row(const Row &k, const Row &up, const Row &dn, unsigned a, float d) {
+  const float l = from_left(k.v[3]), r = from_right(k.v[0]);
+  Row v;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float sum = (((i ? k.v[i ? i - 1 : 0] : l) + (i < 3 ? k.v[i < 3 ? i + 1 : 3] : r)) + up.v[i]) + dn.v[i];
+    v.v[i] = a & (1u << i) ? d * k.v[i] - sum : 0.0f;
+  }
+  return v;
+}
+
+// p' = z + beta p (p' = z on the first iteration) and p'.q, q = A_0 p' at active
+// cells. The strips beside read p, so p' is another array. q is not stored: the
+// step evaluates it again from p', which it reads anyway (8 of 41 bytes a cell
+// and iteration saved).
 __global__ void __launch_bounds__(kStripWarps * 32) k_cg_apply(const Geo *__restrict__ geo,
                                                                const int4 *__restrict__ bmap, const Geo one,
                                                                const uint8_t *__restrict__ flags,
                                                                const uint8_t *__restrict__ act,
                                                                const float *__restrict__ z, const float *__restrict__ p,
-                                                               float *__restrict__ pn, float *__restrict__ q,
+                                                               float *__restrict__ pn,
                                                                const double *__restrict__ run, Sums sums, int first) {
   const int4 bt = entry_of(bmap, one);
   const int c = blockIdx.z, lane = threadIdx.x & 31;
@@ -1044,16 +1062,9 @@ __global__ void __launch_bounds__(kStripWarps * 32) k_cg_apply(const Geo *__rest
       fa = fetch_a(y + 1);
       if (t.own && y >= t.y0 && y < t.y1) st_row(pn + at + (long long)y * g.P, n);
       const int j = y - 1;
-      const float l = from_left(k.v[3]), r = from_right(k.v[0]);
+      const Row v = apply_row(k, m, n, ak, d);
       if (j >= t.y0) {
-        Row v;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float sum = (((i ? k.v[i ? i - 1 : 0] : l) + (i < 3 ? k.v[i < 3 ? i + 1 : 3] : r)) + m.v[i]) + n.v[i];
-          v.v[i] = ak & (1u << i) ? d * k.v[i] - sum : 0.0f;
-        }
         if (t.own) {
-          st_row(q + at + (long long)j * g.P, v);
 #pragma unroll
           for (int i = 0; i < 4; ++i) acc = fma((double)k.v[i], (double)v.v[i], acc);
         }
@@ -1071,14 +1082,14 @@ __global__ void __launch_bounds__(kStripWarps * 32) k_cg_apply(const Geo *__rest
   if (unit_sum(g, c, sums, &pq)) sc[S_PQ] = pq;
 }
 
-// x += alpha p, r -= alpha q (alpha = rho / p.q); ||r||^2
+// x += alpha p, r -= alpha q (alpha = rho / p.q, q = A_0 p); ||r||^2
 __global__ void __launch_bounds__(kStripWarps * 32) k_cg_step(const Geo *__restrict__ geo,
                                                               const int4 *__restrict__ bmap, const Geo one,
                                                               const uint8_t *__restrict__ flags,
-                                                              const float *__restrict__ p, const float *__restrict__ q,
-                                                              float *__restrict__ x, float *__restrict__ r,
-                                                              const double *__restrict__ run, Sums sums,
-                                                              double *__restrict__ rr) {
+                                                              const uint8_t *__restrict__ act,
+                                                              const float *__restrict__ p, float *__restrict__ x,
+                                                              float *__restrict__ r, const double *__restrict__ run,
+                                                              Sums sums, double *__restrict__ rr) {
   const int4 bt = entry_of(bmap, one);
   const int c = blockIdx.z, lane = threadIdx.x & 31;
   if (c >= bt.z || run[bt.y + c] == 0.0) return;  // a stopped unit: x and r stay
@@ -1086,32 +1097,55 @@ __global__ void __launch_bounds__(kStripWarps * 32) k_cg_step(const Geo *__restr
   const double *sc = sums.sc + (long long)(g.unit0 + c) * S_N;
   Strip t;
   if (strip_of(g, flags, t)) {
-    const float alpha = sc[S_PQ] > 0.0 ? (float)(sc[S_RHO] / sc[S_PQ]) : 0.0f;
+    const float alpha = sc[S_PQ] > 0.0 ? (float)(sc[S_RHO] / sc[S_PQ]) : 0.0f, d = g.d;
     const long long at = g.oc + (long long)c * g.P * g.H + t.x0;
+    const uint8_t *a0 = act + g.o + t.x0;
+    // p was written only in bands with active cells: elsewhere it is 0
+    auto fetch = [&](int y, unsigned a) {
+      Row v = t.in && y >= 0 && y < g.H ? ld_row(p + at + (long long)y * g.P) : row0();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v.v[i] = a & (1u << i) ? v.v[i] : 0.0f;
+      return v;
+    };
+    auto flag = [&](int y) {
+      return t.in && y >= 0 && y < g.H ? nibble(*reinterpret_cast<const uint32_t *>(a0 + (long long)y * g.P)) : 0u;
+    };
     double acc = 0.0;
+    unsigned a = flag(t.y0);
+    Row up = fetch(t.y0 - 1, flag(t.y0 - 1)), k = fetch(t.y0, a);
     // the rows of a band in two halves, each half's loads before its stores
-    for (int j0 = t.y0; j0 < t.y1; j0 += kBand / 2) {
-      const int n = min(kBand / 2, t.y1 - j0);
-      if (t.own) {
-        Row P[kBand / 2], Q[kBand / 2], X[kBand / 2], S[kBand / 2];
+    constexpr int kHalf = kBand / 2;
+    for (int j0 = t.y0; j0 < t.y1; j0 += kHalf) {
+      const int n = min(kHalf, t.y1 - j0);
+      unsigned an[kHalf];
+      Row P[kHalf], X[kHalf], S[kHalf];
 #pragma unroll
-        for (int k = 0; k < kBand / 2; ++k) {
-          const long long o = at + (long long)(j0 + min(k, n - 1)) * g.P;
-          P[k] = ld_row(p + o); Q[k] = ld_row(q + o); X[k] = ld_row(x + o); S[k] = ld_row(r + o);
-        }
+      for (int q = 0; q < kHalf; ++q) an[q] = flag(j0 + q + 1);
 #pragma unroll
-        for (int k = 0; k < kBand / 2; ++k) {
-          if (k >= n) break;
-          const long long o = at + (long long)(j0 + k) * g.P;
+      for (int q = 0; q < kHalf; ++q) {
+        const long long o = at + (long long)(j0 + min(q, n - 1)) * g.P;
+        P[q] = fetch(j0 + q + 1, an[q]);
+        X[q] = t.own ? ld_row(x + o) : row0();
+        S[q] = t.own ? ld_row(r + o) : row0();
+      }
+#pragma unroll
+      for (int q = 0; q < kHalf; ++q) {
+        if (q >= n) break;
+        const Row Q = apply_row(k, up, P[q], a, d);
+        if (t.own) {
+          const long long o = at + (long long)(j0 + q) * g.P;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            X[k].v[i] = X[k].v[i] + alpha * P[k].v[i];
-            S[k].v[i] = S[k].v[i] - alpha * Q[k].v[i];
-            acc = fma((double)S[k].v[i], (double)S[k].v[i], acc);
+            X[q].v[i] = X[q].v[i] + alpha * k.v[i];
+            S[q].v[i] = S[q].v[i] - alpha * Q.v[i];
+            acc = fma((double)S[q].v[i], (double)S[q].v[i], acc);
           }
-          st_row(x + o, X[k]);
-          st_row(r + o, S[k]);
+          st_row(x + o, X[q]);
+          st_row(r + o, S[q]);
         }
+        up = k;
+        k = P[q];
+        a = an[q];
       }
       const int j = j0 + n - 1;
       if ((j & (kBand - 1)) == kBand - 1 || j == t.y1 - 1) {
@@ -1125,7 +1159,8 @@ __global__ void __launch_bounds__(kStripWarps * 32) k_cg_step(const Geo *__restr
 }
 
 // out = interleave(u) at interior cells, the anchor elsewhere (bit for bit);
-// level-0 tiles, grid.z 1
+// level-0 tiles, grid.z 1. A thread takes four consecutive values of a row of
+// the interleaved image; whole where both images allow (16-byte alignment).
 __global__ void __launch_bounds__(kTx * kTy) k_mg_emit(const Geo *__restrict__ geo,
                                                        const int4 *__restrict__ bmap, const Geo one,
                                                        const Io *__restrict__ io, const uint8_t *__restrict__ act,
@@ -1134,16 +1169,47 @@ __global__ void __launch_bounds__(kTx * kTy) k_mg_emit(const Geo *__restrict__ g
   const int gi = bt.x;
   const Geo g = bmap ? geo[gi] : one;
   const Io f = io[gi];
-  const int C = g.C, W = g.W, H = g.H, b = tile_b(g), i = (b % g.gx) * kTx + threadIdx.x;
-  const size_t N = (size_t)g.P * H;
+  const int C = g.C, W = g.W, H = g.H, b = tile_b(g);
+  const size_t N = (size_t)g.P * H, row = (size_t)W * C;
   const uint8_t *a = act + g.o;
   const double *u0 = u + g.oc;
-  for (int j = (b / g.gx) * kTy + threadIdx.y; j < H && i < W; j += g.gy * kTy) {
-    const size_t q = (size_t)j * W + i, k = (size_t)j * g.P + i;
-    const bool in = a[k] != 0;
-    for (int c = 0; c < C; ++c)  // a warp writes 32 whole pixels: C * 32 adjacent floats
-      f.out[q * C + c] = in ? (float)u0[c * N + k] : f.anchor[q * C + c];
-  }
+  const int first = (b % g.gx) * kTx, values = min(kTx, W - first) * C;
+  const bool whole = ((reinterpret_cast<uintptr_t>(f.out) | reinterpret_cast<uintptr_t>(f.anchor)) & 15) == 0 && row % 4 == 0;
+  for (int j = (b / g.gx) * kTy + threadIdx.y; j < H; j += g.gy * kTy)
+    // the tile's columns hold C values each: the lanes walk over them
+    for (int e = 4 * threadIdx.x; e < values; e += 4 * kTx) {
+      int i = first + e / C, c = e % C;
+      const int n = min(4, values - e);
+      float v[4];
+      const size_t o = j * row + (size_t)first * C + e;
+      const float *from = f.anchor + o;
+      if (whole && n == 4) {
+        const float4 q = *reinterpret_cast<const float4 *>(from);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = k < n ? from[k] : 0.0f;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (k < n) {
+          const size_t at = (size_t)j * g.P + i;
+          if (a[at]) v[k] = (float)u0[c * N + at];
+        }
+        if (++c == C) {
+          c = 0;
+          ++i;
+        }
+      }
+      float *to = f.out + o;
+      if (whole && n == 4) {
+        *reinterpret_cast<float4 *>(to) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (k < n) to[k] = v[k];
+      }
+    }
 }
 
 // ---- host ----------------------------------------------------------------------
@@ -1533,7 +1599,7 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
   const uint8_t *fl0 = m.at<uint8_t>(m.lv[0].flags);
   double *u = m.at<double>(m.u), *bl = m.at<double>(m.bl), *r64 = m.at<double>(m.r64), *red = m.at<double>(m.red),
          *sc = m.at<double>(m.sc), *scale = m.at<double>(m.scale), *run = m.at<double>(m.run);
-  float *x = m.at<float>(m.x), *r = m.at<float>(m.r), *z = m.at<float>(m.z), *q = m.at<float>(m.q);
+  float *x = m.at<float>(m.x), *r = m.at<float>(m.r), *z = m.at<float>(m.z);
   float *pp[2] = {m.at<float>(m.p[0]), m.at<float>(m.p[1])};
   const Sums sums{m.at<double>(m.part), m.at<unsigned>(m.done), sc};
   k_mg_assemble<<<m.grid(A, 1), kBlock2, 0, m.st>>>(m.geo(A), m.bmap(A), A.one, iod, act0, u, bl,
@@ -1630,8 +1696,8 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
     float *p = pp[kind == 1 ? 0 : 1], *pn = pp[kind == 1 ? 1 : 0];
     const int first = kind == 0;
     vcycle(m, first);
-    k_cg_apply<<<gs, kStrip, 0, m.st>>>(g0, b0, S0.one, fl0, act0, z, p, pn, q, run, sums, first);
-    k_cg_step<<<gs, kStrip, 0, m.st>>>(g0, b0, S0.one, fl0, pn, q, x, r, run, sums, red);
+    k_cg_apply<<<gs, kStrip, 0, m.st>>>(g0, b0, S0.one, fl0, act0, z, p, pn, run, sums, first);
+    k_cg_step<<<gs, kStrip, 0, m.st>>>(g0, b0, S0.one, fl0, act0, pn, x, r, run, sums, red);
     m.launches += 2;
     per_iteration = m.launches - l0;
     return cudaGetLastError();
