@@ -140,9 +140,10 @@ struct Tile {
 // How a cluster of thread blocks holds a region (rbsor_cluster.cu). The box is
 // cut into patches of 8 columns x `rows` rows from (x0, y0), one per thread: nq
 // across, and m rows of patches in each of the n blocks (the last one what is
-// left of the box's bm). limit: patches a block may hold.
+// left of the box's bm). limit: patches a block may hold; option: which of the
+// splits below it is.
 struct Route {
-  int n, x0, y0, nq, bm, m, rows, limit;
+  int n, x0, y0, nq, bm, m, rows, limit, option;
 };
 
 constexpr int kClusterMax = 16;       // blocks per cluster
@@ -150,34 +151,43 @@ constexpr int kClusterMost = 480;     // patches per block at most (a warp more 
 constexpr int kClusterLeast = 224;    // ... and the least that are asked for before a second block
 
 // The split of a region with this bounding box, or false when it does not fit
-// a cluster. It depends on the box alone, so a system's partial sums, and with
-// them its results, do not depend on what else the call solves.
-__host__ __device__ inline bool cluster_route(int bx0, int by0, int bx1, int by1, Route *r) {
+// a cluster; `many`: the call fills the GPU with clusters. A box inside another
+// never takes more blocks, larger ones or a later split than that one (it has no
+// more columns or rows of patches), which plan_clusters counts on.
+__host__ __device__ inline bool cluster_route(int bx0, int by0, int bx1, int by1, bool many, Route *r) {
   if (bx1 < bx0 || by1 < by0) return false;
   const int x0 = (bx0 - 1) & ~7, y0 = by0 & ~1;  // an even first row: a row's colours sit alike in every patch
   const int nq = (bx1 + 1 - x0) / 8 + 1, bh = by1 + 1 - y0;
-  // two-row patches halve a half-sweep's latency, four-row ones hold more and
-  // convert less; blocks of the least size leave an SM room for a second one
+  // Two-row patches halve a half-sweep's latency (512 x 512 RGB: 7.0 ms, with
+  // four rows 9.0; 97 x 71 RGB: 0.53 and 0.69). Four-row ones need half the
+  // blocks, so that twice the clusters run at a time, and convert less: `many`
+  // tries them first (128 of 256 x 256: 7.3 ms, with two rows 9.4). Blocks of
+  // the least size leave an SM room for a second one.
   for (int k = 0; k < 4; ++k) {
-    const int rows = k & 1 ? 4 : 2, t = k < 2 ? kClusterLeast : kClusterMost;
+    const int rows = ((k & 1) != 0) != many ? 4 : 2, t = k < 2 ? kClusterLeast : kClusterMost;
     const int bm = (bh + rows - 1) / rows;
     if (nq > t || (bm + t / nq - 1) / (t / nq) > kClusterMax) continue;
     // even shares; of a region that needs more than the least blocks, to all 16
     const int n = k > 1 ? kClusterMax : (bm + t / nq - 1) / (t / nq);
     const int m = (bm + n - 1) / n;
-    r->x0 = x0; r->y0 = y0; r->nq = nq; r->bm = bm; r->m = m; r->rows = rows; r->limit = t;
+    r->x0 = x0; r->y0 = y0; r->nq = nq; r->bm = bm; r->m = m; r->rows = rows; r->limit = t; r->option = k;
     r->n = (bm + m - 1) / m;
     return true;
   }
   return false;
 }
 
-// A block's windows in shared memory (rbsor_cluster.cu): four arrays of first
-// and last rows, (m + 1) nq <= most + nq <= 2 most groups of four, and four of
-// edges, m (nq + 2) <= 3 most pairs. Fixed places, so that a thread's accesses
-// differ by constants; two blocks of the least size fit an SM.
-constexpr int kWinRows = 16 * 2 * kClusterMost, kWinEdges = 8 * 3 * kClusterMost;
-constexpr int kClusterSmem = 4 * kWinRows + 4 * kWinEdges;
+// A block's windows in shared memory (rbsor_cluster.cu), for patches up to
+// `limit`: four arrays of first and last rows, (m + 1) nq <= limit + nq <= 2
+// limit groups of four, and four of edges, m (nq + 2) <= 3 limit pairs. Fixed
+// places, so that a thread's accesses differ by constants. Four-row patches also
+// keep their right-hand side there, 128 bytes each (in registers it spilled:
+// 9.5 against 7.3 ms on 128 regions of 256 x 256). Two blocks of the least size
+// fit an SM.
+__host__ __device__ constexpr int win_rows(int limit) { return 16 * 2 * limit; }
+__host__ __device__ constexpr int win_edges(int limit) { return 8 * 3 * limit; }
+__host__ __device__ constexpr int win_bytes(int limit) { return 4 * win_rows(limit) + 4 * win_edges(limit); }
+constexpr int cluster_smem(int rows, int limit) { return win_bytes(limit) + (rows == 4 ? 128 * limit : 0); }
 
 struct KParams {
   const SysDesc *sys;
@@ -208,6 +218,7 @@ struct KParams {
   int *rsize;              // per pixel: region size, at the root
   int *rmax;               // per RegionDesc: largest region size
   Route *route;            // per system: its cluster's split, n = 0 for k_solve's (null: all are)
+  bool many;               // the call fills the GPU with clusters (cluster_route)
 };
 
 }  // namespace ptk

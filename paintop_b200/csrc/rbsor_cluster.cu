@@ -8,9 +8,10 @@
 // Here a system's region stays on the chip from its first sweep to its last: a
 // cluster of n blocks holds the bounding box of its interior cells, a band of
 // rows each. A thread owns a patch of 8 columns x R rows (both colours) whose
-// correction and right-hand side live in its registers; shared memory carries
-// only what other threads read, a patch's first and last rows and one value a
-// row for the patch beside it. A band's first and last rows also go into the
+// correction lives in its registers, and the right-hand side of two-row patches
+// too (four-row ones keep it in shared memory of their own); otherwise shared
+// memory carries only what other threads read, a patch's first and last rows and
+// one value a row for the patch beside it. A band's first and last rows also go into the
 // neighbour block's shared memory, by stores that count their bytes off a
 // barrier there (st.async): a block waits for its two neighbours' rows, not for
 // the cluster, and nobody for a fence. No cell is swept twice (there are no
@@ -35,8 +36,6 @@
 // steps, decided from the same sums by the same code; every wait for another
 // warp's or block's data is bounded (bar_wait). The wall budget is tested by
 // the first block once a step and passed on with its sums.
-#include <initializer_list>
-
 #include "rbsor.cuh"
 #include "rbsor_device.cuh"
 #include "rbsor_launch.h"
@@ -125,12 +124,14 @@ __device__ __forceinline__ double residual(float l, float r, float u, float dn, 
   return fma(-dd, (double)e, ns) - (double)g;
 }
 
-// A patch's state in registers: e and g by colour and row, four cells each;
+// A patch's state in registers: e (and g) by colour and row, four cells each;
 // bit 16 h + 4 r + i of fl: cell i of colour h in row r is interior.
 template <int R>
 struct Patch {
-  float4 e[2][R], g[2][R];
+  float4 e[2][R];
+  float4 g[R == 2 ? 2 : 1][R == 2 ? 2 : 1];  // two-row patches: the right-hand side
   uint32_t fl;
+  unsigned ag;                               // four-row ones: its address in shared memory (rhs_row)
 };
 
 // The shared-memory windows of a block. TOP(h, j), BOT(h, j): colour h of the
@@ -138,8 +139,12 @@ struct Patch {
 // last at BOT j + 1; BOT 0 and TOP m are the neighbour blocks'. RIGHT(h, j, v):
 // the values of patch (j, v) that the patch to its right reads (the last of
 // each row whose cells sit one column right), LEFT the ones for its left.
-// (As shared-memory addresses, kWinRows and kWinEdges apart by colour.)
-enum Window { W_TOP = 0, W_BOT = 2 * kWinRows, W_RIGHT = 4 * kWinRows, W_LEFT = 4 * kWinRows + 2 * kWinEdges };
+// (As shared-memory addresses, ROWS and EDGES bytes apart by colour.)
+template <int T>
+struct Windows {
+  static constexpr int ROWS = win_rows(T), EDGES = win_edges(T);
+  static constexpr int TOP = 0, BOT = 2 * ROWS, RIGHT = 4 * ROWS, LEFT = 4 * ROWS + 2 * EDGES, G = 4 * ROWS + 4 * EDGES;
+};
 
 __device__ __forceinline__ void st_win(unsigned a, const float4 &v) {
   asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
@@ -177,16 +182,24 @@ __device__ __forceinline__ void row_neighbours(const Patch<R> &p, const Near &b,
   }
 }
 
+// Row r of colour H's right-hand side; in shared memory a warp's groups of four
+// lie side by side.
+template <int H, int T, int R>
+__device__ __forceinline__ float4 rhs_row(const Patch<R> &p, int r) {
+  if constexpr (R == 2) return p.g[H][r];
+  else return ld_rows(p.ag + (unsigned)((H * R + r) * 16 * T));
+}
+
 // One half-sweep of colour H over the thread's patch. FULL: every cell of the
 // warp's patches is interior, and no flag is tested.
-template <int H, bool FULL, int R>
+template <int H, bool FULL, int T, int R>
 __device__ __forceinline__ void relax(Patch<R> &p, const Near &b, float w, float inv) {
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const float4 up = r == 0 ? b.up : p.e[1 - H][r - 1], dn = r == R - 1 ? b.dn : p.e[1 - H][r + 1];
     float n[5];
     row_neighbours<H>(p, b, r, n);
-    const float4 g = p.g[H][r], e = p.e[H][r];
+    const float4 g = rhs_row<H, T>(p, r), e = p.e[H][r];
     const uint32_t f = p.fl >> (16 * H + 4 * r);
     float4 ne = e;
     if (FULL || (f & 1u)) ne.x = fmaf(w, ((((n[0] + n[1]) + up.x) + dn.x) - g.x) * inv - e.x, e.x);
@@ -199,7 +212,7 @@ __device__ __forceinline__ void relax(Patch<R> &p, const Near &b, float w, float
 
 // The sum of squares of the FP64 residual at colour H's interior cells, whose
 // values are e[].
-template <int H, bool FULL, int R>
+template <int H, bool FULL, int T, int R>
 __device__ __forceinline__ double squares(const Patch<R> &p, const float4 (&e)[R], const Near &b, double dd) {
   double part = 0.0;
 #pragma unroll
@@ -207,7 +220,7 @@ __device__ __forceinline__ double squares(const Patch<R> &p, const float4 (&e)[R
     const float4 up = r == 0 ? b.up : p.e[1 - H][r - 1], dn = r == R - 1 ? b.dn : p.e[1 - H][r + 1];
     float n[5];
     row_neighbours<H>(p, b, r, n);
-    const float4 g = p.g[H][r];
+    const float4 g = rhs_row<H, T>(p, r);
     const uint32_t f = p.fl >> (16 * H + 4 * r);
     const double x0 = residual(n[0], n[1], up.x, dn.x, e[r].x, g.x, dd), x1 = residual(n[1], n[2], up.y, dn.y, e[r].y, g.y, dd),
                  x2 = residual(n[2], n[3], up.z, dn.z, e[r].z, g.z, dd), x3 = residual(n[3], n[4], up.w, dn.w, e[r].w, g.w, dd);
@@ -336,7 +349,7 @@ __device__ __forceinline__ void keep_books(const KParams &P, Shared &sh, unsigne
   }
 }
 
-template <int R>
+template <int R, int T>
 __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, Shared &sh, const int sys,
                                              const unsigned rank, const int TW, const int TH, unsigned char *smem) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -348,7 +361,7 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
   const int py = rt.y0 + (j0 + jr) * R, gi = (rt.x0 >> 1) + 4 * v;  // its first row, its plane index
   const bool to_up = mine && jr == 0 && rank > 0, to_dn = mine && jr == mr - 1 && (int)rank + 1 < n;
 
-  for (int k = tid; k < kClusterSmem / 4; k += blockDim.x) reinterpret_cast<float *>(smem)[k] = 0.0f;
+  for (int k = tid; k < win_bytes(T) / 4; k += blockDim.x) reinterpret_cast<float *>(smem)[k] = 0.0f;
   const unsigned bar0 = (unsigned)__cvta_generic_to_shared(sh.bars);
   const unsigned row_bytes = 16u * (unsigned)nq;
   if (tid == 0) {
@@ -370,22 +383,29 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
 
   // ---- the patch: interior flags and the right-hand side; e = 0. Tiles
   // without interior cells were not assembled: their cells are not interior.
+  using W = Windows<T>;
   Patch<R> p;
   p.fl = 0;
+  p.ag = (unsigned)__cvta_generic_to_shared(smem) + W::G + 16u * (unsigned)min(tid, T - 1);
+  auto set_rhs = [&](int h, int r, const float4 &v) {
+    if constexpr (R == 2) p.g[h][r] = v;
+    else if (!books) st_win(p.ag + (unsigned)((h * R + r) * 16 * T), v);
+  };
 #pragma unroll
   for (int h = 0; h < 2; ++h)
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
       p.e[h][r] = z;
-      p.g[h][r] = z;
+      float4 g = z;
       const int y = py + r;
       if (mine && y < d.H && gi < d.pw && P.tcount[d.tile0 + (y / TH) * d.ntx + (2 * gi) / TW] > 0) {
         const uint32_t c = *reinterpret_cast<const uint32_t *>(P.cell + pool(h, r));
         const uint32_t f = (c & 1u) | ((c >> 7) & 2u) | ((c >> 14) & 4u) | ((c >> 21) & 8u);
         p.fl |= f << (16 * h + 4 * r);
-        if (f) p.g[h][r] = __ldcg(reinterpret_cast<const float4 *>(P.g + pool(h, r)));
+        if (f) g = __ldcg(reinterpret_cast<const float4 *>(P.g + pool(h, r)));
       }
+      set_rhs(h, r, g);
     }
   cluster_sync();  // every block's windows are zeroed and its barriers set before a neighbour stores
   if (books) {
@@ -413,17 +433,17 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
     float2 right, left;
     if (h) edges<R, 1>(p, right, left);
     else edges<R, 0>(p, right, left);
-    st_win(aw + W_TOP + h * kWinRows, a);
-    st_win(aw + below + W_BOT + h * kWinRows, b);
-    st_win(ae + W_RIGHT + h * kWinEdges, right);
-    st_win(ae + W_LEFT + h * kWinEdges, left);
+    st_win(aw + W::TOP + h * W::ROWS, a);
+    st_win(aw + below + W::BOT + h * W::ROWS, b);
+    st_win(ae + W::RIGHT + h * W::EDGES, right);
+    st_win(ae + W::LEFT + h * W::EDGES, left);
     if (to_up) {
-      if (async) st_async(to_top + W_TOP + h * kWinRows, a, bars_up + 8u * (B_DN + h));
-      else st_remote(to_top + W_TOP + h * kWinRows, a);
+      if (async) st_async(to_top + W::TOP + h * W::ROWS, a, bars_up + 8u * (B_DN + h));
+      else st_remote(to_top + W::TOP + h * W::ROWS, a);
     }
     if (to_dn) {
-      if (async) st_async(to_bot + W_BOT + h * kWinRows, b, bars_dn + 8u * (B_UP + h));
-      else st_remote(to_bot + W_BOT + h * kWinRows, b);
+      if (async) st_async(to_bot + W::BOT + h * W::ROWS, b, bars_dn + 8u * (B_UP + h));
+      else st_remote(to_bot + W::BOT + h * W::ROWS, b);
     }
   };
   // bit h: the parity of colour h's rows; bit 2: of the meetings; bits 3, 4: of
@@ -454,8 +474,8 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
     phase ^= 4u;
   };
   auto near = [&](int o) {
-    return Near{ld_rows(aw + W_BOT + o * kWinRows), ld_rows(aw + below + W_TOP + o * kWinRows),
-                ld_edge(ae - 8 + W_RIGHT + o * kWinEdges), ld_edge(ae + 8 + W_LEFT + o * kWinEdges)};
+    return Near{ld_rows(aw + W::BOT + o * W::ROWS), ld_rows(aw + below + W::TOP + o * W::ROWS),
+                ld_edge(ae - 8 + W::RIGHT + o * W::EDGES), ld_edge(ae + 8 + W::LEFT + o * W::EDGES)};
   };
 
   const float w = d.omega, inv = d.inv_denom;
@@ -505,14 +525,14 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
 #pragma unroll
       for (int r = 0; r < R; ++r) old[r] = p.e[0][r];
       if (!last) {
-        if (full) relax<0, true>(p, b, w, inv);
-        else if (red_any) relax<0, false>(p, b, w, inv);
+        if (full) relax<0, true, T>(p, b, w, inv);
+        else if (red_any) relax<0, false, T>(p, b, w, inv);
         if (mine) show(0, true);
         arrive(B_MEET);
       }
       if (j > 0) {
-        if (full) carry += squares<0, true>(p, old, b, dd);
-        else if (red_any) carry += squares<0, false>(p, old, b, dd);
+        if (full) carry += squares<0, true, T>(p, old, b, dd);
+        else if (red_any) carry += squares<0, false, T>(p, old, b, dd);
         give(t, j - 1, carry);
       }
       if (last) break;
@@ -520,12 +540,12 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
       wait_rows(0);
       carry = 0.0;
       if (black_any) b = near(0);
-      if (full) relax<1, true>(p, b, w, inv);
-      else if (black_any) relax<1, false>(p, b, w, inv);
+      if (full) relax<1, true, T>(p, b, w, inv);
+      else if (black_any) relax<1, false, T>(p, b, w, inv);
       if (mine) show(1, true);
       arrive(B_MEET);
-      if (full) carry = squares<1, true>(p, p.e[1], b, dd);
-      else if (black_any) carry = squares<1, false>(p, p.e[1], b, dd);
+      if (full) carry = squares<1, true, T>(p, p.e[1], b, dd);
+      else if (black_any) carry = squares<1, false, T>(p, p.e[1], b, dd);
     }
     arrive(B_SUMS + (int)(t & 1u));
   };
@@ -607,7 +627,7 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
           if (!f) continue;
           const long long o = pool(h, r), oo = pool(1 - h, r);
           const int q = (h + r) & 1;
-          float *g = reinterpret_cast<float *>(&p.g[h][r]);
+          float g[4] = {0.f, 0.f, 0.f, 0.f};  // (a cell that is not interior: not read)
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             if (!(f & (1u << i))) continue;
@@ -617,6 +637,7 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
             g[i] = (float)(-res);
             a = fma(res, res, a);
           }
+          set_rhs(h, r, make_float4(g[0], g[1], g[2], g[3]));
         }
       give(t, 0, a);
       arrive(B_SUMS + (int)(t & 1u));
@@ -632,45 +653,58 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
 
 // A class of systems whose regions may take patches of two rows, or of four;
 // each launch's blocks take theirs.
-template <int R>
-__global__ void __launch_bounds__(kClusterMost + 32, 1) k_cluster_solve(KParams P, const int *__restrict__ list, int TW,
-                                                                        int TH) {
+template <int R, int T>
+__global__ void __launch_bounds__(T + 32, T == kClusterLeast ? 2 : 1) k_cluster_solve(KParams P,
+                                                                                     const int *__restrict__ list,
+                                                                                     int TW, int TH) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ Shared sh;
   const unsigned rank = cluster_rank();
   const int sys = list[blockIdx.x / cluster_size()];
   const Route rt = P.route[sys];
   if ((int)rank >= rt.n || rt.rows != R) return;  // (the cluster's barriers count the threads that stay)
-  solve_region<R>(P, rt, sh, sys, rank, TW, TH, smem);
+  solve_region<R, T>(P, rt, sh, sys, rank, TW, TH, smem);
 }
 
+namespace {
+// f(kernel, rows, limit) for each instance, until one fails
+template <class F>
+cudaError_t each_instance(F f) {
+  cudaError_t e = f(k_cluster_solve<2, kClusterLeast>, 2, kClusterLeast);
+  if (e == cudaSuccess) e = f(k_cluster_solve<4, kClusterLeast>, 4, kClusterLeast);
+  if (e == cudaSuccess) e = f(k_cluster_solve<2, kClusterMost>, 2, kClusterMost);
+  if (e == cudaSuccess) e = f(k_cluster_solve<4, kClusterMost>, 4, kClusterMost);
+  return e;
+}
+}  // namespace
+
 cudaError_t prepare_cluster() {
-  static_assert(kClusterAlone >= kClusterSmem, "the most any class asks for");
-  for (auto k : {k_cluster_solve<2>, k_cluster_solve<4>}) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterAlone);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  static_assert(kClusterAlone >= cluster_smem(4, kClusterMost) && cluster_smem(4, kClusterLeast) <= 110 * 1024,
+                "shared memory of the blocks");
+  return each_instance([](auto k, int, int) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterAlone);
+  });
 }
 
 cudaError_t launch_cluster(const KParams &P, const TileConfig &tc, const ClusterClass &k, const int *list,
                            cudaStream_t stream) {
   if (k.count == 0) return cudaSuccess;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)k.count * (unsigned)k.blocks);
-  cfg.blockDim = dim3((unsigned)k.limit + 32u);
-  cfg.dynamicSmemBytes = (size_t)k.smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = (unsigned)k.blocks;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, k_cluster_solve<2>, P, list + k.first, tc.tw, tc.th);
-  if (e == cudaSuccess && k.rows4) e = cudaLaunchKernelEx(&cfg, k_cluster_solve<4>, P, list + k.first, tc.tw, tc.th);
-  return e;
+  return each_instance([&](auto kernel, int rows, int limit) {
+    if (limit != k.limit || !(rows == 2 ? k.rows2 : k.rows4)) return cudaSuccess;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)k.count * (unsigned)k.blocks);
+    cfg.blockDim = dim3((unsigned)limit + 32u);
+    cfg.dynamicSmemBytes = (size_t)(k.alone ? kClusterAlone : cluster_smem(rows, limit));
+    cfg.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)k.blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P, list + k.first, tc.tw, tc.th);
+  });
 }
 
 }  // namespace ptk

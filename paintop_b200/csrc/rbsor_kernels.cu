@@ -368,7 +368,7 @@ __global__ void k_init(KParams P) {
   // k_solve it counts as done
   Route r{};
   if (P.route) {
-    if (s.mode != M_DONE && cluster_route(bx0, by0, bx1, by1, &r)) atomicAdd(P.bar + 2, 1u);
+    if (s.mode != M_DONE && cluster_route(bx0, by0, bx1, by1, P.many, &r)) atomicAdd(P.bar + 2, 1u);
     P.route[sys] = r;
   }
   P.st[sys] = s;

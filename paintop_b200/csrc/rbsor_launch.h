@@ -28,13 +28,13 @@ cudaError_t prepare_solve(const KParams &P, int cfg, int sms, int *grid);
 cudaError_t launch_prepared(const KParams &P, int cfg, int grid, cudaStream_t stream);
 // The systems whose regions a cluster of thread blocks holds (k_cluster_solve,
 // rbsor_cluster.cu), launched in classes of one cluster and block size each:
-// the systems list[first .. first + count), at most `limit` patches and `smem`
-// bytes a block.
+// the systems list[first .. first + count), at most `limit` patches a block.
 struct ClusterClass {
-  int first, count, blocks, limit, smem;
-  bool rows4;  // a region of the class may take patches of four rows
+  int first, count, blocks, limit;
+  bool rows2, rows4;  // a region of the class may take patches of two, of four rows
+  bool alone;         // no two blocks on an SM
 };
-constexpr int kClusterAlone = 120 * 1024;  // shared memory that keeps a second block off the SM
+constexpr int kClusterAlone = 176 * 1024;  // shared memory that keeps a second block off the SM
 cudaError_t prepare_cluster();  // the kernel's attributes (outside a capture)
 cudaError_t launch_cluster(const KParams &P, const TileConfig &tc, const ClusterClass &k, const int *list,
                            cudaStream_t stream);

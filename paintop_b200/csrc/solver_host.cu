@@ -95,6 +95,7 @@ struct Plan {
   long long largest = 0;            // the largest image's pixels
   std::vector<int> clist;           // the systems by cluster class
   std::vector<ClusterClass> classes;
+  bool many = false;                // the call has kFewValues or more (plan_clusters)
 };
 
 // Arena layout (byte offsets) for one call.
@@ -167,39 +168,38 @@ Layout layout(const Plan &pl, bool stage) {
 // than it has places for, each step of it a chain of latencies: 5.9 us a sweep
 // on 512 x 512 RGB against 2.4 here, 5.2 against 1.7 on 97 x 71. A larger call
 // fills k_solve's places, and clusters pay only if all its images fit the least
-// blocks, two to an SM (128 images of 256 x 256: 10.9 against 9.4 ms); with
+// blocks, two to an SM (128 images of 256 x 256: 10.9 against 7.3 ms); with
 // larger ones among them (48 images of side 64 to 1024: 57 against 68 ms) they
 // hold SMs in gangs that the rest could use.
 constexpr double kFewValues = 4.0e6;
 void plan_clusters(Plan &pl, int sms) {
-  struct Want { int blocks, limit; bool rows4; };
-  std::vector<Want> want(pl.sys.size(), Want{0, 0, false});
+  struct Want { int blocks, limit; bool rows2, rows4; };
+  std::vector<Want> want(pl.sys.size(), Want{0, 0, false, false});
   bool least = true;
   double values = 0.0;
+  for (const SysDesc &d : pl.sys) values += (double)d.W * d.H;
+  pl.many = values >= kFewValues;
   for (size_t i = 0; i < pl.sys.size(); ++i) {
     const SysDesc &d = pl.sys[i];
-    values += (double)d.W * d.H;
     if (d.W < 3 || d.H < 3) continue;  // no interior (k_init)
     Route r{};
-    if (!cluster_route(1, 1, d.W - 2, d.H - 2, &r) || r.limit > kClusterLeast) least = false;
+    if (!cluster_route(1, 1, d.W - 2, d.H - 2, pl.many, &r) || r.limit > kClusterLeast) least = false;
     if (r.limit == 0) {
-      want[i] = Want{kClusterMax, kClusterMost, true};
+      want[i] = Want{kClusterMax, kClusterMost, true, true};
       continue;
     }
     // a smaller region takes no larger blocks, and more of them only where
     // this image takes larger ones or four-row patches
-    int blocks = 1;
-    while (blocks < r.n) blocks *= 2;
-    const bool more = r.limit > kClusterLeast || r.rows > 2;
-    want[i] = Want{more ? kClusterMax : blocks, r.limit, more};
+    want[i] = Want{r.option > 0 ? kClusterMax : r.n, r.limit, pl.many ? r.option > 0 : true,
+                   pl.many ? true : r.option > 0};
   }
-  if (values >= kFewValues && !least) return;
+  if (pl.many && !least) return;
   for (size_t i = 0; i < want.size(); ++i) {
     if (!want[i].blocks) continue;
-    ClusterClass k{(int)pl.clist.size(), 0, want[i].blocks, want[i].limit, kClusterSmem,
-                   want[i].rows4};
+    ClusterClass k{(int)pl.clist.size(), 0, want[i].blocks, want[i].limit, want[i].rows2, want[i].rows4, false};
     for (size_t q = i; q < want.size(); ++q) {
-      if (want[q].blocks != k.blocks || want[q].limit != k.limit || want[q].rows4 != k.rows4) continue;
+      if (want[q].blocks != k.blocks || want[q].limit != k.limit || want[q].rows2 != k.rows2 ||
+          want[q].rows4 != k.rows4) continue;
       pl.clist.push_back((int)q);
       k.count += 1;
       want[q].blocks = 0;
@@ -212,7 +212,7 @@ void plan_clusters(Plan &pl, int sms) {
   long long total = 0;
   for (const ClusterClass &k : pl.classes) total += (long long)k.count * k.blocks;
   if (total <= sms * 3 / 4 + 1)
-    for (ClusterClass &k : pl.classes) k.smem = kClusterAlone;
+    for (ClusterClass &k : pl.classes) k.alone = true;
 }
 
 }  // namespace
@@ -409,6 +409,7 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
   P.label = reinterpret_cast<int *>(base + L.label);
   P.rsize = reinterpret_cast<int *>(base + L.rsize);
   P.rmax = reinterpret_cast<int *>(base + L.rmax);
+  P.many = pl.many;
   P.route = pl.classes.empty() ? nullptr : reinterpret_cast<Route *>(base + L.route);
 
   // ---- host buffers: upload only the part of the images the solve reads.
@@ -549,7 +550,7 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
   ctx->last_grid = grid;
   ctx->last_cfg = pl.cfg;
   long long cluster_launches = 0;
-  for (const ClusterClass &k : pl.classes) cluster_launches += k.rows4 ? 2 : 1;
+  for (const ClusterClass &k : pl.classes) cluster_launches += (int)k.rows2 + (int)k.rows4;
   long long launches = 5 + cluster_launches;  // tile count, compaction, assembly, init, solves
   launches += 1;                                                 // emit
   if (!devptr) launches += 1 + (long long)pl.imgs.size();        // the first tile count, band flags

@@ -69,3 +69,24 @@ def test_cluster_batch_and_reruns(ctx):
         for x in (b, alone):
             assert np.array_equal(a[0].view(np.uint32), x[0].view(np.uint32))
             assert [r["residual_history"] for r in a[1]] == [r["residual_history"] for r in x[1]]
+
+
+def test_cluster_of_many_values(ctx):
+    """4e6 values and more in images that the least blocks hold: patches of four rows
+    first. Each region as if solved alone, where patches of two rows come first."""
+    shapes = [(250, 382, (1, 1, 248, 380)), (257, 300, (3, 2, 255, 297)), (64, 700, (1, 1, 62, 698)), (3, 3, (1, 1, 1, 1)),
+              (256, 256, (5, 7, 250, 248)), (9, 200, (7, 1, 7, 198)), (300, 8, (1, 6, 298, 6))]
+    probs = []
+    for k in range(105):
+        w, h, box = shapes[k % 7]
+        src, tgt, mask = _problem(k, w, h, 1, box)
+        probs.append(dict(source=src, target=tgt, mask=mask, width=w, height=h, channels=1, lam=0.01 * (k % 2),
+                          tolerance=1e-6, omega=1.8, max_iterations=120))
+    assert sum(p["width"] * p["height"] for p in probs) >= 4e6
+    many = ctx.solve_batch(probs, want_history=True)
+    for p, a in list(zip(probs, many))[:14] + list(zip(probs, many))[-7:]:
+        alone = ctx.solve_batch([p], want_history=True)[0]
+        assert np.array_equal(a[0].view(np.uint32), alone[0].view(np.uint32))
+        for x, y in zip(a[1], alone[1]):
+            assert (x["iterations"], x["stop_reason"], x["refinements"]) == (y["iterations"], y["stop_reason"], y["refinements"])
+            np.testing.assert_allclose(x["residual_history"], y["residual_history"], rtol=1e-10)
