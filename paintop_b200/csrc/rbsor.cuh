@@ -51,7 +51,7 @@ namespace ptk {
 
 constexpr int kLW = 128;          // loaded tile width in cells
 constexpr int kPWL = kLW / 2;     // plane row width in shared memory (floats)
-constexpr int kThreads = 512;     // threads per block of the tile kernels
+constexpr int kThreads = 512;     // threads per block of the assembly (k_solve: Geo::NT)
 constexpr int kWarps = kThreads / 32;
 
 __host__ __device__ constexpr int halo_y(int S) { return 2 * S + 1; }

@@ -38,12 +38,16 @@ struct Geo {
   static constexpr int LH = TH + 2 * H;
   static constexpr int PLANE = LH * kPWL;  // elements per shared plane
   static constexpr int XOFF = HX - H;      // unused loaded columns on each side
+  // Rows 1..LH-2 in quads, two rows a half-warp, three (or two) quads a warp.
+  static constexpr int QUADS = (LH - 2) / 4, NW = 8, NT = 32 * NW;
+  static_assert((LH - 2) % 4 == 0 && QUADS % NW == 0, "rows 1..LH-2 must split evenly over the warps");
+  static_assert(H % 2 == 1 && TH % 2 == 0, "loaded row 0 is odd, and a half-warp's two rows are owned alike");
   static_assert(HX >= H, "x halo must cover the sweep halo");
   static_assert(TW > 0 && TW % 8 == 0, "tile width must keep plane loads 16-byte aligned");
   static constexpr size_t kSmem = (size_t)2 * PLANE * sizeof(float)   // e
                                   + (size_t)2 * PLANE * sizeof(float) // g
                                   + (size_t)2 * PLANE                 // cell
-                                  + kWarps * sizeof(double);          // reduction scratch
+                                  + NW * sizeof(double);              // reduction scratch
 };
 
 // ----------------------------------------------------------------------------
@@ -501,6 +505,18 @@ __global__ void k_band_flags(KParams P, int sys0, int *spans) {
 // apart, in different shared-memory banks (rows two apart would share all 16).
 __host__ __device__ constexpr int cell_slot(int ly) { return ly ^ ((ly >> 1) & 1); }
 
+// A step of a tile: load it with its halo, s sweeps, store the owned cells.
+//
+// Bound by instructions and their latency (23 a cell and sweep with one row a
+// lane, 54 % of the issue slots), first among them the FP32 -> FP64 conversions
+// of the residual. So a lane takes two rows, which share the values between
+// them: 34 conversions and 10 loads for eight cells, where single rows need 42
+// and 12, and the rows' parity is static. Four warps a scheduler do
+// then (8 warps a block, 128 registers): on 2048 x 2048 RGBA 3.55 ms with 16
+// warps of single rows, 3.24 with 12 warps of two, 3.19 with 8, 3.40 with 6;
+// 48 uneven images 57, 53, 50.5 and 52 ms. Four rows a lane convert less and
+// have too few warps (3.38 to 3.75 ms), and a path without the tests of the
+// cell flags costs more in code than it saves (3.35).
 template <int S, int TH>
 __device__ void sweep_tile(const KParams &P, const SysDesc &d, int t, const Tile &tl, int s,
                            int cur, float *sE, float *sG, uint8_t *sC, double *sred) {
@@ -516,7 +532,7 @@ __device__ void sweep_tile(const KParams &P, const SysDesc &d, int t, const Tile
   // other blocks wrote these planes). Outside the image the copy reads nothing
   // and zero-fills, which is exactly a boundary cell (e = 0, g = 0, cell = 0).
   constexpr int V = kPWL / 4;
-  for (int k = tid; k < 2 * G::LH * V; k += kThreads) {
+  for (int k = tid; k < 2 * G::LH * V; k += G::NT) {
     const int c = k / (G::LH * V);
     const int r = k - c * (G::LH * V);
     const int ly = r / V, v = r - ly * V;
@@ -531,120 +547,102 @@ __device__ void sweep_tile(const KParams &P, const SysDesc &d, int t, const Tile
   cp_async_wait_all();
   __syncthreads();
 
-  const int pl = Y0 & 1;  // colour parity of loaded row 0 (column 0 is even)
   const float w = d.omega, inv = d.inv_denom;
   const double dd = 4.0 + d.lambda;
   constexpr int OX0 = G::HX, OX1 = G::HX + G::TW;  // owned loaded columns
   constexpr int OY0 = G::H, OY1 = G::H + TH;       // owned loaded rows
   constexpr int RQ = kPWL / 4;                      // float4 per plane row (16 lanes)
-  static_assert((G::LH - 2) % 32 == 0, "rows 1..LH-2 must split evenly over the warps");
-  static_assert(TH % 4 == 0, "owned rows come in groups of four");
   static_assert(OX0 % 8 == 0 && OX1 % 8 == 0, "owned columns come in whole lanes");
   static_assert(G::LH % 4 == 0 || G::LH % 4 == 2, "cell slots stay inside the plane");
   constexpr int LO = OX0 / 8, LE = OX1 / 8;         // lanes (l16) whose cells are owned
-  constexpr int kRowPairs = (G::LH - 2) / 2;
-  // Each lane owns four consecutive plane entries (four cells of one colour) of
-  // a row; the two half-warps take rows two apart, so both rows of a warp have
-  // the same colour parity. Every half-sweep relaxes all rows 1..LH-2 and all
-  // columns: cells outside the window that a whole-grid sweep would reproduce
-  // get values nobody reads (they never reach the owned region before the tile
-  // is written back), which keeps the work of every warp identical.
+  // A lane takes four consecutive plane entries (four cells of one colour) of
+  // two rows, a half-warp the rows' whole width. A row's parity is static: loaded
+  // row 0 is odd in every tile and a quad begins at row 1 + 4 k. Every half-sweep
+  // relaxes all rows 1..LH-2 and all columns: cells outside the window that a
+  // whole-grid sweep would reproduce get values nobody reads (they never reach
+  // the owned region before the tile is written back), which keeps the work of
+  // every warp identical.
   const int hw = lane >> 4, l16 = lane & 15;
+  const bool own_x = l16 >= LO && l16 < LE;
   double acc[S];
 #pragma unroll
   for (int j = 0; j < S; ++j) acc[j] = 0.0;
 
-  // the four cells of a lane together: each square added in cell order as
-  // fma(r, r, part); a cell that is not interior adds fma(0, 0, part) = part,
-  // bit for bit what skipping it gives
   auto rval = [&](float l, float r, float u, float dn, float e, float g) -> double {
     const double ns = (((double)l + (double)r) + (double)u) + (double)dn;
     return fma(-dd, (double)e, ns) - (double)g;
   };
-  auto resid4 = [&](double &part, uint32_t cc, float L0, float R0, float L1, float R1, float L2, float R2,
-                    float L3, float R3, const float4 &up, const float4 &dn, const float4 &e, const float4 &g) {
-    double r0 = rval(L0, R0, up.x, dn.x, e.x, g.x), r1 = rval(L1, R1, up.y, dn.y, e.y, g.y),
-           r2 = rval(L2, R2, up.z, dn.z, e.z, g.z), r3 = rval(L3, R3, up.w, dn.w, e.w, g.w);
-    r0 = (cc & 0xffu) ? r0 : 0.0;
-    r1 = (cc & 0xff00u) ? r1 : 0.0;
-    r2 = (cc & 0xff0000u) ? r2 : 0.0;
-    r3 = (cc & 0xff000000u) ? r3 : 0.0;
-    part = fma(r0, r0, part);
-    part = fma(r1, r1, part);
-    part = fma(r2, r2, part);
-    part = fma(r3, r3, part);
+  // One half-sweep of colour h (constants after inlining): relax the cells, if
+  // so asked, and return the sum of squares of the residual at the owned ones,
+  // if so asked: of black's new values, of red's before.
+  auto half_sweep = [&](const int h, const bool relax, const bool duty) -> double {
+    float4 *Ec = reinterpret_cast<float4 *>(sE + h * G::PLANE);
+    const float4 *Eo = reinterpret_cast<const float4 *>(sE + (1 - h) * G::PLANE);
+    const float4 *Gc = reinterpret_cast<const float4 *>(sG + h * G::PLANE);
+    const uint32_t *Cc = reinterpret_cast<const uint32_t *>(sC + h * G::PLANE);
+    double part = 0.0;
+#pragma unroll 1
+    for (int k = warp; k < G::QUADS; k += G::NW) {
+      const int ly = 1 + 4 * k + 2 * hw, r4 = ly * RQ + l16;
+      const float4 o[4] = {Eo[r4 - RQ], Eo[r4], Eo[r4 + RQ], Eo[r4 + 2 * RQ]};
+      float n[2][5];  // left and right neighbours: l = n[.][0..3], r = n[.][1..4]
+      float4 e[2], g[2];
+      uint32_t c[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float4 ct = o[1 + r];
+        if (((h + r) & 1) == 0) {
+          n[r][0] = __shfl_up_sync(0xffffffffu, ct.w, 1, 16);
+          n[r][1] = ct.x; n[r][2] = ct.y; n[r][3] = ct.z; n[r][4] = ct.w;
+        } else {
+          n[r][0] = ct.x; n[r][1] = ct.y; n[r][2] = ct.z; n[r][3] = ct.w;
+          n[r][4] = __shfl_down_sync(0xffffffffu, ct.x, 1, 16);
+        }
+        g[r] = Gc[r4 + r * RQ];
+        e[r] = Ec[r4 + r * RQ];
+        c[r] = Cc[cell_slot(ly + r) * RQ + l16];
+      }
+      float4 ne[2] = {e[0], e[1]};
+      if (relax) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const float4 up = o[r], dn = o[r + 2];
+          if (c[r] & 0xffu) ne[r].x = fmaf(w, ((((n[r][0] + n[r][1]) + up.x) + dn.x) - g[r].x) * inv - e[r].x, e[r].x);
+          if (c[r] & 0xff00u) ne[r].y = fmaf(w, ((((n[r][1] + n[r][2]) + up.y) + dn.y) - g[r].y) * inv - e[r].y, e[r].y);
+          if (c[r] & 0xff0000u) ne[r].z = fmaf(w, ((((n[r][2] + n[r][3]) + up.z) + dn.z) - g[r].z) * inv - e[r].z, e[r].z);
+          if (c[r] & 0xff000000u) ne[r].w = fmaf(w, ((((n[r][3] + n[r][4]) + up.w) + dn.w) - g[r].w) * inv - e[r].w, e[r].w);
+          Ec[r4 + r * RQ] = ne[r];
+        }
+      }
+      // a lane's eight residuals behind one lane-level test, so that their
+      // conversion and FP64 chains interleave
+      if (duty && own_x && ly >= OY0 && ly < OY1 && (c[0] | c[1]) != 0u) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const float4 up = o[r], dn = o[r + 2], v = h ? ne[r] : e[r];
+          const double x0 = rval(n[r][0], n[r][1], up.x, dn.x, v.x, g[r].x), x1 = rval(n[r][1], n[r][2], up.y, dn.y, v.y, g[r].y),
+                       x2 = rval(n[r][2], n[r][3], up.z, dn.z, v.z, g[r].z), x3 = rval(n[r][3], n[r][4], up.w, dn.w, v.w, g[r].w);
+          if (c[r] & 0xffu) part = fma(x0, x0, part);
+          if (c[r] & 0xff00u) part = fma(x1, x1, part);
+          if (c[r] & 0xff0000u) part = fma(x2, x2, part);
+          if (c[r] & 0xff000000u) part = fma(x3, x3, part);
+        }
+      }
+    }
+    return part;
   };
-
 #pragma unroll
   for (int j = 0; j < S; ++j) {
     if (j >= s) break;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      float4 *Ec = reinterpret_cast<float4 *>(sE + h * G::PLANE);
-      const float4 *Eo = reinterpret_cast<const float4 *>(sE + (1 - h) * G::PLANE);
-      const float4 *Gc = reinterpret_cast<const float4 *>(sG + h * G::PLANE);
-      const uint32_t *Cc = reinterpret_cast<const uint32_t *>(sC + h * G::PLANE);
-      const bool duty = (h == 1) || (j > 0);  // residual of black state j / red state j-1
-      double part = 0.0;
-      for (int rp = warp; rp < kRowPairs; rp += kWarps) {
-        const int base = 1 + 4 * (rp >> 1) + (rp & 1);
-        const int ly = base + 2 * hw;
-        const int q = (h + base + pl) & 1;  // same for both rows of the warp
-        const int r4 = ly * RQ + l16;
-        const float4 up = Eo[r4 - RQ], dn = Eo[r4 + RQ], ct = Eo[r4];
-        const float4 gc = Gc[r4];
-        const float4 ec = Ec[r4];
-        const uint32_t cc = Cc[cell_slot(ly) * RQ + l16];
-        const float prev = __shfl_up_sync(0xffffffffu, ct.w, 1, 16);
-        const float next = __shfl_down_sync(0xffffffffu, ct.x, 1, 16);
-        float L0, R0, L1, R1, L2, R2, L3, R3;
-        if (q == 0) {
-          L0 = prev; R0 = ct.x; L1 = ct.x; R1 = ct.y; L2 = ct.y; R2 = ct.z; L3 = ct.z; R3 = ct.w;
-        } else {
-          L0 = ct.x; R0 = ct.y; L1 = ct.y; R1 = ct.z; L2 = ct.z; R2 = ct.w; L3 = ct.w; R3 = next;
-        }
-        float4 ne = ec;
-        if (cc & 0xffu) ne.x = fmaf(w, ((((L0 + R0) + up.x) + dn.x) - gc.x) * inv - ec.x, ec.x);
-        if (cc & 0xff00u) ne.y = fmaf(w, ((((L1 + R1) + up.y) + dn.y) - gc.y) * inv - ec.y, ec.y);
-        if (cc & 0xff0000u) ne.z = fmaf(w, ((((L2 + R2) + up.z) + dn.z) - gc.z) * inv - ec.z, ec.z);
-        if (cc & 0xff000000u) ne.w = fmaf(w, ((((L3 + R3) + up.w) + dn.w) - gc.w) * inv - ec.w, ec.w);
-        // a lane's four residuals together behind one lane-level test, so their
-        // conversion and FP64 chains interleave (the owned columns come in whole
-        // lanes: HX and TW are multiples of 8)
-        if (duty && ly >= OY0 && ly < OY1 && l16 >= LO && l16 < LE && cc != 0u)
-          resid4(part, cc, L0, R0, L1, R1, L2, R2, L3, R3, up, dn, h ? ne : ec, gc);
-        Ec[r4] = ne;
-      }
-      if (h == 1) acc[j] += part;
-      else if (j > 0) acc[j - 1] += part;
-      __syncthreads();
-    }
+    const double red = half_sweep(0, true, j > 0);  // (the residual of the sweep before)
+    if (j > 0) acc[j > 0 ? j - 1 : 0] += red;
+    __syncthreads();
+    acc[j] += half_sweep(1, true, true);
+    __syncthreads();
   }
   // red cells' residual of the final state
   {
-    const float4 *Er = reinterpret_cast<const float4 *>(sE);
-    const float4 *Eb = reinterpret_cast<const float4 *>(sE + G::PLANE);
-    const float4 *Gr = reinterpret_cast<const float4 *>(sG);
-    const uint32_t *Cr = reinterpret_cast<const uint32_t *>(sC);
-    double part = 0.0;
-    for (int rp = warp; rp < TH / 2; rp += kWarps) {
-      const int base = OY0 + 4 * (rp >> 1) + (rp & 1);
-      const int ly = base + 2 * hw;
-      const int q = (base + pl) & 1;
-      const int r4 = ly * RQ + l16;
-      const float4 up = Eb[r4 - RQ], dn = Eb[r4 + RQ], ct = Eb[r4];
-      const float4 gc = Gr[r4], ec = Er[r4];
-      const uint32_t cc = Cr[cell_slot(ly) * RQ + l16];
-      const float prev = __shfl_up_sync(0xffffffffu, ct.w, 1, 16);
-      const float next = __shfl_down_sync(0xffffffffu, ct.x, 1, 16);
-      float L0, R0, L1, R1, L2, R2, L3, R3;
-      if (q == 0) {
-        L0 = prev; R0 = ct.x; L1 = ct.x; R1 = ct.y; L2 = ct.y; R2 = ct.z; L3 = ct.z; R3 = ct.w;
-      } else {
-        L0 = ct.x; R0 = ct.y; L1 = ct.y; R1 = ct.z; L2 = ct.z; R2 = ct.w; L3 = ct.w; R3 = next;
-      }
-      if (l16 >= LO && l16 < LE && cc != 0u) resid4(part, cc, L0, R0, L1, R1, L2, R2, L3, R3, up, dn, ec, gc);
-    }
+    const double part = half_sweep(0, false, true);
 #pragma unroll
     for (int j = 0; j < S; ++j)
       if (j == s - 1) acc[j] += part;
@@ -661,19 +659,19 @@ __device__ void sweep_tile(const KParams &P, const SysDesc &d, int t, const Tile
       double v = acc[j];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) sr[j * kWarps + warp] = v;
+      if (lane == 0) sr[j * G::NW + warp] = v;
     }
     __syncthreads();
     if (tid < s) {
       double tot = 0.0;
-      for (int w = 0; w < kWarps; ++w) tot += sr[tid * kWarps + w];
+      for (int w = 0; w < G::NW; ++w) tot += sr[tid * G::NW + w];
       P.partial[(long long)tid * P.ntiles + t] = tot;
     }
   }
 
   // ---- write the owned cells
   constexpr int OV = G::TW / 8;  // float4 per owned plane row
-  for (int k = tid; k < 2 * TH * OV; k += kThreads) {
+  for (int k = tid; k < 2 * TH * OV; k += G::NT) {
     const int c = k / (TH * OV);
     const int r = k - c * (TH * OV);
     const int ly = G::H + r / OV, v = G::HX / 8 + r % OV;
@@ -692,7 +690,7 @@ __device__ void fold_tile(const KParams &P, const SysDesc &d, const Tile &tl, in
   using G = Geo<S, TH>;
   float *ec = cur ? P.e1 : P.e0;
   constexpr int OV = G::TW / 8;
-  for (int k = threadIdx.x; k < 2 * TH * OV; k += kThreads) {
+  for (int k = threadIdx.x; k < 2 * TH * OV; k += G::NT) {
     const int c = k / (TH * OV);
     const int r = k - c * (TH * OV);
     const int gy = tl.ty * TH + r / OV;
@@ -720,7 +718,7 @@ __device__ void resid_tile(const KParams &P, const SysDesc &d, int t, const Tile
   constexpr int half = G::TW / 2;
   const double lam4 = d.lambda + 4.0;
   double acc = 0.0;
-  for (int k = threadIdx.x; k < 2 * TH * half; k += kThreads) {
+  for (int k = threadIdx.x; k < 2 * TH * half; k += G::NT) {
     const int c = k / (TH * half);
     const int r = k - c * (TH * half);
     const int gy = tl.ty * TH + r / half;
@@ -805,7 +803,7 @@ __device__ int claim_tile(const KParams &P, int rot, int *idx, unsigned *gen,
 }
 
 template <int S, int TH>
-__global__ void __launch_bounds__(kThreads, 2) k_solve(KParams P) {
+__global__ void __launch_bounds__((Geo<S, TH>::NT), 2) k_solve(KParams P) {
   using G = Geo<S, TH>;
   extern __shared__ __align__(16) unsigned char smem[];
   float *sE = reinterpret_cast<float *>(smem);
@@ -863,7 +861,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_solve(KParams P) {
       const int nsum = (mode == M_SWEEP) ? s : (mode == M_RESID ? 1 : 0);
       const int nact = __ldcg(&stp->nact);
       if (nsum > 0) {
-        for (int k = threadIdx.x; k < nact; k += kThreads) {
+        for (int k = threadIdx.x; k < nact; k += G::NT) {
           const int tk = __ldcg(P.act + d.tile0 + k);
 #pragma unroll
           for (int j = 0; j < S; ++j)
@@ -895,7 +893,7 @@ static cudaError_t prepare_solve_t(const KParams &P, int sms, int *grid_out) {
                                        (int)G::kSmem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve<S, TH>, kThreads, G::kSmem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve<S, TH>, G::NT, G::kSmem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   int grid = per_sm * sms;
@@ -911,7 +909,7 @@ static cudaError_t launch_prepared_t(const KParams &P, int grid, cudaStream_t st
   Pc.S = S;
   // No block waits for a particular other block (work is claimed, never
   // assigned), so an ordinary launch suffices; the grid fills the GPU once.
-  k_solve<S, TH><<<grid, kThreads, G::kSmem, stream>>>(Pc);
+  k_solve<S, TH><<<grid, G::NT, G::kSmem, stream>>>(Pc);
   return cudaGetLastError();
 }
 

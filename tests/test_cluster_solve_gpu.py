@@ -90,3 +90,13 @@ def test_cluster_of_many_values(ctx):
         for x, y in zip(a[1], alone[1]):
             assert (x["iterations"], x["stop_reason"], x["refinements"]) == (y["iterations"], y["stop_reason"], y["refinements"])
             np.testing.assert_allclose(x["residual_history"], y["residual_history"], rtol=1e-10)
+
+
+@pytest.mark.parametrize("config", range(5))
+@pytest.mark.parametrize("w,h,box", [(5, 4, (1, 1, 3, 2)), (114, 86, (1, 1, 112, 84)), (113, 85, (1, 2, 111, 82)), (241, 175, (2, 1, 239, 171))])
+def test_tiles_of_every_config(w, h, box, config):
+    """The tile kernel's row and column remainders in each tile size, against the cluster kernel."""
+    from paintop_b200 import _lib
+    with _lib.Context(0) as c:
+        c.set_config(config)
+        test_cluster_matches_tiles(c, w, h, box)
