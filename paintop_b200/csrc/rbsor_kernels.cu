@@ -763,41 +763,67 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
   return v;
 }
 
-// Thread 0: claim the next open tile of any system, starting at system `rot`.
+// Warp 0: claim the next open tile of any system, starting at system `rot`.
 // Returns the system (or -1 when every system is done, an error was raised or
-// the wait for work exceeded its bound) and sets *idx, *gen.
+// the wait for work exceeded its bound), *idx and *gen in every lane.
+//
+// Bound by the latency of its loads: 32 systems are looked at together, where
+// one thread after the other took a claim word's latency a system, and a call
+// of many systems spends its end with most of them done. 48 uneven RGB images
+// (144 systems): 50.5 ms with one thread, 40.0 with a warp; one
+// of 2048 x 2048 RGBA 3.19 and 3.15.
 __device__ int claim_tile(const KParams &P, int rot, int *idx, unsigned *gen,
                           unsigned long long t_start) {
-  unsigned long long idle_from = 0;
+  const int lane = threadIdx.x & 31;
+  unsigned long long idle_from = 0;  // (lane 0's)
   for (;;) {
     // an error anywhere or the wall budget ends every block at its next claim
-    if (ld_vol(P.err) != 0) return -1;
-    if (gtimer() - t_start > P.budget_ns) {
-      atomicCAS(P.err, 0, KERR_DEADLINE);
-      return -1;
-    }
-    for (int k = 0; k < P.nsys; ++k) {
-      int c = rot + k;
-      if (c >= P.nsys) c -= P.nsys;
-      const unsigned nact = (unsigned)__ldcg(&P.st[c].nact);
-      if ((unsigned)ld_acquire_u64(P.claim + c) >= nact) continue;  // step fully handed out
-      const unsigned long long cw = atomicAdd(P.claim + c, 1ull);
-      if ((unsigned)cw < nact) {
-        *idx = (int)(unsigned)cw;
-        *gen = (unsigned)(cw >> 32);
-        __threadfence();  // the claimed generation's state was published before its claim word
-        return c;
+    int stop = 0;
+    if (lane == 0) {
+      stop = ld_vol(P.err) != 0;
+      if (!stop && gtimer() - t_start > P.budget_ns) {
+        atomicCAS(P.err, 0, KERR_DEADLINE);
+        stop = 1;
       }
     }
-    if (ld_acquire(P.bar + 2) >= (unsigned)P.nsys) return -1;
-    const unsigned long long now = gtimer();
-    // every open step is handed out and being finished by other blocks; a
-    // step takes milliseconds at most, so 20 s without work is a fault
-    if (!idle_from) idle_from = now;
-    else if (now - idle_from > 20ull * 1000000000ull) {
-      atomicCAS(P.err, 0, KERR_STALLED);
-      return -1;
+    if (__shfl_sync(0xffffffffu, stop, 0)) return -1;
+    for (int k = 0; k < P.nsys; k += 32) {
+      int c = rot + k + lane;
+      if (c >= P.nsys) c -= P.nsys;
+      unsigned nact = 0;
+      bool open = k + lane < P.nsys;
+      if (open) {
+        nact = (unsigned)__ldcg(&P.st[c].nact);
+        open = (unsigned)ld_acquire_u64(P.claim + c) < nact;  // else the step is fully handed out
+      }
+      for (unsigned m = __ballot_sync(0xffffffffu, open); m; m &= m - 1) {
+        const int at = __ffs((int)m) - 1;
+        unsigned long long cw = 0;
+        bool got = false;
+        if (lane == at) {
+          cw = atomicAdd(P.claim + c, 1ull);
+          got = (unsigned)cw < nact;
+          if (got) __threadfence();  // the claimed generation's state was published before its claim word
+        }
+        if (!__any_sync(0xffffffffu, got)) continue;
+        cw = __shfl_sync(0xffffffffu, cw, at);
+        *idx = (int)(unsigned)cw;
+        *gen = (unsigned)(cw >> 32);
+        return __shfl_sync(0xffffffffu, c, at);
+      }
     }
+    if (lane == 0) {
+      if (ld_acquire(P.bar + 2) >= (unsigned)P.nsys) stop = 1;
+      const unsigned long long now = gtimer();
+      // every open step is handed out and being finished by other blocks; a
+      // step takes milliseconds at most, so 20 s without work is a fault
+      if (!idle_from) idle_from = now;
+      else if (!stop && now - idle_from > 20ull * 1000000000ull) {
+        atomicCAS(P.err, 0, KERR_STALLED);
+        stop = 1;
+      }
+    }
+    if (__shfl_sync(0xffffffffu, stop, 0)) return -1;
     __nanosleep(64);
   }
 }
@@ -816,13 +842,15 @@ __global__ void __launch_bounds__((Geo<S, TH>::NT), 2) k_solve(KParams P) {
   int rot = P.nsys > 0 ? (int)(blockIdx.x % (unsigned)P.nsys) : 0;
 
   for (;;) {
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
       int idx = 0;
       unsigned gen = 0;
       const int sys = claim_tile(P, rot, &idx, &gen, t_start);
-      s_sys = sys;
-      s_idx = idx;
-      s_gen = gen;
+      if (threadIdx.x == 0) {
+        s_sys = sys;
+        s_idx = idx;
+        s_gen = gen;
+      }
     }
     __syncthreads();
     const int sys = s_sys, idx = s_idx;

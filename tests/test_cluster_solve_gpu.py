@@ -100,3 +100,20 @@ def test_tiles_of_every_config(w, h, box, config):
     with _lib.Context(0) as c:
         c.set_config(config)
         test_cluster_matches_tiles(c, w, h, box)
+
+
+@pytest.mark.parametrize("count", [1, 30, 31, 32, 63, 100])
+def test_tiles_of_many_systems(ctx, count):
+    """Systems beside a large image take the tile kernel, whose blocks look for work
+    32 systems at a time; each ends as if solved alone."""
+    big = np.zeros(2048 * 2048, np.float32)
+    probs = [dict(source=big, target=big, mask=big, width=2048, height=2048, channels=1)]
+    for k in range(count):
+        w, h = 20 + 7 * (k % 9), 12 + 5 * (k % 11)
+        src, tgt, mask = _problem(k, w, h, 1, (1, 1, w - 2, h - 2))
+        probs.append(dict(source=src, target=tgt, mask=mask, width=w, height=h, channels=1, lam=0.0, tolerance=1e-6,
+                          omega=1.7, max_iterations=20 + 13 * (k % 7)))
+    for p, a in list(zip(probs, ctx.solve_batch(probs)))[1::7]:
+        alone = ctx.solve_batch([p])[0]
+        assert np.array_equal(a[0].view(np.uint32), alone[0].view(np.uint32))
+        assert [r["iterations"] for r in a[1]] == [r["iterations"] for r in alone[1]]
