@@ -46,3 +46,10 @@ def test_first_iteration_matches_the_model(ctx, w, h, lam):
     _, per, _ = ctx.solve(src, tgt, mask, w, h, 1, lam=lam, tolerance=1e-12, max_iterations=1, flags=_lib.PT_FLAG_MULTIGRID)
     assert per[0]["iterations"] == 1
     assert abs(per[0]["final_residual"] - want) <= 1e-5, (per[0]["final_residual"], want)
+
+
+@pytest.mark.parametrize("w,h", [(241, 64), (20, 8)])
+@pytest.mark.parametrize("lam", [1e-7, 0.3, 7.0, 1e4])
+def test_first_iteration_of_screened_systems(ctx, w, h, lam):
+    """Divisions by a diagonal that is no power of two, far and near 4."""
+    test_first_iteration_matches_the_model(ctx, w, h, lam)
