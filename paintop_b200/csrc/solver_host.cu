@@ -165,11 +165,11 @@ Layout layout(const Plan &pl, bool stage) {
 //
 // Like the tile configuration, the choice of kernel depends on the call's
 // shapes alone. A call of fewer than 4e6 values leaves k_solve with fewer tiles
-// than it has places for, each step of it a chain of latencies: 5.9 us a sweep
-// on 512 x 512 RGB against 2.4 here, 5.2 against 1.7 on 97 x 71. A larger call
+// than it has places for, each step of it a chain of latencies: 5.6 us a sweep
+// on 512 x 512 RGB against 2.4 here, 5.3 against 1.9 on 97 x 71. A larger call
 // fills k_solve's places, and clusters pay only if all its images fit the least
-// blocks, two to an SM (128 images of 256 x 256: 10.9 against 7.3 ms); with
-// larger ones among them (48 images of side 64 to 1024: 57 against 68 ms) they
+// blocks, two to an SM (128 images of 256 x 256: 9.3 against 7.3 ms); with
+// larger ones among them (48 images of side 64 to 1024: 40 against 51 ms) they
 // hold SMs in gangs that the rest could use.
 constexpr double kFewValues = 4.0e6;
 void plan_clusters(Plan &pl, int sms) {
@@ -557,7 +557,8 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
 
   // Everything from here to the results is stream work on the device: with
   // device pointers it is captured once into a CUDA graph and replayed while
-  // the plan (descriptors, pointers, arena, configuration) stays the same.
+  // the plan (descriptors but for the images' addresses, arena, configuration)
+  // stays the same.
   auto record = [&](cudaEvent_t ev, bool capturing) {
     // inside a capture an external record node still times the launch; the
     // flag is only valid while capturing
