@@ -156,21 +156,24 @@ Layout layout(const Plan &pl, bool stage) {
   return L;
 }
 
-// The launches of k_cluster_solve: the systems by the cluster and block size
-// their images can need at most (the masks are on the device, so the regions
-// are not known here; k_init splits each by its bounding box, and a block that
-// a split does not use returns at once). An image that no cluster holds whole
-// may still have a region that one does, so it goes with the largest. Classes
-// keep small regions from being scheduled in gangs of 16 blocks.
+// The launch of k_cluster_solve: the cluster and block size that the systems'
+// images can need at most (the masks are on the device, so the regions are not
+// known here; k_init splits each by its bounding box, and a block that a split
+// does not use returns at once). An image that no cluster holds whole may still
+// have a region that one does, so it takes the largest.
 //
 // Like the tile configuration, the choice of kernel depends on the call's
 // shapes alone. A call of fewer than 4e6 values leaves k_solve with fewer tiles
 // than it has places for, each step of it a chain of latencies: 5.6 us a sweep
 // on 512 x 512 RGB against 2.4 here, 5.3 against 1.9 on 97 x 71. A larger call
 // fills k_solve's places, and clusters pay only if all its images fit the least
-// blocks, two to an SM (128 images of 256 x 256: 9.3 against 7.3 ms); with
-// larger ones among them (48 images of side 64 to 1024: 40 against 51 ms) they
-// hold SMs in gangs that the rest could use.
+// blocks, two to an SM (128 images of 256 x 256: 9.3 against 7.3 ms; 24 of them
+// 3.7 against 2.2, 128 of 96 x 96 1.3 against 0.5). Images that ask for different
+// sizes would be launched one size after the other while k_solve takes all at
+// once, so their call is k_solve's (22 images of side 64 to 256: 2.4 against 4.9
+// ms; 12 to side 800: 7.0 against 12.1), and so is one of more of the largest
+// clusters than run at a time (kLargeClusters: 16 SMs each).
+constexpr int kLargeClusters = 7;
 constexpr double kFewValues = 4.0e6;
 void plan_clusters(Plan &pl, int sms) {
   struct Want { int blocks, limit; bool rows2, rows4; };
@@ -194,18 +197,20 @@ void plan_clusters(Plan &pl, int sms) {
                    pl.many ? true : r.option > 0};
   }
   if (pl.many && !least) return;
+  ClusterClass k{0, 0, 0, 0, false, false, false};
   for (size_t i = 0; i < want.size(); ++i) {
-    if (!want[i].blocks) continue;
-    ClusterClass k{(int)pl.clist.size(), 0, want[i].blocks, want[i].limit, want[i].rows2, want[i].rows4, false};
-    for (size_t q = i; q < want.size(); ++q) {
-      if (want[q].blocks != k.blocks || want[q].limit != k.limit || want[q].rows2 != k.rows2 ||
-          want[q].rows4 != k.rows4) continue;
-      pl.clist.push_back((int)q);
-      k.count += 1;
-      want[q].blocks = 0;
+    const Want &v = want[i];
+    if (!v.blocks) continue;
+    if (k.count == 0) k = ClusterClass{0, 0, v.blocks, v.limit, v.rows2, v.rows4, false};
+    if (v.blocks != k.blocks || v.limit != k.limit || v.rows2 != k.rows2 || v.rows4 != k.rows4) {
+      pl.clist.clear();
+      return;
     }
-    pl.classes.push_back(k);
+    pl.clist.push_back((int)i);
+    k.count += 1;
   }
+  if (k.count > 0 && (k.limit <= kClusterLeast || k.count <= kLargeClusters)) pl.classes.push_back(k);
+  else pl.clist.clear();
   // Blocks whose results are waited for one half-sweep at a time are better
   // off alone on an SM while there are SMs to spare: shared memory asked for
   // beyond their own keeps others away.

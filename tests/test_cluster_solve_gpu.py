@@ -56,13 +56,32 @@ def test_cluster_matches_tiles(ctx, w, h, box):
         np.testing.assert_allclose(a["residual_history"], b["residual_history"], rtol=1e-10)
 
 
-def test_cluster_batch_and_reruns(ctx):
-    """Regions of every class in one call, each as if solved alone, twice the same."""
+def _alike(a, b):
+    """Images and counts bit for bit, histories to the order of their sums."""
+    assert np.array_equal(a[0].view(np.uint32), b[0].view(np.uint32))
+    for x, y in zip(a[1], b[1]):
+        assert (x["iterations"], x["stop_reason"], x["refinements"]) == (y["iterations"], y["stop_reason"], y["refinements"])
+        np.testing.assert_allclose(x["residual_history"], y["residual_history"], rtol=1e-10)
+
+
+def _batch(shapes, cap):
     probs = []
-    for k, (w, h, box) in enumerate(CASES[:11]):
+    for k, (w, h, box) in enumerate(shapes):
         src, tgt, mask = _problem(k, w, h, 1, box)
         probs.append(dict(source=src, target=tgt, mask=mask, width=w, height=h, channels=1, lam=0.01 * (k % 2),
-                          tolerance=1e-6, omega=1.8, max_iterations=300))
+                          tolerance=1e-6, omega=1.8, max_iterations=cap))
+    return probs
+
+
+# images that ask for one cluster size, their regions of many: every split of it
+SAME = [[(250, 250, (1 + k, 2 * k, 248 - 20 * k, 240 - 9 * k)) for k in range(1, 10)],
+        [(64, 64, (1 + k, 1 + k % 3, 62 - 3 * k, 62 - k)) for k in range(12)]]
+
+
+@pytest.mark.parametrize("shapes", SAME)
+def test_cluster_batch_and_reruns(ctx, shapes):
+    """Regions of one call, each as if solved alone, twice the same."""
+    probs = _batch(shapes, 300)
     first, again = (ctx.solve_batch(probs, want_history=True) for _ in range(2))
     for p, a, b in zip(probs, first, again):
         alone = ctx.solve_batch([p], want_history=True)[0]
@@ -71,25 +90,25 @@ def test_cluster_batch_and_reruns(ctx):
             assert [r["residual_history"] for r in a[1]] == [r["residual_history"] for r in x[1]]
 
 
-def test_cluster_of_many_values(ctx):
+def test_batch_of_every_class(ctx):
+    """Images that ask for different clusters, or for too many large ones, are the
+    tile kernel's; each ends as if solved alone."""
+    for probs in (_batch(CASES[:11], 300), _batch([(512, 300, (20, 11, 490, 285))] * 8, 60)):
+        for p, a in zip(probs, ctx.solve_batch(probs, want_history=True)):
+            _alike(a, ctx.solve_batch([p], want_history=True)[0])
+
+
+# (count x width x height is 4e6 and more)
+@pytest.mark.parametrize("count,w,h,box", [(44, 250, 382, (1, 1, 248, 380)), (53, 257, 300, (3, 2, 255, 297)),
+                                           (90, 64, 700, (1, 1, 62, 698)), (62, 256, 256, (5, 7, 250, 248))])
+def test_cluster_of_many_values(ctx, count, w, h, box):
     """4e6 values and more in images that the least blocks hold: patches of four rows
     first. Each region as if solved alone, where patches of two rows come first."""
-    shapes = [(250, 382, (1, 1, 248, 380)), (257, 300, (3, 2, 255, 297)), (64, 700, (1, 1, 62, 698)), (3, 3, (1, 1, 1, 1)),
-              (256, 256, (5, 7, 250, 248)), (9, 200, (7, 1, 7, 198)), (300, 8, (1, 6, 298, 6))]
-    probs = []
-    for k in range(105):
-        w, h, box = shapes[k % 7]
-        src, tgt, mask = _problem(k, w, h, 1, box)
-        probs.append(dict(source=src, target=tgt, mask=mask, width=w, height=h, channels=1, lam=0.01 * (k % 2),
-                          tolerance=1e-6, omega=1.8, max_iterations=120))
-    assert sum(p["width"] * p["height"] for p in probs) >= 4e6
+    x0, y0, x1, y1 = box
+    probs = _batch([(w, h, (x0 + k % 3, y0 + k % 5, x1 - k % 4, y1 - k % 7)) for k in range(count)], 120)
     many = ctx.solve_batch(probs, want_history=True)
-    for p, a in list(zip(probs, many))[:14] + list(zip(probs, many))[-7:]:
-        alone = ctx.solve_batch([p], want_history=True)[0]
-        assert np.array_equal(a[0].view(np.uint32), alone[0].view(np.uint32))
-        for x, y in zip(a[1], alone[1]):
-            assert (x["iterations"], x["stop_reason"], x["refinements"]) == (y["iterations"], y["stop_reason"], y["refinements"])
-            np.testing.assert_allclose(x["residual_history"], y["residual_history"], rtol=1e-10)
+    for p, a in list(zip(probs, many))[::9]:
+        _alike(a, ctx.solve_batch([p], want_history=True)[0])
 
 
 @pytest.mark.parametrize("config", range(5))
