@@ -27,6 +27,9 @@ struct pt_ctx {
   void *pin = nullptr;         // page-locked staging of plans and results, grown to a high-water mark
   size_t pin_cap = 0;
   int solve_grid[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // blocks of k_solve that fit the device, by tile configuration
+  static constexpr int kSides = 7;
+  cudaStream_t side[kSides] = {};       // for launches beside one another (made when first needed)
+  cudaEvent_t forked = nullptr, joined[kSides] = {};
   bool graphs = true;          // capture device-pointer solves into a CUDA graph
   cudaGraphExec_t gexec = nullptr;
   std::string gkey;            // the plan the cached graph was captured for
@@ -64,6 +67,25 @@ struct pt_ctx {
     }
     arena_cap = want;
     return true;
+  }
+
+  // The first n side streams and their events.
+  cudaError_t make_sides(int n) {
+    cudaError_t e = cudaSuccess;
+    if (!forked) e = cudaEventCreateWithFlags(&forked, cudaEventDisableTiming);
+    for (int k = 0; k < n && e == cudaSuccess; ++k) {
+      if (!side[k]) e = cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking);
+      if (e == cudaSuccess && !joined[k]) e = cudaEventCreateWithFlags(&joined[k], cudaEventDisableTiming);
+    }
+    return e;
+  }
+
+  void drop_sides() {
+    for (auto &s : side)
+      if (s) { cudaStreamDestroy(s); s = nullptr; }
+    for (auto &e : joined)
+      if (e) { cudaEventDestroy(e); e = nullptr; }
+    if (forked) { cudaEventDestroy(forked); forked = nullptr; }
   }
 
   // Staging for at least `bytes`; the calls wait for their copies before they

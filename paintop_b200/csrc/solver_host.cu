@@ -169,16 +169,19 @@ Layout layout(const Plan &pl, bool stage) {
 // fills k_solve's places, and clusters pay only if all its images fit the least
 // blocks, two to an SM (128 images of 256 x 256: 9.3 against 7.3 ms; 24 of them
 // 3.7 against 2.2, 128 of 96 x 96 1.3 against 0.5). Images that ask for different
-// sizes would be launched one size after the other while k_solve takes all at
-// once, so their call is k_solve's (22 images of side 64 to 256: 2.4 against 4.9
-// ms; 12 to side 800: 7.0 against 12.1), and so is one of more of the largest
-// clusters than run at a time (kLargeClusters: 16 SMs each).
+// sizes are launched side by side, a stream each size (2, 4 and 7 images of side
+// 64 to 256: 0.68, 0.53 and 0.71 ms against 1.9, 1.5 and 2.0), and only as many
+// as run at a time (their blocks fit the SMs): more of them, or larger images among them,
+// would wait for one another where k_solve takes all at once (22 images of side
+// 64 to 256: 2.4 ms against 4.9 one size after the other; 12 to side 800: 7.0
+// against 12.1). The largest clusters take 16 SMs each, and a call of more than
+// kLargeClusters of them is k_solve's.
 constexpr int kLargeClusters = 7;
 constexpr double kFewValues = 4.0e6;
 void plan_clusters(Plan &pl, int sms) {
   struct Want { int blocks, limit; bool rows2, rows4; };
   std::vector<Want> want(pl.sys.size(), Want{0, 0, false, false});
-  bool least = true;
+  bool least = true, fit = true;
   double values = 0.0;
   for (const SysDesc &d : pl.sys) values += (double)d.W * d.H;
   pl.many = values >= kFewValues;
@@ -188,6 +191,7 @@ void plan_clusters(Plan &pl, int sms) {
     Route r{};
     if (!cluster_route(1, 1, d.W - 2, d.H - 2, pl.many, &r) || r.limit > kClusterLeast) least = false;
     if (r.limit == 0) {
+      fit = false;
       want[i] = Want{kClusterMax, kClusterMost, true, true};
       continue;
     }
@@ -197,20 +201,26 @@ void plan_clusters(Plan &pl, int sms) {
                    pl.many ? true : r.option > 0};
   }
   if (pl.many && !least) return;
-  ClusterClass k{0, 0, 0, 0, false, false, false};
+  int units = 0;  // half SMs
+  for (const Want &v : want) units += v.blocks * (v.limit > kClusterLeast ? 2 : 1);
   for (size_t i = 0; i < want.size(); ++i) {
-    const Want &v = want[i];
-    if (!v.blocks) continue;
-    if (k.count == 0) k = ClusterClass{0, 0, v.blocks, v.limit, v.rows2, v.rows4, false};
-    if (v.blocks != k.blocks || v.limit != k.limit || v.rows2 != k.rows2 || v.rows4 != k.rows4) {
-      pl.clist.clear();
-      return;
+    if (!want[i].blocks) continue;
+    ClusterClass k{(int)pl.clist.size(), 0, want[i].blocks, want[i].limit, want[i].rows2, want[i].rows4, false};
+    for (size_t q = i; q < want.size(); ++q) {
+      if (want[q].blocks != k.blocks || want[q].limit != k.limit || want[q].rows2 != k.rows2 ||
+          want[q].rows4 != k.rows4) continue;
+      pl.clist.push_back((int)q);
+      k.count += 1;
+      want[q].blocks = 0;
     }
-    pl.clist.push_back((int)i);
-    k.count += 1;
+    pl.classes.push_back(k);
   }
-  if (k.count > 0 && (k.limit <= kClusterLeast || k.count <= kLargeClusters)) pl.classes.push_back(k);
-  else pl.clist.clear();
+  bool off = pl.classes.size() > 1 && (!fit || units > sms || pl.classes.size() > (size_t)pt_ctx::kSides + 1);
+  for (const ClusterClass &k : pl.classes) off |= k.limit > kClusterLeast && k.count > kLargeClusters;
+  if (off) {
+    pl.classes.clear();
+    pl.clist.clear();
+  }
   // Blocks whose results are waited for one half-sweep at a time are better
   // off alone on an SM while there are SMs to spare: shared memory asked for
   // beyond their own keeps others away.
@@ -551,6 +561,10 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
     if (ce == cudaSuccess) ce = prepare_solve(all, pl.cfg, ctx->sms, &ctx->solve_grid[pl.cfg]);
     if (ce != cudaSuccess) return cuda_fail(ctx, ce, "solve prepare");
   }
+  if (pl.classes.size() > 1) {
+    ce = ctx->make_sides((int)pl.classes.size() - 1);
+    if (ce != cudaSuccess) return cuda_fail(ctx, ce, "side streams");
+  }
   grid = std::max(1, std::min(ctx->solve_grid[pl.cfg], P.ntiles));
   ctx->last_grid = grid;
   ctx->last_cfg = pl.cfg;
@@ -576,8 +590,17 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
     if (e == cudaSuccess) e = cudaMemsetAsync(base + L.err, 0, sizeof(int), st);
     if (e == cudaSuccess) e = launch_assembly(P, pl.tc, st, any_warm);
     if (e == cudaSuccess) e = record(ctx->ev[1], capturing);
-    for (const ClusterClass &k : pl.classes)
-      if (e == cudaSuccess) e = launch_cluster(P, pl.tc, k, reinterpret_cast<const int *>(base + L.clist), st);
+    // the first size on this stream, the others beside it
+    const size_t nk = pl.classes.size();
+    if (e == cudaSuccess && nk > 1) e = cudaEventRecord(ctx->forked, st);
+    for (size_t k = 1; k < nk && e == cudaSuccess; ++k) {
+      cudaStream_t side = ctx->side[k - 1];
+      e = cudaStreamWaitEvent(side, ctx->forked, 0);
+      if (e == cudaSuccess) e = launch_cluster(P, pl.tc, pl.classes[k], reinterpret_cast<const int *>(base + L.clist), side);
+      if (e == cudaSuccess) e = cudaEventRecord(ctx->joined[k - 1], side);
+    }
+    if (e == cudaSuccess && nk > 0) e = launch_cluster(P, pl.tc, pl.classes[0], reinterpret_cast<const int *>(base + L.clist), st);
+    for (size_t k = 1; k < nk && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(st, ctx->joined[k - 1], 0);
     if (e == cudaSuccess) e = launch_prepared(P, pl.cfg, grid, st);
     if (e == cudaSuccess) e = record(ctx->ev[2], capturing);
     if (e == cudaSuccess)
@@ -758,6 +781,7 @@ pt_status pt_ctx_destroy(pt_ctx *ctx) {
       cudaSetDevice(ctx->device);
       if (ctx->stream) cudaStreamSynchronize(ctx->stream);
       ctx->release();
+      ctx->drop_sides();
       if (ctx->stream) cudaStreamDestroy(ctx->stream);
     }
     delete ctx;
