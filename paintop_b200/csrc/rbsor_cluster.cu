@@ -62,6 +62,13 @@ __device__ __forceinline__ void cluster_sync() {
   __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
+// Where the warps of all blocks meet around rows shown by plain stores. Before
+// them, since an asynchronous store of an earlier half-sweep to the same row may
+// still be on its way: its sender waits for its neighbours' rows, never for its own
+// to arrive, and a later plain store of the same thread is not ordered behind
+// it. Every block has waited for all rows sent to it when it comes here. And
+// after them, before the rows are read.
+__device__ __forceinline__ void cluster_meet() { cluster_sync(); }
 __device__ __forceinline__ unsigned remote(unsigned smem_addr, unsigned rank) {
   unsigned a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
@@ -271,7 +278,10 @@ __device__ __forceinline__ void keep_books(const KParams &P, Shared &sh, unsigne
   int mode = sh.st.mode, s = sh.st.s, it = 0;
   unsigned x = 0, dc = 0;  // exchanges and decisions so far
   for (unsigned t = 0; mode != M_DONE; ++t) {
-    if (mode != M_SWEEP) cluster_sync();  // the other warps' (a re-run's start, or after the fold)
+    if (mode != M_SWEEP) {  // a re-run's start, or the fold: before and after the other warps show it
+      cluster_meet();
+      cluster_meet();
+    }
     bar_wait(bar0 + 8u * (B_SUMS + (t & 1u)), (t >> 1) & 1u, &sh.gave_up, P.err);
     const int nsum = mode == M_SWEEP ? s : (mode == M_FOLD ? 1 : 0);  // (a fold step ends with the new residual)
     double nrm[kMaxS], rel[kMaxS];
@@ -586,14 +596,16 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
         it += ahead;
       }
     } else if (mode == M_REDO) {  // step t - 1 or t - 2 again from its start, with fewer sweeps
+      cluster_meet();
       if (mine) {
         show(0, false);
         show(1, false);
       }
-      cluster_sync();
+      cluster_meet();
       sweeps(t++, s, true);
       decision();
     } else {  // M_FOLD: u += e on interior cells, e = 0; then g = -r(u), r in FP64 exactly as residual_l2 (poisson.rs:315-321)
+      cluster_meet();
 #pragma unroll
       for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -616,7 +628,7 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
         show(1, false);
       }
       __threadfence();
-      cluster_sync();
+      cluster_meet();
       const double lam4 = d.lambda + 4.0;
       double a = 0.0;
 #pragma unroll
