@@ -219,6 +219,8 @@ struct KParams {
   int *rmax;               // per RegionDesc: largest region size
   Route *route;            // per system: its cluster's split, n = 0 for k_solve's (null: all are)
   bool many;               // the call fills the GPU with clusters (cluster_route)
+  bool silent;             // tests: a cluster's last block sends no sums, so that a wait runs out
+  unsigned long long wait_ns;  // limit of a wait inside a cluster
 };
 
 }  // namespace ptk

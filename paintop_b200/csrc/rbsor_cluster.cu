@@ -62,13 +62,6 @@ __device__ __forceinline__ void cluster_sync() {
   __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
-// Where the warps of all blocks meet around rows shown by plain stores. Before
-// them, since an asynchronous store of an earlier half-sweep to the same row may
-// still be on its way: its sender waits for its neighbours' rows, never for its own
-// to arrive, and a later plain store of the same thread is not ordered behind
-// it. Every block has waited for all rows sent to it when it comes here. And
-// after them, before the rows are read.
-__device__ __forceinline__ void cluster_meet() { cluster_sync(); }
 __device__ __forceinline__ unsigned remote(unsigned smem_addr, unsigned rank) {
   unsigned a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
@@ -98,6 +91,11 @@ __device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
 __device__ __forceinline__ void bar_arrive(unsigned bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// The same, ordering the thread's (and, after a __syncwarp, its warp's) stores
+// before what other blocks do after they have seen it.
+__device__ __forceinline__ void bar_arrive_cluster(unsigned bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ bool bar_try(unsigned bar, unsigned parity) {
   unsigned ok;
   asm volatile(
@@ -107,23 +105,35 @@ __device__ __forceinline__ bool bar_try(unsigned bar, unsigned parity) {
       : "memory");
   return ok != 0;
 }
-constexpr unsigned long long kWaitNs = 2ull * 1000000000ull;
-// Wait for a barrier's phase, at most kWaitNs (the clock is read every 4096
+// Wait for a barrier's phase, at most P.wait_ns (the clock is read every 4096
 // tries); a block whose wait gave up raises the kernel's error word and its own
-// flag and waits no more, and the cluster ends at its next decision.
-__device__ __forceinline__ void bar_wait(unsigned bar, unsigned parity, volatile int *gave_up, int *err) {
+// flag and waits no more, and its neighbours give up on the error word or on it.
+__device__ __forceinline__ void bar_wait(unsigned bar, unsigned parity, volatile int *gave_up, const KParams &P) {
   unsigned long long t0 = 0;
   for (unsigned k = 1; !bar_try(bar, parity); ++k) {
     if (k & 4095u) continue;
     if (*gave_up) return;
     const unsigned long long now = gtimer();
     if (!t0) t0 = now;
-    if (now - t0 > kWaitNs) {
+    if (ld_vol(P.err) != 0 || now - t0 > P.wait_ns) {
       *gave_up = 1;
-      atomicCAS(err, 0, KERR_STALLED);
+      atomicCAS(P.err, 0, KERR_STALLED);
       return;
     }
   }
+}
+
+// The end of every thread: the only hardware barrier of the cluster after the
+// first, so that it pairs with nothing else wherever a block gave up, and nobody
+// leaves while another block may still store into its shared memory. After an
+// error asynchronous stores may be under way that nobody waited for: their block
+// stays for kSettleNs more, a thousand times what one takes.
+constexpr unsigned long long kSettleNs = 1000000ull;
+__device__ __forceinline__ void leave(const KParams &P) {
+  cluster_sync();
+  if (ld_vol(P.err) == 0) return;
+  const unsigned long long t0 = gtimer();
+  while (gtimer() - t0 < kSettleNs) __nanosleep(1000);
 }
 
 __device__ __forceinline__ double residual(float l, float r, float u, float dn, float e, float g, double dd) {
@@ -251,8 +261,9 @@ __device__ __forceinline__ void edges(const Patch<R> &p, float2 &right, float2 &
 // A block's shared variables. bars: the rows of colours 0, 1 from the block
 // above (0, 1) and below (2, 3); the cluster's sums, by the exchange's parity
 // (4, 5); the warps' meetings (6); the block's sums and the decisions, by the
-// step's parity (7, 8 and 9, 10).
-enum Bar { B_UP = 0, B_DN = 2, B_SLOT = 4, B_MEET = 6, B_SUMS = 7, B_DECIDED = 9, B_COUNT = 11 };
+// step's parity (7, 8 and 9, 10); the cluster's meetings: the block's warps have
+// come (11), all blocks' have, by the meeting's parity (12, 13).
+enum Bar { B_UP = 0, B_DN = 2, B_SLOT = 4, B_MEET = 6, B_SUMS = 7, B_DECIDED = 9, B_HERE = 11, B_ALL = 12, B_COUNT = 14 };
 struct Shared {
   SysDesc d;
   SysState st;
@@ -276,13 +287,19 @@ __device__ __forceinline__ void keep_books(const KParams &P, Shared &sh, unsigne
   const unsigned long long t_start = gtimer();
   const unsigned slot0 = (unsigned)__cvta_generic_to_shared(&sh.slot[0][rank][0]);
   int mode = sh.st.mode, s = sh.st.s, it = 0;
-  unsigned x = 0, dc = 0;  // exchanges and decisions so far
+  unsigned x = 0, dc = 0, meets = 0;  // exchanges, decisions and cluster meetings so far
+  auto cluster_meet = [&]() {  // the block's warps have come: tell every block
+    bar_wait(bar0 + 8u * B_HERE, meets & 1u, &sh.gave_up, P);
+    __syncwarp();
+    if (lane < n) bar_arrive_cluster(remote(bar0 + 8u * (B_ALL + (meets & 1u)), lane));
+    ++meets;
+  };
   for (unsigned t = 0; mode != M_DONE; ++t) {
     if (mode != M_SWEEP) {  // a re-run's start, or the fold: before and after the other warps show it
       cluster_meet();
       cluster_meet();
     }
-    bar_wait(bar0 + 8u * (B_SUMS + (t & 1u)), (t >> 1) & 1u, &sh.gave_up, P.err);
+    bar_wait(bar0 + 8u * (B_SUMS + (t & 1u)), (t >> 1) & 1u, &sh.gave_up, P);
     const int nsum = mode == M_SWEEP ? s : (mode == M_FOLD ? 1 : 0);  // (a fold step ends with the new residual)
     double nrm[kMaxS], rel[kMaxS];
     bool late = false;
@@ -295,7 +312,7 @@ __device__ __forceinline__ void keep_books(const KParams &P, Shared &sh, unsigne
       for (int o = 8; o > 0; o >>= 1)
 #pragma unroll
         for (int j = 0; j < kMaxS; ++j) mine[j] += __shfl_xor_sync(0xffffffffu, mine[j], o);
-      if (lane < n) {
+      if (lane < n && !(P.silent && (int)rank == n - 1)) {
         const unsigned rto = remote(to, lane), rbar = remote(bar, lane);
 #pragma unroll
         for (int j = 0; j < kMaxS; ++j)
@@ -305,7 +322,7 @@ __device__ __forceinline__ void keep_books(const KParams &P, Shared &sh, unsigne
       }
       if (lane == 0) bar_expect(bar, 8u * (unsigned)(n * nsum + 1));
       __syncwarp();
-      bar_wait(bar, (x >> 1) & 1u, &sh.gave_up, P.err);
+      bar_wait(bar, (x >> 1) & 1u, &sh.gave_up, P);
       __syncwarp();
 #pragma unroll
       for (int j = 0; j < kMaxS; ++j) mine[j] = lane < n && j < nsum ? sh.slot[x & 1u][lane][j] : 0.0;
@@ -349,7 +366,7 @@ __device__ __forceinline__ void keep_books(const KParams &P, Shared &sh, unsigne
       it += s;
       if (next != M_SWEEP && next != M_DONE && next_block(P, sh, it) > 0) {
         ++t;  // the block of sweeps begun meanwhile is void
-        bar_wait(bar0 + 8u * (B_SUMS + (t & 1u)), (t >> 1) & 1u, &sh.gave_up, P.err);
+        bar_wait(bar0 + 8u * (B_SUMS + (t & 1u)), (t >> 1) & 1u, &sh.gave_up, P);
       }
     }
     it = sh.st.iterations;
@@ -379,7 +396,9 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
     sh.st = load_sys_state(P.st + sys);
     sh.gave_up = 0;
     for (int k = 0; k < B_COUNT; ++k)
-      bar_init(bar0 + 8u * k, k == B_MEET || k == B_SUMS || k == B_SUMS + 1 ? (unsigned)nwa : 1u);
+      bar_init(bar0 + 8u * k, k == B_MEET || k == B_SUMS || k == B_SUMS + 1 || k == B_HERE ? (unsigned)nwa
+                              : k == B_ALL || k == B_ALL + 1                              ? (unsigned)n
+                                                                                          : 1u);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int k = 0; k < 2; ++k) {
       if (rank > 0) bar_expect(bar0 + 8u * (B_UP + k), row_bytes);
@@ -421,7 +440,7 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
   if (books) {
     keep_books(P, sh, bar0, n, nwa, rank);
     if (rank == 0 && lane == 0) P.st[sys] = sh.st;
-    cluster_sync();
+    leave(P);
     return;
   }
   if (warp >= nwa) return;  // (the cluster's barriers count the threads that stay)
@@ -437,7 +456,7 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
   const unsigned to_bot = to_dn ? remote(base, rank + 1) + 16u * (unsigned)v : 0u;
   // what the neighbours read of colour h (a constant after inlining); async:
   // the rows for other blocks count off their barriers (in a half-sweep; else
-  // a cluster barrier follows)
+  // the blocks meet before and after)
   auto show = [&](int h, bool async) {
     const float4 a = p.e[h][0], b = p.e[h][R - 1];
     float2 right, left;
@@ -457,18 +476,18 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
     }
   };
   // bit h: the parity of colour h's rows; bit 2: of the meetings; bits 3, 4: of
-  // the even and odd decisions
+  // the even and odd decisions; from bit 5 on: cluster meetings so far
   unsigned phase = 0;
   // the other blocks' rows of colour h, by the threads that read them; the
   // first of a row arms the barrier's next phase
   auto wait_rows = [&](int h) {
     const unsigned par = (phase >> h) & 1u;
     if (to_up) {
-      bar_wait(bar0 + 8u * (B_UP + h), par, &sh.gave_up, P.err);
+      bar_wait(bar0 + 8u * (B_UP + h), par, &sh.gave_up, P);
       if (v == 0) bar_expect(bar0 + 8u * (B_UP + h), row_bytes);
     }
     if (to_dn) {
-      bar_wait(bar0 + 8u * (B_DN + h), par, &sh.gave_up, P.err);
+      bar_wait(bar0 + 8u * (B_DN + h), par, &sh.gave_up, P);
       if (v == 0) bar_expect(bar0 + 8u * (B_DN + h), row_bytes);
     }
     phase ^= 1u << h;
@@ -480,8 +499,21 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
     if (lane == 0) bar_arrive(bar0 + 8u * bar);
   };
   auto meet_wait = [&]() {
-    bar_wait(bar0 + 8u * B_MEET, (phase >> 2) & 1u, &sh.gave_up, P.err);
+    bar_wait(bar0 + 8u * B_MEET, (phase >> 2) & 1u, &sh.gave_up, P);
     phase ^= 4u;
+  };
+  // All blocks' warps meet, around rows shown by plain stores. Before them, since
+  // an asynchronous store of an earlier half-sweep to the same row may still be on
+  // its way: its sender waits for its neighbours' rows, never for its own to
+  // arrive, and a later plain store of the same thread is not ordered behind it.
+  // Every block has waited for all rows sent to it when it comes here. And after
+  // them, before the rows are read. Two barriers in turn: a block comes to the
+  // meeting after next only when all have passed this one.
+  auto cluster_meet = [&]() {
+    __syncwarp();
+    if (lane == 0) bar_arrive_cluster(bar0 + 8u * B_HERE);
+    bar_wait(bar0 + 8u * (B_ALL + ((phase >> 5) & 1u)), (phase >> 6) & 1u, &sh.gave_up, P);
+    phase += 32u;
   };
   auto near = [&](int o) {
     return Near{ld_rows(aw + W::BOT + o * W::ROWS), ld_rows(aw + below + W::TOP + o * W::ROWS),
@@ -563,7 +595,7 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
   int mode = sh.st.mode, s = sh.st.s;
   auto decision = [&]() {
     const unsigned k = dc & 1u;
-    bar_wait(bar0 + 8u * (B_DECIDED + k), (phase >> (3 + k)) & 1u, &sh.gave_up, P.err);
+    bar_wait(bar0 + 8u * (B_DECIDED + k), (phase >> (3 + k)) & 1u, &sh.gave_up, P);
     phase ^= 8u << k;
     ++dc;
     if (sh.gave_up) { mode = M_DONE; return; }
@@ -658,7 +690,7 @@ __device__ __forceinline__ void solve_region(const KParams &P, const Route &rt, 
       it = sh.st.iterations;
     }
   }
-  cluster_sync();  // nobody leaves while another block may still store into its shared memory
+  leave(P);
 }
 
 }  // namespace

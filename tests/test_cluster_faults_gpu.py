@@ -1,0 +1,41 @@
+"""A cluster solve whose wait runs out, made without a GPU fault: with
+PAINTOP_CUDA_FAULT=cluster-silent the last block of every cluster sends no sums of
+squares, the blocks' waits for them end after 20 ms, all blocks leave together, the
+call returns PT_TIMEOUT and the context stays usable."""
+import numpy as np
+import pytest
+
+from tests import device_solve
+from tests.test_fault_injection_gpu import injected
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(w, h, c):
+    rng = np.random.default_rng(w * 7 + h)
+    src, tgt = rng.random(h * w * c, dtype=np.float32), rng.random(h * w * c, dtype=np.float32)
+    mask = np.zeros((h, w), np.float32)
+    mask[1:h - 1, 1:w - 1] = 1.0
+    return src, tgt, mask.reshape(-1)
+
+
+# one block; several; sixteen of four-row patches
+@pytest.mark.parametrize("w,h,c", [(30, 20, 1), (97, 71, 3), (300, 200, 2), (400, 400, 1)])
+@pytest.mark.parametrize("device", [False, True])
+def test_silent_block_ends_in_a_timeout_and_the_context_survives(ctx, w, h, c, device):
+    from paintop_b200 import _lib
+    src, tgt, mask = _problem(w, h, c)
+    p = dict(source=src, target=tgt, mask=mask, width=w, height=h, channels=c, tolerance=1e-7, max_iterations=200)
+
+    def solve():
+        out, per = (device_solve.solve_batch(ctx, [p]) if device else ctx.solve_batch([p]))[0][:2]
+        return out, [(r["iterations"], r["stop_reason"]) for r in per]
+
+    want, reports = solve()
+    for _ in range(2):
+        with injected("cluster-silent"):
+            with pytest.raises(_lib.CudaError) as e:
+                solve()
+        assert e.value.status == _lib.PT_TIMEOUT and "gave up" in ctx.last_error()
+        got, again = solve()
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32)) and again == reports

@@ -11,7 +11,7 @@ SOURCE = open(os.path.join(ROOT, "paintop_b200", "csrc", "rbsor_cluster.cu")).re
 def _body(head):
     """The content of the brace that `head` opens."""
     at = SOURCE.index(head)
-    i = start = at + head.index("{")
+    i = start = at + head.index("{") if "{" in head else SOURCE.index("{", at)
     depth = 0
     while True:
         depth += {"{": 1, "}": -1}.get(SOURCE[i], 0)
@@ -41,3 +41,19 @@ def test_the_books_meet_as_often_as_the_workers():
     books = _body("if (mode != M_SWEEP) {")
     for body in _branches():
         assert books.count("cluster_meet()") == body.count("cluster_meet()")
+
+
+def test_the_hardware_barrier_pairs_only_starts_and_ends():
+    """barrier.cluster is anonymous: a block that gave up a wait and leaves must not
+    pair with another's re-run or fold. So a thread takes it once before its first
+    bounded wait and once in leave()."""
+    region = _body("__device__ __forceinline__ void solve_region(")
+    assert region.count("cluster_sync()") == 1
+    assert region.index("cluster_sync()") < region.index("keep_books(")
+    assert "cluster_sync()" not in _body("__device__ __forceinline__ void keep_books(")
+    leave = _body("__device__ __forceinline__ void leave(")
+    assert leave.count("cluster_sync()") == 1 and SOURCE.count("barrier.cluster.arrive") == 1
+    # every way out after the first barrier is leave(), except for warps without patches before it counts them
+    rest = region[region.index("cluster_sync()"):]
+    ends = re.findall(r"leave\(P\);\s*(?:return;|$)", rest.rstrip())
+    assert len(ends) == 2
