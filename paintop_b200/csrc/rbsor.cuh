@@ -126,9 +126,10 @@ struct SysState {
   int pad2;
 };
 
-// Control words of the persistent kernel: [2] systems done. The host zeroes
-// them before every launch.
-constexpr int kBarWords = 16;
+// Control words of a call's kernels, zeroed by the host before every launch:
+// [2] systems done; [4], [5] the clock when k_init ran, from which the wall
+// budget of every kernel after it counts; [6] a wait inside a cluster gave up.
+constexpr int kBarWords = 16, kBarStart = 4, kBarGaveUp = 6;
 // A claim word's low half once its system is done: never below any tile count,
 // and far from overflowing into the generation half however often it is bumped.
 constexpr unsigned kClaimDone = 0x7fffffffu;

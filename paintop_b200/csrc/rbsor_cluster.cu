@@ -35,7 +35,9 @@
 // groups of four need 21 for four). Every block of a cluster takes the same
 // steps, decided from the same sums by the same code; every wait for another
 // warp's or block's data is bounded (bar_wait). The wall budget is tested by
-// the first block once a step and passed on with its sums.
+// the first block once a step and passed on with its sums; it counts from the
+// call's start (call_start), for clusters that run one after another and for
+// k_solve after them alike.
 #include "rbsor.cuh"
 #include "rbsor_device.cuh"
 #include "rbsor_launch.h"
@@ -106,8 +108,9 @@ __device__ __forceinline__ bool bar_try(unsigned bar, unsigned parity) {
   return ok != 0;
 }
 // Wait for a barrier's phase, at most P.wait_ns (the clock is read every 4096
-// tries); a block whose wait gave up raises the kernel's error word and its own
-// flag and waits no more, and its neighbours give up on the error word or on it.
+// tries); a block whose wait gave up raises the kernel's error word, the call's
+// word of that and its own flag and waits no more, and others give up on the
+// call's word, or on the block.
 __device__ __forceinline__ void bar_wait(unsigned bar, unsigned parity, volatile int *gave_up, const KParams &P) {
   unsigned long long t0 = 0;
   for (unsigned k = 1; !bar_try(bar, parity); ++k) {
@@ -115,9 +118,10 @@ __device__ __forceinline__ void bar_wait(unsigned bar, unsigned parity, volatile
     if (*gave_up) return;
     const unsigned long long now = gtimer();
     if (!t0) t0 = now;
-    if (ld_vol(P.err) != 0 || now - t0 > P.wait_ns) {
+    if (*reinterpret_cast<volatile unsigned *>(P.bar + kBarGaveUp) != 0 || now - t0 > P.wait_ns) {
       *gave_up = 1;
       atomicCAS(P.err, 0, KERR_STALLED);
+      atomicExch(P.bar + kBarGaveUp, 1u);
       return;
     }
   }
@@ -125,13 +129,13 @@ __device__ __forceinline__ void bar_wait(unsigned bar, unsigned parity, volatile
 
 // The end of every thread: the only hardware barrier of the cluster after the
 // first, so that it pairs with nothing else wherever a block gave up, and nobody
-// leaves while another block may still store into its shared memory. After an
-// error asynchronous stores may be under way that nobody waited for: their block
+// leaves while another block may still store into its shared memory. After a wait
+// gave up asynchronous stores may be under way that nobody waited for: every block
 // stays for kSettleNs more, a thousand times what one takes.
 constexpr unsigned long long kSettleNs = 1000000ull;
 __device__ __forceinline__ void leave(const KParams &P) {
   cluster_sync();
-  if (ld_vol(P.err) == 0) return;
+  if (*reinterpret_cast<volatile unsigned *>(P.bar + kBarGaveUp) == 0) return;
   const unsigned long long t0 = gtimer();
   while (gtimer() - t0 < kSettleNs) __nanosleep(1000);
 }
@@ -284,7 +288,7 @@ __device__ __forceinline__ int next_block(const KParams &P, const Shared &sh, in
 __device__ __forceinline__ void keep_books(const KParams &P, Shared &sh, unsigned bar0, const int n, const int nwa,
                                            const unsigned rank) {
   const int lane = threadIdx.x & 31;
-  const unsigned long long t_start = gtimer();
+  const unsigned long long t_start = *call_start(P);
   const unsigned slot0 = (unsigned)__cvta_generic_to_shared(&sh.slot[0][rank][0]);
   int mode = sh.st.mode, s = sh.st.s, it = 0;
   unsigned x = 0, dc = 0, meets = 0;  // exchanges, decisions and cluster meetings so far
@@ -318,7 +322,7 @@ __device__ __forceinline__ void keep_books(const KParams &P, Shared &sh, unsigne
         for (int j = 0; j < kMaxS; ++j)
           if (j < nsum) st_async(rto + 8u * (unsigned)j, mine[j], rbar);
         if (rank == 0)
-          st_async(rto + 8u * kMaxS, ld_vol(P.err) != 0 || gtimer() - t_start > P.budget_ns ? 1.0 : 0.0, rbar);
+          st_async(rto + 8u * kMaxS, ld_vol(P.err) != 0 || over_budget(P, t_start) ? 1.0 : 0.0, rbar);
       }
       if (lane == 0) bar_expect(bar, 8u * (unsigned)(n * nsum + 1));
       __syncwarp();

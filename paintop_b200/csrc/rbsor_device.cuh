@@ -21,6 +21,16 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
   return v;
 }
 
+// The call's clock: its start, and whether its wall budget is spent. (Another
+// multiprocessor's clock may lag behind the one that stored the start.)
+__device__ __forceinline__ unsigned long long *call_start(const KParams &P) {
+  return reinterpret_cast<unsigned long long *>(P.bar + kBarStart);
+}
+__device__ __forceinline__ bool over_budget(const KParams &P, unsigned long long t_start) {
+  const unsigned long long now = gtimer();
+  return now > t_start && now - t_start > P.budget_ns;
+}
+
 __device__ __forceinline__ int ld_vol(const int *p) { return *reinterpret_cast<const volatile int *>(p); }
 
 // Deterministic block sum: fixed xor-butterfly inside each warp, then warps in

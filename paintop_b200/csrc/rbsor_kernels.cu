@@ -304,6 +304,7 @@ __global__ void k_init(KParams P) {
   }
   __syncthreads();
   if (threadIdx.x != 0) return;
+  if (sys == 0) *call_start(P) = gtimer();
   const int bx0 = sbox[0], by0 = sbox[1], bx1 = sbox[2], by1 = sbox[3];
   int n = 0;
   for (int w = 0; w < (int)(blockDim.x >> 5); ++w) n += sn[w];
@@ -781,7 +782,7 @@ __device__ int claim_tile(const KParams &P, int rot, int *idx, unsigned *gen,
     int stop = 0;
     if (lane == 0) {
       stop = ld_vol(P.err) != 0;
-      if (!stop && gtimer() - t_start > P.budget_ns) {
+      if (!stop && over_budget(P, t_start)) {
         atomicCAS(P.err, 0, KERR_DEADLINE);
         stop = 1;
       }
@@ -838,7 +839,7 @@ __global__ void __launch_bounds__((Geo<S, TH>::NT), 2) k_solve(KParams P) {
   double *sred = reinterpret_cast<double *>(sC + 2 * G::PLANE);
   __shared__ int s_last, s_sys, s_idx;
   __shared__ unsigned s_gen;
-  const unsigned long long t_start = gtimer();
+  const unsigned long long t_start = *call_start(P);
   int rot = P.nsys > 0 ? (int)(blockIdx.x % (unsigned)P.nsys) : 0;
 
   for (;;) {

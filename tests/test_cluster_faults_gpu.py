@@ -39,3 +39,45 @@ def test_silent_block_ends_in_a_timeout_and_the_context_survives(ctx, w, h, c, d
         assert e.value.status == _lib.PT_TIMEOUT and "gave up" in ctx.last_error()
         got, again = solve()
         assert np.array_equal(got.view(np.uint32), want.view(np.uint32)) and again == reports
+
+
+def test_budget_bounds_a_call_of_more_clusters_than_run_at_a_time(cuda_lib):
+    """All systems sweep to their cap, so that a call's time is that of its waves of
+    clusters; a budget of half of it ends the call, and twice it does not."""
+    from paintop_b200 import _lib
+    c = _lib.Context(0)
+    try:
+        src, tgt, mask = _problem(256, 256, 1)
+        probs = [dict(source=src, target=tgt, mask=mask, width=256, height=256, channels=1, tolerance=1e-30,
+                      omega=1.0, max_iterations=3000)] * 256
+        c.solve_batch(probs[:1])
+        one = c.last_timing()[0]
+        want = c.solve_batch(probs)[-1]
+        assert want[1][0]["iterations"] == 3000
+        whole = c.last_timing()[0]
+        assert whole > 4 * one  # waves
+        c.set_budget(whole / 2e3)
+        for solve in (c.solve_batch, lambda p: device_solve.solve_batch(c, p)):
+            with pytest.raises(_lib.CudaError) as e:
+                solve(probs)
+            assert e.value.status == _lib.PT_TIMEOUT and "wall budget" in c.last_error()
+        c.set_budget(whole * 2e-3)
+        again = c.solve_batch(probs)[-1]
+        assert np.array_equal(again[0].view(np.uint32), want[0].view(np.uint32))
+    finally:
+        c.close()
+
+
+def test_budget_ends_one_cluster(cuda_lib):
+    from paintop_b200 import _lib
+    c = _lib.Context(0)
+    try:
+        src, tgt, mask = _problem(97, 71, 3)
+        c.set_budget(1e-4)
+        with pytest.raises(_lib.CudaError) as e:
+            c.solve(src, tgt, mask, 97, 71, 3, max_iterations=100000, tolerance=1e-30, omega=1.0)
+        assert e.value.status == _lib.PT_TIMEOUT and "wall budget" in c.last_error()
+        c.set_budget(600)
+        assert c.solve(src, tgt, mask, 97, 71, 3, max_iterations=10)[1][0]["iterations"] == 10
+    finally:
+        c.close()
