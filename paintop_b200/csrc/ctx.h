@@ -45,10 +45,18 @@ struct pt_ctx {
     mgkey.clear();
   }
 
+  // Until nothing of a call runs any more, on the side streams either: a call
+  // that failed between its fork and its join left those unwaited for.
+  void wait_all() {
+    cudaStreamSynchronize(stream);
+    for (cudaStream_t s : side)
+      if (s) cudaStreamSynchronize(s);
+  }
+
   bool reserve(size_t bytes) {
     if (bytes <= arena_cap) return true;
     if (arena) {
-      cudaStreamSynchronize(stream);
+      wait_all();
       drop_graphs();
       cudaFree(arena);
       arena = nullptr;

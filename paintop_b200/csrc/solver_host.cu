@@ -384,14 +384,15 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
     }
   }
   h2d += L.plan_end;
-  // (a call that fails below leaves the staging only when its copies are done)
+  // (a call that fails below leaves the staging and the arena only when nothing
+  // of it runs any more)
   struct Settle {
-    cudaStream_t st;
+    pt_ctx *ctx;
     bool done = false;
     ~Settle() {
-      if (!done) cudaStreamSynchronize(st);
+      if (!done) ctx->wait_all();
     }
-  } settle{st};
+  } settle{ctx};
   auto stage = [&](size_t at, const void *from, size_t bytes) {
     if (bytes) std::memcpy(pin + at, from, bytes);
   };
@@ -790,7 +791,7 @@ pt_status pt_ctx_destroy(pt_ctx *ctx) {
     {
       std::lock_guard<std::mutex> lock(ctx->mu);
       cudaSetDevice(ctx->device);
-      if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+      if (ctx->stream) ctx->wait_all();
       ctx->release();
       ctx->drop_sides();
       if (ctx->stream) cudaStreamDestroy(ctx->stream);
