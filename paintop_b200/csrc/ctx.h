@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <cstdlib>
 #include <mutex>
 #include <string>
 
@@ -24,8 +25,9 @@ struct pt_ctx {
   double last_call_ms = 0.0;   // whole call from first upload to last download
   long long last_launches = 0; // kernels launched by the last call
   unsigned long long last_h2d = 0, last_d2h = 0;  // bytes the last solve moved each way
-  void *pin = nullptr;         // page-locked staging of plans and results, grown to a high-water mark
+  void *pin = nullptr;         // staging of plans and results, grown to a high-water mark
   size_t pin_cap = 0;
+  bool pin_paged = false;      // page-locked memory was not to be had
   int solve_grid[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // blocks of k_solve that fit the device, by tile configuration
   static constexpr int kSides = 7;
   cudaStream_t side[kSides] = {};       // for launches beside one another (made when first needed)
@@ -96,17 +98,27 @@ struct pt_ctx {
     if (forked) { cudaEventDestroy(forked); forked = nullptr; }
   }
 
-  // Staging for at least `bytes`; the calls wait for their copies before they
-  // return, so what is there is free.
-  bool reserve_pin(size_t bytes) {
-    if (bytes <= pin_cap) return true;
-    if (pin) cudaFreeHost(pin);
+  void drop_pin() {
+    if (pin) {
+      if (pin_paged) std::free(pin);
+      else cudaFreeHost(pin);
+    }
     pin = nullptr;
     pin_cap = 0;
+    pin_paged = false;
+  }
+
+  // Staging for at least `bytes`; the calls wait for their copies before they
+  // return, so what is there is free. Where no more memory can be page-locked,
+  // pageable memory does: its copies are slower, and as safe.
+  bool reserve_pin(size_t bytes) {
+    if (bytes <= pin_cap) return true;
+    drop_pin();
     if (cudaMallocHost(&pin, bytes + bytes / 4) != cudaSuccess) {
       cudaGetLastError();
-      pin = nullptr;
-      return false;
+      pin = std::malloc(bytes + bytes / 4);
+      if (!pin) return false;
+      pin_paged = true;
     }
     pin_cap = bytes + bytes / 4;
     return true;
@@ -114,9 +126,7 @@ struct pt_ctx {
 
   void release() {
     drop_graphs();
-    if (pin) cudaFreeHost(pin);
-    pin = nullptr;
-    pin_cap = 0;
+    drop_pin();
     for (auto &e : ev)
       if (e) { cudaEventDestroy(e); e = nullptr; }
     if (arena) cudaFree(arena);

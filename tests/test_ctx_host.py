@@ -70,3 +70,16 @@ def test_a_failed_solve_waits_for_the_whole_context():
     text = open(os.path.join(ROOT, "paintop_b200", "csrc", "solver_host.cu")).read()
     settle = text[text.index("~Settle() {"):]
     assert "ctx->wait_all();" in settle[:settle.index("}")]
+
+
+def test_staging_without_page_locked_memory(tmp_path):
+    """A call needs the staging; page-locked memory is a matter of speed."""
+    run(tmp_path, """
+  pinned_fails = true;
+  CHECK(x.reserve_pin(1000) && x.pin && x.pin_cap >= 1000);
+  static_cast<char *>(x.pin)[999] = 1;
+  CHECK(x.reserve_pin(5000) && x.pin_cap >= 5000);
+  pinned_fails = false;
+  CHECK(x.reserve_pin(50000) && x.pin_cap >= 50000);
+  x.release();
+  CHECK(!x.pin && !x.pin_cap);""")
