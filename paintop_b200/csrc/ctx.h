@@ -29,6 +29,7 @@ struct pt_ctx {
   size_t pin_cap = 0;
   bool pin_paged = false;      // page-locked memory was not to be had
   int solve_grid[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // blocks of k_solve that fit the device, by tile configuration
+  int cluster_room = -1;       // largest clusters that fit the device at a time (-1: not asked yet)
   static constexpr int kSides = 7;
   cudaStream_t side[kSides] = {};       // for launches beside one another (made when first needed)
   cudaEvent_t forked = nullptr, joined[kSides] = {};

@@ -42,6 +42,9 @@
 #include "rbsor_device.cuh"
 #include "rbsor_launch.h"
 
+#include <algorithm>
+#include <climits>
+
 namespace ptk {
 
 namespace {
@@ -724,14 +727,37 @@ cudaError_t each_instance(F f) {
   if (e == cudaSuccess) e = f(k_cluster_solve<4, kClusterMost>, 4, kClusterMost);
   return e;
 }
+
+// The launch of `count` clusters of `blocks` blocks; `at` is its storage.
+cudaLaunchConfig_t cluster_config(int limit, int blocks, int count, int smem, cudaStream_t stream,
+                                  cudaLaunchAttribute *at) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)count * (unsigned)blocks);
+  cfg.blockDim = dim3((unsigned)limit + 32u);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = stream;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = (unsigned)blocks;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
 }  // namespace
 
-cudaError_t prepare_cluster() {
+cudaError_t prepare_cluster(int *room) {
   static_assert(kClusterAlone >= cluster_smem(4, kClusterMost) && cluster_smem(4, kClusterLeast) <= 110 * 1024,
                 "shared memory of the blocks");
-  return each_instance([](auto k, int, int) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterAlone);
+  *room = INT_MAX;
+  return each_instance([room](auto k, int, int limit) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterAlone);
+    cudaLaunchAttribute at{};
+    cudaLaunchConfig_t cfg = cluster_config(limit, kClusterMax, 1, kClusterAlone, nullptr, &at);
+    int fit = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fit, k, &cfg);
+    *room = std::min(*room, fit);
+    return e;
   });
 }
 
@@ -740,17 +766,9 @@ cudaError_t launch_cluster(const KParams &P, const TileConfig &tc, const Cluster
   if (k.count == 0) return cudaSuccess;
   return each_instance([&](auto kernel, int rows, int limit) {
     if (limit != k.limit || !(rows == 2 ? k.rows2 : k.rows4)) return cudaSuccess;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)k.count * (unsigned)k.blocks);
-    cfg.blockDim = dim3((unsigned)limit + 32u);
-    cfg.dynamicSmemBytes = (size_t)(k.alone ? kClusterAlone : cluster_smem(rows, limit));
-    cfg.stream = stream;
     cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)k.blocks;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    const cudaLaunchConfig_t cfg =
+        cluster_config(limit, k.blocks, k.count, k.alone ? kClusterAlone : cluster_smem(rows, limit), stream, &at);
     return cudaLaunchKernelEx(&cfg, kernel, P, list + k.first, tc.tw, tc.th);
   });
 }

@@ -35,7 +35,9 @@ struct ClusterClass {
   bool alone;         // no two blocks on an SM
 };
 constexpr int kClusterAlone = 176 * 1024;  // shared memory that keeps a second block off the SM
-cudaError_t prepare_cluster();  // the kernel's attributes (outside a capture)
+// The kernel's attributes (outside a capture); *room: the largest clusters, alone
+// on their SMs, that the device holds at a time.
+cudaError_t prepare_cluster(int *room);
 cudaError_t launch_cluster(const KParams &P, const TileConfig &tc, const ClusterClass &k, const int *list,
                            cudaStream_t stream);
 // k_tile_count alone (interior cells and box per tile; reads only the masks).

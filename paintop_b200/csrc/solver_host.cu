@@ -62,6 +62,11 @@ bool cluster_silent() {
   const char *f = std::getenv("PAINTOP_CUDA_FAULT");
   return f && !std::strcmp(f, "cluster-silent");
 }
+// PAINTOP_CUDA_FAULT=cluster-room: as on a device that can place no clusters.
+bool no_cluster_room() {
+  const char *f = std::getenv("PAINTOP_CUDA_FAULT");
+  return f && !std::strcmp(f, "cluster-room");
+}
 constexpr unsigned long long kClusterWaitNs = 2000000000ull, kSilentWaitNs = 20000000ull;
 
 bool finite(double v) { return std::isfinite(v); }
@@ -179,15 +184,17 @@ Layout layout(const Plan &pl, bool stage) {
 // blocks, two to an SM (128 images of 256 x 256: 9.3 against 7.3 ms; 24 of them
 // 3.7 against 2.2, 128 of 96 x 96 1.3 against 0.5). Images that ask for different
 // sizes are launched side by side, a stream each size (2, 4 and 7 images of side
-// 64 to 256: 0.68, 0.53 and 0.71 ms against 1.9, 1.5 and 2.0), and only as many
-// as run at a time (their blocks fit the SMs): more of them, or larger images among them,
-// would wait for one another where k_solve takes all at once (22 images of side
-// 64 to 256: 2.4 ms against 4.9 one size after the other; 12 to side 800: 7.0
-// against 12.1). The largest clusters take 16 SMs each, and a call of more than
-// kLargeClusters of them is k_solve's.
-constexpr int kLargeClusters = 7;
+// 64 to 256: 0.68, 0.53 and 0.71 ms against 1.9, 1.5 and 2.0), but only while
+// their blocks take no more than half the GPU's places: each size's clusters need
+// SMs beside one another, and more of them, or larger images among them, wait for one
+// another where k_solve takes all at once (12 and 22 images of side 64 to 256,
+// one size after the other: 3.2 and 4.9 ms against 2.7 and 2.4; 12 to side 800: 12.1
+// against 7.0). The largest clusters take 16 SMs each, seven fit a B200, and a call
+// of more of them than fit is k_solve's (6 images of 512 x 512: 3.5 ms against 4.1; 30: 10.9
+// against 5.5).
+// (room: the largest clusters that the device holds at a time)
 constexpr double kFewValues = 4.0e6;
-void plan_clusters(Plan &pl, int sms) {
+void plan_clusters(Plan &pl, int sms, int room) {
   struct Want { int blocks, limit; bool rows2, rows4; };
   std::vector<Want> want(pl.sys.size(), Want{0, 0, false, false});
   bool least = true, fit = true;
@@ -210,7 +217,7 @@ void plan_clusters(Plan &pl, int sms) {
                    pl.many ? true : r.option > 0};
   }
   if (pl.many && !least) return;
-  int units = 0;  // half SMs
+  int units = 0;  // half SMs: a block of the least size takes one, a larger one two
   for (const Want &v : want) units += v.blocks * (v.limit > kClusterLeast ? 2 : 1);
   for (size_t i = 0; i < want.size(); ++i) {
     if (!want[i].blocks) continue;
@@ -225,17 +232,17 @@ void plan_clusters(Plan &pl, int sms) {
     pl.classes.push_back(k);
   }
   bool off = pl.classes.size() > 1 && (!fit || units > sms || pl.classes.size() > (size_t)pt_ctx::kSides + 1);
-  for (const ClusterClass &k : pl.classes) off |= k.limit > kClusterLeast && k.count > kLargeClusters;
+  for (const ClusterClass &k : pl.classes) off |= k.limit > kClusterLeast && k.count > room;
   if (off) {
     pl.classes.clear();
     pl.clist.clear();
   }
   // Blocks whose results are waited for one half-sweep at a time are better
-  // off alone on an SM while there are SMs to spare: shared memory asked for
+  // off alone on an SM while all clusters fit that way: shared memory asked for
   // beyond their own keeps others away.
   long long total = 0;
   for (const ClusterClass &k : pl.classes) total += (long long)k.count * k.blocks;
-  if (total <= sms * 3 / 4 + 1)
+  if (total <= (long long)room * kClusterMax)
     for (ClusterClass &k : pl.classes) k.alone = true;
 }
 
@@ -336,11 +343,16 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
     return PT_OK;
   }
 
-  plan_clusters(pl, ctx->sms);
-
   std::lock_guard<std::mutex> lock(ctx->mu);
   cudaError_t ce = cudaSetDevice(ctx->device);
   if (ce != cudaSuccess) return cuda_fail(ctx, ce, "cudaSetDevice");
+  // a device, or a share of one, that cannot place the largest clusters leaves
+  // every region to k_solve, which asks for no particular place
+  if (ctx->cluster_room < 0 && prepare_cluster(&ctx->cluster_room) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->cluster_room = 0;
+  }
+  if (ctx->cluster_room > 0 && !no_cluster_room()) plan_clusters(pl, ctx->sms, ctx->cluster_room);
   const Layout L = layout(pl, !devptr);
   if (!ctx->reserve(L.total)) return fail(ctx, PT_OOM, "device arena allocation failed");
   if (!ctx->reserve_pin(std::max(L.plan_end, L.results_end - L.st))) return fail(ctx, PT_OOM, "host staging allocation failed");
@@ -569,8 +581,7 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
   if (!ctx->solve_grid[pl.cfg]) {  // once a context and configuration
     KParams all = P;
     all.ntiles = INT32_MAX;
-    ce = prepare_cluster();
-    if (ce == cudaSuccess) ce = prepare_solve(all, pl.cfg, ctx->sms, &ctx->solve_grid[pl.cfg]);
+    ce = prepare_solve(all, pl.cfg, ctx->sms, &ctx->solve_grid[pl.cfg]);
     if (ce != cudaSuccess) return cuda_fail(ctx, ce, "solve prepare");
   }
   if (pl.classes.size() > 1) {
@@ -628,8 +639,8 @@ pt_status ptk_solve_batch(pt_ctx *ctx, const pt_problem *ps, uint32_t n, float *
       d.out = nullptr;
     }
     std::string key(reinterpret_cast<const char *>(shapes.data()), shapes.size() * sizeof(SysDesc));
-    const long long extra[6] = {pl.cfg, grid, (long long)(uintptr_t)base, (long long)L.total,
-                                (long long)pl.tiles.size(), (long long)P.budget_ns};
+    const long long extra[7] = {pl.cfg, grid, (long long)(uintptr_t)base, (long long)L.total,
+                                (long long)pl.tiles.size(), (long long)P.budget_ns, (long long)pl.classes.size()};
     key.append(reinterpret_cast<const char *>(extra), sizeof(extra));
     if (!ctx->gexec || key != ctx->gkey) {
       if (ctx->gexec) { cudaGraphExecDestroy(ctx->gexec); ctx->gexec = nullptr; }

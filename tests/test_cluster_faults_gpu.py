@@ -81,3 +81,22 @@ def test_budget_ends_one_cluster(cuda_lib):
         assert c.solve(src, tgt, mask, 97, 71, 3, max_iterations=10)[1][0]["iterations"] == 10
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("device", [False, True])
+def test_without_room_for_clusters_the_tiles_solve(ctx, device):
+    """PAINTOP_CUDA_FAULT=cluster-room: as where the device can place no cluster of
+    sixteen blocks. The call takes k_solve alone (fewer launches) and gives the same image."""
+    src, tgt, mask = _problem(97, 71, 3)
+    p = dict(source=src, target=tgt, mask=mask, width=97, height=71, channels=3, tolerance=1e-7, max_iterations=200)
+
+    def solve():
+        got = (device_solve.solve_batch(ctx, [p]) if device else ctx.solve_batch([p]))[0][0]
+        return got, ctx.last_timing()[2]
+
+    want, launches = solve()
+    with injected("cluster-room"):
+        got, fewer = solve()
+    again, same = solve()
+    assert fewer < launches == same
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32)) and np.array_equal(again.view(np.uint32), want.view(np.uint32))
