@@ -1335,7 +1335,7 @@ struct Mg {
   size_t tab = 0, io = 0;
   size_t u = 0, bl = 0, uw = 0, r64 = 0, part = 0, done = 0, red = 0, sc = 0, scale = 0, run = 0, x = 0, r = 0, z = 0,
          q = 0;
-  size_t p[2] = {0, 0};          // the search direction's two arrays (k_cg_apply)
+  size_t p[2] = {0, 0};          // the search direction's two arrays (k_cg_apply), in r64's place
   long long launches = 0;
   template <class T> T *at(size_t off) { return reinterpret_cast<T *>(base + off); }
   const Geo *geo(const Launch &l) { return at<Geo>(tab + l.geo); }
@@ -1544,7 +1544,11 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
   m.part = take((size_t)P * 8); m.done = take((size_t)U * sizeof(unsigned)); m.red = take((size_t)U * 8); m.sc = take((size_t)U * S_N * 8);
   m.scale = take((size_t)U * 8); m.run = take((size_t)U * 8);
   m.x = take(NC * 4); m.r = take(NC * 4); m.z = take(NC * 4); m.q = take(NC * 4);
-  m.p[0] = take(NC * 4); m.p[1] = take(NC * 4);
+  // The search direction lies where the FP64 residual does: k_mg_scale reads that
+  // for the last time before a run's first k_cg_apply, which reads no direction, and
+  // k_mg_residual64 writes it anew after the run. (A call then needs 45 bytes a
+  // cell and channel of level 0.)
+  m.p[0] = m.r64; m.p[1] = m.r64 + NC * 4;
   for (Inst &I : m.in) {
     if (I.dev) continue;
     const size_t n = (size_t)I.W * I.H, nc = n * I.C;

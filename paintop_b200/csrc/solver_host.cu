@@ -190,8 +190,8 @@ Layout layout(const Plan &pl, bool stage) {
 // another where k_solve takes all at once (12 and 22 images of side 64 to 256,
 // one size after the other: 3.2 and 4.9 ms against 2.7 and 2.4; 12 to side 800: 12.1
 // against 7.0). The largest clusters take 16 SMs each, seven fit a B200, and a call
-// of more of them than fit is k_solve's (6 images of 512 x 512: 3.5 ms against 4.1; 30: 10.9
-// against 5.5).
+// of more of them than fit is k_solve's (6 images of side 64 to 512: 3.5 ms against
+// 4.1; 30 of them 10.9 against 5.5).
 // (room: the largest clusters that the device holds at a time)
 constexpr double kFewValues = 4.0e6;
 void plan_clusters(Plan &pl, int sms, int room) {
