@@ -43,7 +43,6 @@
 // when the CG iterations reach max_iterations; stalled when an outer step fails to
 // lower the FP64 residual, or at once (0 iterations, interior set to NaN)
 // when a NaN or infinity in the inputs makes the residual non-finite.
-#include <cfloat>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -55,6 +54,7 @@
 
 #include "../../include/paintop_cuda.h"
 #include "ctx.h"
+#include "quotient.h"
 
 namespace {
 
@@ -310,20 +310,6 @@ __device__ __forceinline__ void ring_drain() { asm volatile("cp.async.wait_group
 __device__ __forceinline__ Row ring_row(const RowRing &q, int k) {
   const float4 x = q.v[k][threadIdx.x & 31];
   return Row{{x.x, x.y, x.z, x.w}};
-}
-
-// v / d by a divisor known in advance, inv = 1 / d rounded to nearest: the product
-// v inv corrected once by its residual, which fma gives exactly, is the correctly
-// rounded quotient (Brisebarre, Muller and Raina, "Accelerating correctly rounded
-// floating-point division when the divisor is known in advance", IEEE Trans.
-// Computers 53, 2004) while the residual is no smaller than FP32's smallest number
-// (|v| from 2^-100 on; below it is good to one unit in the last place). Infinities
-// and NaN keep the product. A division a cell made the strips of a screened system
-// slow, which wait for their own results: 700 x 420 RGBA, lambda 0.01, five
-// iterations: 2.15 ms with it, 1.11 so; 2048 x 2048 RGBA 4.57 and 2.49.
-__device__ __forceinline__ float divided(float v, float d, float inv) {
-  const float q = v * inv, r = fmaf(-q, d, v);
-  return fabsf(r) <= FLT_MAX ? fmaf(r, inv, q) : q;
 }
 
 // v / d. With POW2 d is a power of two (lambda 0) and the product with its
