@@ -21,23 +21,30 @@
 // c = fma(t, x1 - x0, x0) depends on the row and the edge only, and a
 // subsample column x_q = (q + 0.5) / 4 lies left of c exactly when
 // q < ceil(4c - 0.5), an integer computed exactly from c. So a warp owns a
-// span of 2048 pixels of one pixel row: its lanes compute each (edge, subsample
+// span of up to 2048 pixels of one pixel row: its lanes compute each (edge, subsample
 // row)'s crossing once, turn it into that integer, add crossings right of the
 // whole span to a span-wide winding, drop those left of it and keep the few
 // inside it. Then each lane sums up one 128-pixel run of the span; a run without
-// a crossing inside has one coverage and is stored as such, the others resolve
-// their pixels' 16 subsamples with integer compares. The arithmetic of every
-// crossing is the reference's and winding sums and parities do not depend on
-// the order crossings are visited in, so the mask is bit-identical to the
-// reference's rasterize(). More than 256 edges: a block a span, edges in chunks.
+// a crossing inside has one coverage and is stored as such. In the others the
+// lanes look at a crossing each, and the pixels' 16 subsamples are resolved from
+// those inside the run: up to seven one after the other, more by their sums over the
+// run's columns. The arithmetic of every crossing is the reference's and winding sums
+// and parities do not depend on the order crossings are visited in, so the mask is
+// bit-identical to the reference's rasterize(). More than 256 edges: a block a
+// span, edges in chunks.
 //
-// Bound by the stores of the plane (4096 x 4096: 67 MB). A block a span with a
-// barrier a row, every thread visiting every crossing, took 50 us for the
-// 12-vertex star; a warp a span takes 25 (19 in the
-// profiler, at 65% of the issue slots; writing the plane alone is 10).
+// Bound by the stores of the plane where it is large (4096 x 4096: 67 MB) and by a
+// warp's instructions, one after the other, where it is small. Kernel times in us, of a
+// block a span with a barrier a row and every thread visiting every crossing; of a warp a
+// span of 2048 pixels, every lane visiting every crossing; and of this one, whose
+// spans get shorter on small images:
+//   4096 x 4096, 12 vertices     62   22   23      256 vertices  186  133  111
+//   1000 x  700, 12 vertices     11   12   12      256 vertices   26   80   25
+//   2049 x   33, 12 vertices      7   15    8      256 vertices   15  131   13
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <mutex>
 #include <string>
@@ -135,27 +142,39 @@ __device__ __forceinline__ void store_row(float *out, int W, int j, int px, int 
 }
 
 // Polygons of at most kRowThreads edges: a warp a unit of one row and one span of
-// kRuns runs; crossings inside the span by subsample row in shared memory
-// (room for nedges each).
+// `span` runs; crossings inside the span by subsample row in shared memory
+// (room for nedges each). MANY: more than kManyEdges edges; then a run's columns
+// too, for a run of many crossings. (Of 12 vertices 4096 x 4096 takes 24 us that way, 22
+// with every lane looking at every crossing.)
 constexpr int kRun = 32 * kPix;               // pixels of a run: a float4 a lane
-constexpr int kRuns = 16;                     // runs of a span
-constexpr int kUnitWarps = kRowThreads / 32;  // warps per block
-size_t rows_smem(int nedges) { return (size_t)nedges * (sizeof(double4) + kUnitWarps * kSub * sizeof(int2)); }
+constexpr int kRuns = 16;                     // runs of a span at most
+constexpr int kUnitWarps = kRowThreads / 32;  // warps per block at most
+// Units an SM below which spans get shorter (1920 x 1080, 12 vertices: 12 us with 8, 14
+// with 16, 19 with 32; of 256 vertices 45 with 16, 53 with 32, 65 with 4).
+constexpr int kFewUnits = 8;
+constexpr int kManyEdges = 32;                // more than one crossing a lane
+size_t rows_smem(int nedges, int warps) {
+  return (size_t)nedges * (sizeof(double4) + warps * kSub * sizeof(int2)) +
+         (nedges > kManyEdges ? (size_t)warps * kRun * kSub * sizeof(int) : 0);
+}
 
-__global__ void __launch_bounds__(kRowThreads) k_mask_polygon_rows(int W, int H, const double4 *__restrict__ edges,
+template <bool MANY>
+__global__ void __launch_bounds__(kRowThreads, MANY ? 4 : 3) k_mask_polygon_rows(int W, int H, const double4 *__restrict__ edges,
                                                                   int nedges, int even_odd, double ymin, double ymax,
-                                                                  int vec4, int spans, float *__restrict__ out) {
+                                                                  int vec4, int span, int spans,
+                                                                  float *__restrict__ out) {
   extern __shared__ __align__(32) unsigned char smem[];
   double4 *sedge = reinterpret_cast<double4 *>(smem);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   int2 *cross = reinterpret_cast<int2 *>(sedge + nedges) + warp * kSub * nedges;  // [kSub][nedges] (column, direction)
+  int *last = reinterpret_cast<int *>(reinterpret_cast<int2 *>(sedge + nedges) + warps * kSub * nedges) + warp * kRun * kSub;
   const double step = 1.0 / (double)kSub;
-  for (int k = threadIdx.x; k < nedges; k += kRowThreads) sedge[k] = edges[k];
+  for (int k = threadIdx.x; k < nedges; k += blockDim.x) sedge[k] = edges[k];
   __syncthreads();
   const long long units = (long long)H * spans;
-  for (long long u = blockIdx.x * (long long)kUnitWarps + warp; u < units; u += (long long)gridDim.x * kUnitWarps) {
-    const int j = (int)(u / spans), x0 = (int)(u - (long long)j * spans) * (kRuns * kRun);
-    const int q0 = 4 * x0, q1 = 4 * min(x0 + kRuns * kRun, W);
+  for (long long u = blockIdx.x * (long long)warps + warp; u < units; u += (long long)gridDim.x * warps) {
+    const int j = units <= INT_MAX ? (int)u / spans : (int)(u / spans), x0 = (int)(u - (long long)j * spans) * (span * kRun);
+    const int q0 = 4 * x0, q1 = 4 * min(x0 + span * kRun, W);
     int count[kSub], base[kSub];
 #pragma unroll
     for (int t = 0; t < kSub; ++t) count[t] = base[t] = 0;
@@ -167,28 +186,40 @@ __global__ void __launch_bounds__(kRowThreads) k_mask_polygon_rows(int W, int H,
       for (int e0 = 0; e0 < nedges; e0 += 32) {
         const bool have = e0 + lane < nedges;
         const double4 E = have ? sedge[e0 + lane] : make_double4(0., 0., 0., 0.);
+        // all its ends at or above the first subsample row, or below the last: no crossing
+        if (MANY && __all_sync(0xffffffffu, fmax(E.y, E.w) <= ylo || fmin(E.y, E.w) > yhi)) continue;
+        // two rows' crossings at a time without a branch between them, so that their
+        // divisions' chains overlap (four would spill); where there is none the value is
+        // not used (and its divisor is 1, as 0 takes all lanes through the division's
+        // special cases)
 #pragma unroll
-        for (int t = 0; t < kSub; ++t) {
-          const double sy = fma((double)t + 0.5, step, (double)j);
-          const bool below0 = E.y <= sy, below1 = E.w <= sy;
-          int qc = 0, d = 0;
-          if (have && below0 != below1) {
-            const double tt = (sy - E.y) / (E.w - E.y);
-            qc = columns_left_of(fma(tt, E.z - E.x, E.x), W);
-            d = below0 ? 1 : -1;
+        for (int t0 = 0; t0 < kSub; t0 += 2) {
+          int qs[2], ds[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const double sy = fma((double)(t0 + i) + 0.5, step, (double)j);
+            const bool below0 = E.y <= sy, below1 = E.w <= sy;
+            const double tt = (sy - E.y) / (below0 == below1 ? 1.0 : E.w - E.y);
+            qs[i] = columns_left_of(fma(tt, E.z - E.x, E.x), W);
+            ds[i] = below0 == below1 ? 0 : (below0 ? 1 : -1);
           }
-          const bool right = d && qc >= q1, in = d && !right && qc > q0;  // (qc <= q0: no column of the span is left of it)
-          base[t] += __popc(__ballot_sync(0xffffffffu, right && d > 0)) - __popc(__ballot_sync(0xffffffffu, right && d < 0));
-          const unsigned m = __ballot_sync(0xffffffffu, in);
-          if (in) cross[t * nedges + count[t] + __popc(m & ((1u << lane) - 1u))] = make_int2(qc, d);
-          count[t] += __popc(m);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int t = t0 + i, qc = qs[i], d = ds[i];
+            const bool right = d && qc >= q1, in = d && !right && qc > q0;  // (qc <= q0: no column of the span is left of it)
+            base[t] += __popc(__ballot_sync(0xffffffffu, right && d > 0)) - __popc(__ballot_sync(0xffffffffu, right && d < 0));
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (in) cross[t * nedges + count[t] + __popc(m & ((1u << lane) - 1u))] = make_int2(qc, d);
+            count[t] += __popc(m);
+          }
         }
       }
       __syncwarp();
     }
-    // lane r: run r's coverage, or -1 where a crossing lies inside it
-    float run = 0.0f;
-    if (lane < kRuns) {
+    // lane r: run r's coverage, or -1 where a crossing lies inside it -- if the walk
+    // over the span's crossings costs less than resolving its runs
+    float run = -1.0f;
+    if (lane < span && count[0] + count[1] + count[2] + count[3] <= 16 * (span - 1)) {
       const int r0 = q0 + lane * 4 * kRun, r1 = r0 + 4 * kRun;
       int n = 0;
       bool crossed = false;
@@ -204,35 +235,56 @@ __global__ void __launch_bounds__(kRowThreads) k_mask_polygon_rows(int W, int H,
       }
       run = crossed ? -1.0f : (float)n * (1.0f / (float)(kSub * kSub));  // k / 16, exact
     }
-    const int runs = (min(x0 + kRuns * kRun, W) - x0 + kRun - 1) / kRun;
+    const int runs = (min(x0 + span * kRun, W) - x0 + kRun - 1) / kRun;
     for (int r = 0; r < runs; ++r) {
       const float n = __shfl_sync(0xffffffffu, run, r);
       const int px = x0 + r * kRun + lane * kPix;
       if (n >= 0.0f) {
         store_row(out, W, j, px, vec4, n, n, n, n);
       } else {
-        const int qp = 4 * px;
+        const int qp = 4 * px, r0 = q0 + r * 4 * kRun, r1 = r0 + 4 * kRun;
         int inside[kPix] = {0, 0, 0, 0};
 #pragma unroll
         for (int t = 0; t < kSub; ++t) {
-          int wt = base[t];
+          int wt = base[t], within = 0;
           const int m = count[t];
-          // the 16 columns' windings in a nibble each, 8 more than they are:
-          // up to seven crossings among them leave every nibble in 1 .. 15
+          const int2 *list = cross + t * nedges;
+          auto crossing = [&](int k) { return k < m ? list[k] : make_int2(r0, 0); };
+          // the 16 columns' windings in a nibble each, 8 more than they are; up to
+          // seven crossings leave every nibble in 1 .. 15
           constexpr unsigned long long kOnes = 0x1111111111111111ull;
           unsigned long long w = 8 * kOnes;
-          int own = 0;
-          for (int k = 0; k < m; ++k) {
-            const int2 c = cross[t * nedges + k];
-            if (c.x >= qp + kPix * kSub) {
-              wt += c.y;
-            } else if (c.x > qp) {  // columns qp .. c.x - 1 are left of it
-              const unsigned long long left = kOnes >> (4 * (kPix * kSub - (c.x - qp)));
-              w += c.y > 0 ? left : 0ull - left;
-              ++own;
+          auto count_one = [&](int x, int d) {
+            if (x >= qp + kPix * kSub) {
+              wt += d;
+            } else if (x > qp) {  // columns qp .. x - 1 are left of it
+              const unsigned long long left = kOnes >> (4 * (kPix * kSub - (x - qp)));
+              w += d > 0 ? left : 0ull - left;
+              if (!MANY) ++within;  // (the lane's)
+            }
+          };
+          if (!MANY || m <= 7) {  // every lane looks at every crossing
+            for (int k = 0; k < m; ++k) {
+              const int2 c = list[k];
+              count_one(c.x, c.y);
+            }
+          } else {
+            // a crossing a lane: those right of the run count alike for all columns
+            for (int k0 = 0; k0 < m; k0 += 32) {
+              const int2 c = crossing(k0 + lane);
+              wt += __popc(__ballot_sync(0xffffffffu, c.x >= r1 && c.y > 0)) - __popc(__ballot_sync(0xffffffffu, c.x >= r1 && c.y < 0));
+              within += __popc(__ballot_sync(0xffffffffu, c.x > r0 && c.x < r1));
+            }
+            // ... and only those inside it one after the other
+            for (int k0 = 0; k0 < m && within <= 7; k0 += 32) {
+              const int2 c = crossing(k0 + lane);
+              for (unsigned in = __ballot_sync(0xffffffffu, c.x > r0 && c.x < r1); in; in &= in - 1) {
+                const int from = __ffs((int)in) - 1;
+                count_one(__shfl_sync(0xffffffffu, c.x, from), __shfl_sync(0xffffffffu, c.y, from));
+              }
             }
           }
-          if (own <= 7) {
+          if (within <= 7) {
             unsigned long long in;  // a one in each covered column's nibble
             if (even_odd) {
               in = (w & kOnes) ^ ((wt & 1) ? kOnes : 0ull);
@@ -244,17 +296,55 @@ __global__ void __launch_bounds__(kRowThreads) k_mask_polygon_rows(int W, int H,
             }
 #pragma unroll
             for (int p = 0; p < kPix; ++p) inside[p] += __popc((unsigned)(in >> (16 * p)) & 0xffffu);
-          } else {  // column by column
+          } else if (!MANY) {  // column by column
 #pragma unroll
             for (int p = 0; p < kPix; ++p)
               for (int l = p * kSub; l < (p + 1) * kSub; ++l) {
                 int v = wt;
                 for (int k = 0; k < m; ++k) {
-                  const int2 c = cross[t * nedges + k];
+                  const int2 c = list[k];
                   if (c.x > qp && c.x < qp + kPix * kSub && qp + l < c.x) v += c.y;
                 }
                 inside[p] += even_odd ? (v & 1) : (v != 0);
               }
+          } else {
+            // many: each at the last column left of it; a column's winding is the sum
+            // from it to the run's end
+            int4 *own = reinterpret_cast<int4 *>(last + lane * kPix * kSub);
+#pragma unroll
+            for (int p = 0; p < kPix; ++p) own[p] = make_int4(0, 0, 0, 0);
+            __syncwarp();
+            for (int k = lane; k < m; k += 32) {
+              const int2 c = list[k];
+              if (c.x > r0 && c.x < r1) atomicAdd(last + (c.x - r0 - 1), c.y);
+            }
+            __syncwarp();
+            int sum = 0;
+#pragma unroll
+            for (int p = 0; p < kPix; ++p) {
+              const int4 v = own[p];
+              sum += v.x + v.y + v.z + v.w;
+            }
+            asm volatile("" ::: "memory");  // (they are read again below: held, they would spill)
+            int from = sum;  // this lane's and all later lanes'
+#pragma unroll
+            for (int o = 1; o < 32; o *= 2) {
+              const int x = __shfl_down_sync(0xffffffffu, from, o);
+              if (lane + o < 32) from += x;
+            }
+            int acc = wt + from - sum;
+            auto column = [&](int d) {
+              acc += d;
+              return even_odd ? (acc & 1) : (int)(acc != 0);
+            };
+#pragma unroll
+            for (int p = kPix - 1; p >= 0; --p) {
+              const int4 v = own[p];
+              inside[p] += column(v.w);
+              inside[p] += column(v.z);
+              inside[p] += column(v.y);
+              inside[p] += column(v.x);
+            }
           }
         }
         constexpr float u = 1.0f / (float)(kSub * kSub);  // k / 16, exact
@@ -478,14 +568,26 @@ extern "C" pt_status pt_mask_polygon(pt_ctx *ctx, uint32_t width, uint32_t heigh
       k_mask_polygon_chunked<<<grid, kRowThreads, 0, ctx->stream>>>((int)width, (int)height, dedges,
                                                                     (int)n_points, even_odd, ymin, ymax, vec4, out);
     } else {
-      // a unit a warp, at most eight blocks an SM
-      const int spans = (int)((width + kRuns * kRun - 1) / (kRuns * kRun));
-      const long long units = (long long)height * spans;
-      const unsigned blocks = (unsigned)std::min<long long>((units + kUnitWarps - 1) / kUnitWarps, (long long)ctx->sms * 8);
-      ce = cudaFuncSetAttribute(k_mask_polygon_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem(kRowThreads));
-      if (ce != cudaSuccess) return mfail(ctx, PT_LAUNCH_FAILED, cudaGetErrorString(ce));
-      k_mask_polygon_rows<<<blocks, kRowThreads, rows_smem((int)n_points), ctx->stream>>>(
-          (int)width, (int)height, dedges, (int)n_points, even_odd, ymin, ymax, vec4, spans, out);
+      // a unit a warp, at most eight blocks an SM; on images whose rows of whole
+      // spans leave SMs idle, shorter spans (a warp goes through its crossings one after
+      // the other) and smaller blocks
+      int span = kRuns, warps = kUnitWarps;
+      auto count = [&](int s) { return (long long)height * ((width + s * kRun - 1) / (s * kRun)); };
+      const bool many = n_points > (uint32_t)kManyEdges;
+      const int few = many ? 2 * kFewUnits : kFewUnits;  // (of many crossings each unit takes longer)
+      while (span > 1 && count(span) < (long long)ctx->sms * few) span /= 2;
+      const long long units = count(span);
+      while (warps > 1 && units < (long long)ctx->sms * warps) warps /= 2;
+      const unsigned blocks = (unsigned)std::min<long long>((units + warps - 1) / warps, (long long)ctx->sms * 8);
+      const size_t smem = rows_smem((int)n_points, warps);
+      if (smem > 48 * 1024) {  // (more than a launch may ask for unasked)
+        ce = cudaFuncSetAttribute(k_mask_polygon_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)rows_smem(kRowThreads, kUnitWarps));
+        if (ce != cudaSuccess) return mfail(ctx, PT_LAUNCH_FAILED, cudaGetErrorString(ce));
+      }
+      (many ? k_mask_polygon_rows<true> : k_mask_polygon_rows<false>)<<<blocks, 32 * warps, smem, ctx->stream>>>(
+          (int)width, (int)height, dedges, (int)n_points, even_odd, ymin, ymax, vec4, span,
+          (int)((width + span * kRun - 1) / (span * kRun)), out);
     }
     cudaEventRecord(ctx->ev[2], ctx->stream);
     return mask_finish(ctx, npx, dev, mask, out, 1);
