@@ -39,6 +39,7 @@ struct pt_ctx {
   cudaGraphExec_t mgexec[3] = {nullptr, nullptr, nullptr};  // multigrid-CG iteration: first / odd / even
   std::string mgkey;           // the problem shape and arena the multigrid graphs were captured for
   long long mgnodes = 0;       // kernels in one of those iterations
+  bool mg_prepared = false;    // the multigrid kernels' attributes are set
 
   void drop_graphs() {
     if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }  // they point into the arena

@@ -105,6 +105,24 @@ struct Io {
   float *out;
 };
 
+// Strips (below): columns, those owned, the halo either side; rows of a band, and
+// one flag a band and strip column: it has active cells among the owned ones.
+constexpr int kStripCols = 128, kStripStep = 112, kStripHalo = 8;
+constexpr int kStripWarps = 4;   // per block
+constexpr int kBand = 8;
+
+__host__ __device__ inline int strip_cols(int w) {
+  return w <= kStripCols ? 1 : 1 + (w - kStripCols + kStripStep - 1) / kStripStep;
+}
+
+// The flag of active cell (i, j)'s band (several threads may set one; all were
+// cleared before). With a kernel a level for them, reading the interior flags again,
+// a call without iterations took 129 us on 300 x 200, now 97.
+__device__ __forceinline__ void set_flag(const Geo &g, uint8_t *__restrict__ flags, int i, int j) {
+  const int gx = strip_cols(g.W), sx = i < kStripHalo ? 0 : min((i - kStripHalo) / kStripStep, gx - 1);
+  flags[g.f + (long long)(j / kBand) * gx + sx] = 1;
+}
+
 // ---- assembly ----------------------------------------------------------------
 // interior flag, u = anchor (or the warm guess at interior cells), b' =
 // fma(lambda, -anchor, laplacian(guidance)) at interior cells; level-0 tiles,
@@ -112,6 +130,7 @@ struct Io {
 __global__ void __launch_bounds__(kTx * kTy) k_mg_assemble(const Geo *__restrict__ geo,
                                                            const int4 *__restrict__ bmap, const Geo one,
                                                            const Io *__restrict__ io, uint8_t *__restrict__ act,
+                                                           uint8_t *__restrict__ flags,
                                                            double *__restrict__ u, double *__restrict__ bl,
                                                            double *__restrict__ uw) {
   const int4 bt = entry_of(bmap, one);
@@ -133,6 +152,7 @@ __global__ void __launch_bounds__(kTx * kTy) k_mg_assemble(const Geo *__restrict
     };
     const bool in = interior(i, j);
     a[k] = in ? 1 : 0;
+    if (in) set_flag(g, flags, i, j);
     // u is read at interior cells and their neighbours, b' at interior cells:
     // elsewhere neither is written (all cells of 4096 x 4096 took 285 us)
     if (!in && !interior(i - 1, j) && !interior(i + 1, j) && !interior(i, j - 1) && !interior(i, j + 1)) continue;
@@ -172,7 +192,8 @@ constexpr float kSmoothOmega = 1.25f;
 // fine plane is the entry's second).
 __global__ void __launch_bounds__(kTx * kTy) k_mg_coarsen(const Geo *__restrict__ geo,
                                                           const int4 *__restrict__ bmap, const Geo one,
-                                                          const uint8_t *__restrict__ af, uint8_t *__restrict__ ac) {
+                                                          const uint8_t *__restrict__ af, uint8_t *__restrict__ ac,
+                                                          uint8_t *__restrict__ flags) {
   const int4 bt = entry_of(bmap, one);
   const Geo g = bmap ? geo[bt.x] : one;
   const int Hc = g.H, Wf = g.W2, Hf = g.H2, b = tile_b(g), I = (b % g.gx) * kTx + threadIdx.x;
@@ -186,6 +207,7 @@ __global__ void __launch_bounds__(kTx * kTy) k_mg_coarsen(const Geo *__restrict_
         if (i < Wf && j < Hf) n += f[(size_t)j * g.P2 + i];
       }
     cc[(size_t)J * g.P + I] = n >= kCoarseRule ? 1 : 0;
+    if (n >= kCoarseRule) set_flag(g, flags, I, J);
   }
 }
 
@@ -210,14 +232,6 @@ __global__ void __launch_bounds__(kTx * kTy) k_mg_coarsen(const Geo *__restrict_
 // Border cells are inactive on every level (a coarse border cell has at most
 // two active children), so neighbours outside the image, which the edge lanes
 // replace by their own values, are never used.
-constexpr int kStripCols = 128, kStripStep = 112, kStripHalo = 8;
-constexpr int kStripWarps = 4;   // per block
-constexpr int kBand = 8;
-
-__host__ __device__ inline int strip_cols(int w) {
-  return w <= kStripCols ? 1 : 1 + (w - kStripCols + kStripStep - 1) / kStripStep;
-}
-
 struct Strip {
   int x0;        // the lane's first column
   int y0, y1;    // rows, trimmed to bands with active cells
@@ -247,26 +261,6 @@ __device__ __forceinline__ bool strip_of(const Geo &g, const uint8_t *__restrict
 
 __device__ __forceinline__ unsigned nibble(uint32_t c) {  // four flag bytes -> four bits
   return (c & 1u) | ((c >> 7) & 2u) | ((c >> 14) & 4u) | ((c >> 21) & 8u);
-}
-
-// Bands with active cells: one warp a band and strip column (its owned cells).
-__global__ void __launch_bounds__(kStripWarps * 32) k_mg_flags(const Geo *__restrict__ geo,
-                                                               const int4 *__restrict__ bmap, const Geo one,
-                                                               const uint8_t *__restrict__ act,
-                                                               uint8_t *__restrict__ flags) {
-  const int4 bt = entry_of(bmap, one);
-  const Geo g = bmap ? geo[bt.x] : one;
-  const int lane = threadIdx.x & 31, s = tile_b(g) * kStripWarps + (threadIdx.x >> 5);
-  const int sx = s % g.gx, b = s / g.gx;
-  if (b >= g.gy) return;
-  const int x0 = kStripStep * sx + 4 * lane;
-  const int lo = sx ? kStripStep * sx + kStripHalo : 0, hi = sx + 1 == g.gx ? g.P : kStripStep * (sx + 1) + kStripHalo;
-  uint32_t any = 0;
-  if (x0 >= lo && x0 < hi)
-    for (int y = b * kBand; y < min(g.H, (b + 1) * kBand); ++y)
-      any |= *reinterpret_cast<const uint32_t *>(act + g.o + (long long)y * g.P + x0);
-  const unsigned m = __ballot_sync(0xffffffffu, any != 0);
-  if (lane == 0) flags[g.f + (long long)b * g.gx + sx] = m != 0;
 }
 
 // A lane's four cells of a row
@@ -1314,7 +1308,7 @@ struct Mg {
   std::vector<Inst> in;
   std::vector<LevelArr> lv;
   Launch tiles0, strips0, dot0;  // level 0: tiles; strips; strips of instances without a finer level than the coarsest
-  std::vector<Launch> strips, flags, coarsen;  // per level
+  std::vector<Launch> strips, coarsen;  // per level
   size_t tails = 0;              // table of the tails, in the table area
   int ntails = 0;
   size_t tail_smem = 0;
@@ -1483,12 +1477,11 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
     m.strips0 = make_launch(blob, gs, true);
     m.dot0 = make_launch(blob, gd, true);
   }
-  m.strips.resize(Lmax); m.flags.resize(Lmax); m.coarsen.resize(Lmax);
+  m.strips.resize(Lmax); m.coarsen.resize(Lmax);
   for (int k = 0; k < Lmax; ++k) {
-    std::vector<Geo> gs, gf, gc;
+    std::vector<Geo> gs, gc;
     const int rows = rows_for(k, k == 0);
     for (const Inst &I : m.in) {
-      if (k < I.L) gf.push_back(stripped(geo_at(I, k), kBand));
       if (k < I.k0) {
         Geo g = geo_at(I, k);
         second(g, I, k + 1);
@@ -1501,7 +1494,6 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
       }
     }
     m.strips[k] = make_launch(blob, gs, true);
-    m.flags[k] = make_launch(blob, gf, true);
     m.coarsen[k] = make_launch(blob, gc, false);
   }
 
@@ -1516,18 +1508,21 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
   m.lv.resize(Lmax);
   for (int k = 0; k < Lmax; ++k) {
     m.lv[k].act = take((size_t)cells[k]);
-    m.lv[k].flags = take((size_t)nflags[k]);
     if (k > 0) {
       m.lv[k].e = take((size_t)ccells[k] * sizeof(float));
       m.lv[k].rhs = take((size_t)ccells[k] * sizeof(float));
     }
   }
-  const size_t up0 = o;  // the corrections after the passes up, cleared once
+  // cleared once a call, in one piece: the corrections after the passes up, the
+  // bands' flags and partial sums, the counts of finished blocks
+  const size_t clear0 = o;
   for (int k = 1; k < Lmax; ++k) m.lv[k].eu = take((size_t)ccells[k] * sizeof(float));
-  const size_t up1 = o;
+  for (int k = 0; k < Lmax; ++k) m.lv[k].flags = take((size_t)nflags[k]);
+  m.part = take((size_t)P * 8); m.done = take((size_t)U * sizeof(unsigned));
+  const size_t clear1 = o;
   const size_t NC = (size_t)ccells[0];
   m.u = take(NC * 8); m.bl = take(NC * 8); m.uw = any_warm ? take(NC * 8) : 0; m.r64 = take(NC * 8);
-  m.part = take((size_t)P * 8); m.done = take((size_t)U * sizeof(unsigned)); m.red = take((size_t)U * 8); m.sc = take((size_t)U * S_N * 8);
+  m.red = take((size_t)U * 8); m.sc = take((size_t)U * S_N * 8);
   m.scale = take((size_t)U * 8); m.run = take((size_t)U * 8);
   m.x = take(NC * 4); m.r = take(NC * 4); m.z = take(NC * 4); m.q = take(NC * 4);
   // The search direction lies where the FP64 residual does: k_mg_scale reads that
@@ -1568,12 +1563,14 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
   static_assert(sizeof(Tail) % 16 == 0, "the tails lie one after another");
 
   // tables and inputs
-  cudaError_t ce = cudaFuncSetAttribute(k_mg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
+  cudaError_t ce = cudaSuccess;
+  if (!ctx->mg_prepared) {  // once a context
+    ce = cudaFuncSetAttribute(k_mg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
+    ctx->mg_prepared = ce == cudaSuccess;
+  }
   if (ce == cudaSuccess)
     ce = cudaMemcpyAsync(m.base + m.tab, blob.b.data(), blob.b.size(), cudaMemcpyHostToDevice, m.st);
-  if (ce == cudaSuccess) ce = cudaMemsetAsync(m.base + m.part, 0, (size_t)P * 8, m.st);
-  if (ce == cudaSuccess) ce = cudaMemsetAsync(m.base + m.done, 0, (size_t)U * sizeof(unsigned), m.st);
-  if (ce == cudaSuccess && up1 > up0) ce = cudaMemsetAsync(m.base + up0, 0, up1 - up0, m.st);
+  if (ce == cudaSuccess) ce = cudaMemsetAsync(m.base + clear0, 0, clear1 - clear0, m.st);
   std::vector<Io> io(m.in.size());
   for (size_t k = 0; k < m.in.size() && ce == cudaSuccess; ++k) {
     const Inst &I = m.in[k];
@@ -1607,17 +1604,14 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
   float *x = m.at<float>(m.x), *r = m.at<float>(m.r), *z = m.at<float>(m.z);
   float *pp[2] = {m.at<float>(m.p[0]), m.at<float>(m.p[1])};
   const Sums sums{m.at<double>(m.part), m.at<unsigned>(m.done), sc};
-  k_mg_assemble<<<m.grid(A, 1), kBlock2, 0, m.st>>>(m.geo(A), m.bmap(A), A.one, iod, act0, u, bl,
+  k_mg_assemble<<<m.grid(A, 1), kBlock2, 0, m.st>>>(m.geo(A), m.bmap(A), A.one, iod, act0, m.at<uint8_t>(m.lv[0].flags), u, bl,
                                                      any_warm ? m.at<double>(m.uw) : nullptr);
   m.launches = 1;
   for (int k = 0; k < Lmax; ++k) {
-    const Launch &F = m.flags[k], &K = m.coarsen[k];
-    k_mg_flags<<<m.grid(F, 1), kStrip, 0, m.st>>>(m.geo(F), m.bmap(F), F.one, m.at<uint8_t>(m.lv[k].act),
-                                                  m.at<uint8_t>(m.lv[k].flags));
-    ++m.launches;
+    const Launch &K = m.coarsen[k];
     if (!K.n) continue;
     k_mg_coarsen<<<m.grid(K, 1), kBlock2, 0, m.st>>>(m.geo(K), m.bmap(K), K.one, m.at<uint8_t>(m.lv[k].act),
-                                                     m.at<uint8_t>(m.lv[k + 1].act));
+                                                     m.at<uint8_t>(m.lv[k + 1].act), m.at<uint8_t>(m.lv[k + 1].flags));
     ++m.launches;
   }
   cudaEventRecord(ctx->ev[1], m.st);
@@ -1636,7 +1630,6 @@ pt_status solve_group(pt_ctx *ctx, const pt_problem *ps, const std::vector<int> 
   // FP64 residual norms per unit of the current u -> host
   std::vector<double> nrm(U);
   auto residual = [&](const double *uu) -> cudaError_t {
-    cudaMemsetAsync(red, 0, (size_t)U * 8, m.st);  // (a unit without active cells has no strips)
     k_mg_residual64<<<gs, kStrip, 0, m.st>>>(g0, b0, S0.one, fl0, act0, uu, bl, r64, sums, red);
     ++m.launches;
     cudaError_t e = cudaMemcpyAsync(nrm.data(), red, (size_t)U * 8, cudaMemcpyDeviceToHost, m.st);
