@@ -69,6 +69,13 @@ UNIT = "solves/s"
 # reads u, b' and the cell flag (9 B)
 BYTES_PER_SWEEP = 13
 BYTES_PER_RESIDUAL = 9
+# one multigrid-CG iteration per level-0 cell and channel, every array crossing
+# memory once a pass: pass down r 4 B, flags 1, e 4, coarse right-hand side 1; pass up
+# e 4, r 4, flags 1, coarse correction 1, z 4; direction and operator z 4, p 4 + 4,
+# flags 1; step p 4, x 4 + 4, r 4 + 4, flags 1 -- 58 B, and the coarser levels'
+# passes a third of the two passes' 24 B
+MG_BYTES_PER_ITERATION = 66.0
+SOR_KERNELS = "ptk::k_solve (ptk::k_cluster_solve where a call's regions fit clusters)"
 
 
 def _dist():
@@ -543,12 +550,8 @@ def multigrid_arm(args):
     e2e_elapsed, _ = timed(False)
     its = [int(reps[c].iterations) for c in range(C)]
     interior = int((inst.mask[1:-1, 1:-1] > 0.5).sum())
-    # Modelled bytes of one CG iteration per level-0 cell and channel, as the
-    # kernels move them: 8 red-black half-sweeps (rhs 2 B, e 4 + 2 B, mask 1 B
-    # each), residual 13, restriction 4, prolongation 9, zeroing 4, r.z 8,
-    # direction 12, operator 9, update 24 -> 155 B; coarser levels add a third.
     cells = W * H * C
-    bytes_per_iter = 155.0 * cells * 4.0 / 3.0
+    bytes_per_iter = MG_BYTES_PER_ITERATION * cells
     solve_s = float(np.mean([t[0] for t in info])) / 1e3  # the iterative part (CUDA events)
     achieved = bytes_per_iter * float(np.mean(its)) / solve_s / 1e9
     peak, peak_kind = _peaks()
@@ -1062,9 +1065,7 @@ def measure_batch(ctx, dev, insts, interior, steps: int, warmup: int, multigrid:
     iters = [[r[c].iterations for c in range(i.channels)] for r, i in zip(rep_arr, insts)]
     conv = all(r[c].converged for r, i in zip(rep_arr, insts) for c in range(i.channels))
     if multigrid:
-        # the multigrid model: 155 B per level-0 cell and channel per CG
-        # iteration, a third more for the coarser levels (multigrid_arm)
-        alg = sum(155.0 * 4.0 / 3.0 * i.width * i.height * sum(it) for it, i in zip(iters, insts))
+        alg = sum(MG_BYTES_PER_ITERATION * i.width * i.height * sum(it) for it, i in zip(iters, insts))
     else:
         alg = sum(n_int * (BYTES_PER_SWEEP * sum(it) + BYTES_PER_RESIDUAL * (
             sum(it) + sum(r[c].refinements for c in range(i.channels))))
@@ -1139,7 +1140,7 @@ def batch_leg(ctx, dev, steps: int = 3, warmup: int = 1) -> dict:
             "roofline": {"bound": "hbm", "achieved": r["alg"] / (kmean / 1e3) / 1e9, "peak": peak,
                          "unit": "GB/s", "frac": r["alg"] / (kmean / 1e3) / 1e9 / peak,
                          "peak_kind": peak_kind,
-                         "kernel": "multigrid-CG iteration (modelled bytes)" if mg else "ptk::k_solve"},
+                         "kernel": "multigrid-CG iteration (modelled bytes)" if mg else SOR_KERNELS},
             "gpu_launches_per_batch": r["launches"] // max(1, steps), "clocks": r["clocks"],
             **({} if mg else {"tile_config": tile_config_label(r["config"]),
                               "tuned_entry": tuned_entry(probs)}),
@@ -1345,7 +1346,7 @@ def batch_arm(args):
             "roofline": {"bound": "hbm", "achieved": alg / (kmean / 1e3) / 1e9, "peak": peak,
                          "unit": "GB/s", "frac": alg / (kmean / 1e3) / 1e9 / peak, "traffic": None,
                          "kernel": "multigrid-CG iteration (all kernels, modelled bytes)" if args.multigrid
-                         else "ptk::k_solve", "peak_kind": peak_kind, "kernel_ms_mean": kmean},
+                         else SOR_KERNELS, "peak_kind": peak_kind, "kernel_ms_mean": kmean},
             "cpu_baseline": cpu, "gpu_launches": int(r["launches"]),
             "clocks": r["clocks"],
             "solver": {"converged": conv, "max_iterations": int(max(max(x) for x in iters)),
