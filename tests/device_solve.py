@@ -21,7 +21,7 @@ def solve_batch(ctx, problems, want_history=False):
                                   p["max_iterations"], p["tolerance"], p.get("omega", 1.8),
                                   p.get("flags", 0) | _lib.PT_FLAG_DEVICE_POINTERS)
         outs[i] = out.data_ptr()
-    torch.cuda.synchronize()
+    torch.cuda.current_stream().synchronize()  # (not the device: another thread may be capturing a graph)
     st = _lib.lib().pt_poisson_solve_batch(
         ctx.h, arr, n, outs, (C.POINTER(_lib.PtReport) * n)(*(C.cast(r, C.POINTER(_lib.PtReport)) for r in reps)),
         (C.c_void_p * n)(*(h.data_ptr() for h in hists)) if want_history else None)
