@@ -243,9 +243,9 @@ const char *pt_status_str(pt_status s);
 /* Last CUDA / watchdog detail recorded on this context ("" if none). */
 const char *pt_ctx_last_error(const pt_ctx *ctx);
 
-/* Wall budget of one persistent solve in seconds (default 600). A solve that
- * exceeds it stops at the next step boundary and returns PT_TIMEOUT; the
- * context stays usable. */
+/* Wall budget of one red-black call, all its images together, in seconds
+ * (default 600). A call that exceeds it stops at the next step boundary and
+ * returns PT_TIMEOUT; the context stays usable. */
 pt_status pt_ctx_set_budget(pt_ctx *ctx, double seconds);
 
 /* The context's CUDA stream (a cudaStream_t), for callers that order their own
